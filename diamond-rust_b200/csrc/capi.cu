@@ -59,7 +59,7 @@ struct Seqs {
   uint64_t* offsets = nullptr;
   uint32_t* owner = nullptr;
   std::vector<uint64_t> h_offsets;
-  uint64_t n = 0, total = 0;
+  uint64_t n = 0, total = 0, max_len = 0;
   Seqs() = default;
   Seqs(const Seqs&) = delete;
   ~Seqs() {
@@ -72,8 +72,10 @@ struct Seqs {
     n = count;
     h_offsets.assign(off, off + n + 1);
     total = off[n];
-    for (uint64_t i = 0; i < n; ++i)
+    for (uint64_t i = 0; i < n; ++i) {
       if (off[i + 1] < off[i]) throw Error(DRG_ERR_INVALID, "offsets must be non-decreasing");
+      max_len = std::max(max_len, off[i + 1] - off[i]);
+    }
     DRG_CUDA(cudaMalloc(&letters, total + 64));
     DRG_CUDA(cudaMalloc(&offsets, (n + 1) * sizeof(uint64_t)));
     DRG_CUDA(cudaMalloc(&owner, (total + 1) * sizeof(uint32_t)));
@@ -87,7 +89,7 @@ struct Seqs {
       launch_clamp_letters(letters, total, score_letters, c->stream);
     }
   }
-  DevSeqs view() const { return DevSeqs{letters, offsets, &h_offsets, score_letters}; }
+  DevSeqs view() const { return DevSeqs{letters, offsets, &h_offsets, score_letters, max_len}; }
 };
 
 template <typename T>
@@ -178,10 +180,12 @@ int drg_ctx_create(int device, drg_ctx** out) {
       // the side stream carries the long warps of the score pass: its blocks
       // are dispatched ahead of the bulk class's whenever an SM frees up
       cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&c->side2, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
       cudaMemPoolCreate(&c->pool, &props) != cudaSuccess ||
       cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, (void*)&keep) != cudaSuccess) {
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->side) cudaStreamDestroy(c->side);
+    if (c->side2) cudaStreamDestroy(c->side2);
     if (c->pool) cudaMemPoolDestroy(c->pool);
     release_slot(c->slot);
     delete c;
@@ -205,8 +209,10 @@ void drg_ctx_destroy(drg_ctx* c) {
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
   cudaStreamSynchronize(c->side);
+  cudaStreamSynchronize(c->side2);
   cudaStreamDestroy(c->stream);
   cudaStreamDestroy(c->side);
+  cudaStreamDestroy(c->side2);
   cudaMemPoolDestroy(c->pool);  // released once the last resident buffer is freed
   release_slot(c->slot);
   delete c;
@@ -473,8 +479,7 @@ int drg_extend_span_batch(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, uin
   Seqs qs, ss;
   qs.upload(c, ql, qo, nq);
   ss.upload(c, sl, so, ns);
-  // one Band per job (whole query as the window); the band kernels take what
-  // they support and the exact kernel the rest, as in the search's traceback
+  // one Band per job (whole query as the window), as in the search's traceback
   std::vector<Band> hb(n);
   std::vector<uint64_t> ops_off(n + 1, 0);
   for (uint64_t i = 0; i < n; ++i) {
@@ -496,17 +501,13 @@ int drg_extend_span_batch(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, uin
   DevArr<ExactOut> dout(n);
   DevArr<uint32_t> dops(ooff + 1);
   DevArr<uint64_t> doff(n + 1);
-  DevArr<int64_t> cnt(2);
-  DevArr<unsigned long long> cells(4);  // evaluated, lane, issued cells, transposed bands
-  DRG_CUDA(cudaMemsetAsync(cells.p, 0, 4 * sizeof(unsigned long long), c->stream));
   if (n) {
     DRG_CUDA(cudaMemcpyAsync(db_.p, hb.data(), n * sizeof(Band), cudaMemcpyHostToDevice, c->stream));
     DRG_CUDA(cudaMemsetAsync(dout.p, 0, n * sizeof(ExactOut), c->stream));
   }
   DRG_CUDA(cudaMemcpyAsync(doff.p, ops_off.data(), (n + 1) * 8, cudaMemcpyHostToDevice, c->stream));
   drg_run_stats st{};
-  run_bands(c, db_.p, n, qs.view(), ss.view(), sc, true, nullptr, nullptr, dout.p, dops.p, doff.p, &ops_off, st,
-            cnt.p, cells.p);
+  trace_bands(c, db_.p, n, qs.view(), ss.view(), sc, dout.p, dops.p, doff.p, st);
   std::vector<ExactOut> eo(n);
   std::vector<uint32_t> hops(ooff);
   if (n) DRG_CUDA(cudaMemcpyAsync(eo.data(), dout.p, n * sizeof(ExactOut), cudaMemcpyDeviceToHost, c->stream));
@@ -577,21 +578,21 @@ int drg_extend_span_scores(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, ui
   }
   DevArr<Band> db_(n);
   DevArr<int32_t> ds(n);
-  DevArr<int64_t> cnt(2);
-  DevArr<unsigned long long> cells(4);  // evaluated, lane, issued cells, transposed bands
-  DRG_CUDA(cudaMemsetAsync(cells.p, 0, 4 * sizeof(unsigned long long), c->stream));
+  // evaluated, lane, issued cells, transposed bands, -, bands in 32-bit lanes
+  DevArr<unsigned long long> cells(6);
+  DRG_CUDA(cudaMemsetAsync(cells.p, 0, 6 * sizeof(unsigned long long), c->stream));
   if (n) DRG_CUDA(cudaMemcpyAsync(db_.p, hb.data(), n * sizeof(Band), cudaMemcpyHostToDevice, c->stream));
   drg_run_stats st{};
-  run_bands(c, db_.p, n, qs.view(), ss.view(), sc, false, ds.p, nullptr, nullptr, nullptr, nullptr, nullptr, st, cnt.p,
-            cells.p);
+  score_bands(c, db_.p, n, qs.view(), ss.view(), sc, ds.p, nullptr, st, cells.p);
   if (n) DRG_CUDA(cudaMemcpyAsync(scores, ds.p, n * 4, cudaMemcpyDeviceToHost, c->stream));
-  unsigned long long cg[4] = {0, 0, 0, 0};
+  unsigned long long cg[6] = {};
   DRG_CUDA(cudaMemcpyAsync(cg, cells.p, sizeof(cg), cudaMemcpyDeviceToHost, c->stream));
   sync(c);
   st.dp_cells_gpu = cg[0];
   st.dp_cells_lane = cg[1];
   st.dp_cells_issued = cg[2];
   st.sw_transposed_bands = cg[3];
+  st.exact_bands = cg[5];
   if (stats) *stats = st;
   API_END(c)
 }

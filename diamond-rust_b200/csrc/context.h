@@ -20,6 +20,7 @@ struct drg_ctx {
   int slot = -1;                // constant-memory bank of this context (kConstSlots of them)
   cudaStream_t stream = nullptr;
   cudaStream_t side = nullptr;  // concurrent launches (wide-band classes)
+  cudaStream_t side2 = nullptr;  // a third one (traceback routes)
   cudaMemPool_t pool = nullptr;  // resident databases and batches (kept across calls)
   std::string err;
   // seed stage
@@ -30,8 +31,8 @@ struct drg_ctx {
   drg::DevBuf hits, hits_s, hits_u, flags, idx, segs, seg_keys, segs_c, keep;
   // bands and DP
   drg::DevBuf bands, bands_c, band_valid, pair_first, sw_keys, sw_keys_s, sw_order, sw_order_s, sw_tasks, scores,
-      state, sel_idx, sel_bands, exact_jobs, exact_out, exact_scratch, exact_ops;
-  drg::DevBuf tband, task_size, task_off, trace, rev, ex_bands, ops_off, trace_out, task_max;
+      state, sel_idx, sel_bands, sel_records, trace_ops;
+  drg::DevBuf sys_list, sys_list_redo, sys_wrap, sys_jobs, trace, ops_off, trace_out;
   drg::DevBuf sw_tasks_u, task_key, task_key_s, task_val, task_val_s, best_row, band_jobs_u, band_jobs, sw_rows, sw_rows_s,
       sw_keys_r, sw_order_r;
   drg::DevBuf bj_key, bj_key_s, bj_val, bj_val_s, bj_size, bj_off, bj_max, ops_cnt, ops_coff, ops_compact, verdict,
@@ -85,6 +86,7 @@ struct DevSeqs {
   const uint64_t* offsets;
   const std::vector<uint64_t>* h_offsets;
   const uint8_t* score_letters = nullptr;  // letters clamped to 24, when some code is above 24
+  uint64_t max_len = 0;                    // longest sequence
   // what the DP kernels read: they index residue profiles by the code
   const uint8_t* dp_letters() const { return score_letters ? score_letters : letters; }
 };
@@ -134,10 +136,12 @@ class TimeLog {
 struct ExactOut;
 // With a TimeLog the kernel times go into it; without one they are read
 // before returning (which waits for the launches).
-void run_bands(drg_ctx* c, const Band* bands, uint64_t n_bands, const DevSeqs& q, const DevSeqs& s,
-               const Scoring& sc, bool trace, int32_t* scores, int32_t* best_row, ExactOut* out, uint32_t* ops,
-               const uint64_t* d_ops_off, const std::vector<uint64_t>* h_ops_off, drg_run_stats& st,
-               int64_t* d_count, unsigned long long* cells_gpu, TimeLog* times = nullptr);
+void score_bands(drg_ctx* c, const Band* bands, uint64_t n_bands, const DevSeqs& q, const DevSeqs& s,
+                 const Scoring& sc, int32_t* scores, int32_t* best_row, drg_run_stats& st,
+                 unsigned long long* cells_gpu, TimeLog* times = nullptr);
+void trace_bands(drg_ctx* c, const Band* bands, uint64_t n, const DevSeqs& q, const DevSeqs& s, const Scoring& sc,
+                 ExactOut* out, uint32_t* ops, const uint64_t* d_ops_off, drg_run_stats& st,
+                 TimeLog* times = nullptr);
 // Whole-path search over resident inputs (pipeline.cu).
 void search(drg_ctx* ctx, const drg_db* db, const drg_batch* b, const drg_search_config* cfg, drg_result* out);
 // Whether n device letters hold a code above 24; syncs the context's stream.

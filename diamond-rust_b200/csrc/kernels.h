@@ -246,13 +246,6 @@ struct SwTask {        // one warp: up to 32 bands sharing a query window
   uint32_t transposed; // 1: rows are the subject, columns the query window (diagonals negated)
   uint32_t pad;
 };
-// Trace-pass result of one band: where its nibbles are and its first maximum.
-struct TraceBand {
-  uint64_t trace_off;  // first nibble word of the band
-  uint32_t row_first, width;
-  int32_t score, best_i, best_j;
-  int32_t stride;      // words between consecutive column steps of the band
-};
 struct SwScoreArgs {
   const Band* bands;
   const uint32_t* order;  // sorted band indices
@@ -266,8 +259,6 @@ struct SwScoreArgs {
   int32_t* score;     // score mode: per band (indexed like bands)
   int32_t* best_row;  // score mode: first DP row holding the best (0 if none)
   unsigned long long* cells_eval;  // optional: [0] DP cells the lanes evaluated (after skipping), [2] the warps' (idle lanes too)
-  uint2* trace;       // trace mode: nibble buffer
-  TraceBand* tband;   // trace mode: per band (indexed like bands)
   int8_t scores625[628];  // substitution scores, row-major
 };
 // One band of the intra-band (one warp per band) kernel.
@@ -276,22 +267,6 @@ struct SwBandJob {
   uint32_t row_first;  // first DP row (1-based)
   uint32_t n_strips;   // 16-row strips from row_first
   uint32_t pad;
-  uint64_t trace_off;  // trace mode: first uint2 of the band's nibbles
-};
-struct ExactOut;
-// Where a traced band's walk writes (per band t: ops at ops_off[t], n + m
-// slots; rev the same bytes as scratch; out[t] the record).
-struct WalkEnv {
-  const uint2* trace;
-  const uint8_t* q_letters;
-  const uint64_t* q_offsets;
-  const uint8_t* s_letters;
-  const uint64_t* s_offsets;
-  const uint64_t* ops_off;
-  uint8_t* rev;
-  uint32_t* ops;
-  ExactOut* out;
-  int exact_below;  // bands whose best is below this are left to the exact kernel
 };
 struct SwBandArgs {
   const Band* bands;
@@ -302,29 +277,21 @@ struct SwBandArgs {
   const uint8_t* s_letters;
   const uint64_t* s_offsets;
   int gap_open, gap_extend;
-  int32_t* score;     // score mode: per band
-  int32_t* best_row;  // score mode: first DP row holding the best
-  uint2* trace;       // trace mode: nibbles, strip k's step c at trace_off + k (W + 16) + c
-  TraceBand* tband;   // trace mode: per band
-  WalkEnv walk;       // trace mode: each band is walked right after its DP
+  int32_t* score;     // per band
+  int32_t* best_row;  // first DP row holding the best
   uint32_t xbuf_words;  // set by the launcher
   int8_t scores625[628];
 };
 size_t sw_band_smem(int max_width);
-void launch_sw_band(SwBandArgs a, int max_width, bool trace, cudaStream_t st);
+void launch_sw_band(SwBandArgs a, int max_width, cudaStream_t st);
 // Bands by width: route 0 (W <= 134), 1 (<= 271), 2 (<= 559) run in groups
 // of 8, 16, 32 lanes with rotating strips; route 3 (wider) in the block
-// kernel.  The traceback pass's few bands keep a warp each (route 2 up to
-// W 559): with several bands per warp too few warps remain to hide the
-// step's dependency chain.  max_width matters for route 3 only.
-__host__ __device__ inline int sw_band_route(int width, bool trace) {
-  if (width > 559) return 3;
-  if (trace) return 2;
-  return width <= 134 ? 0 : (width <= 271 ? 1 : 2);
+// kernel.  max_width matters for route 3 only.
+__host__ __device__ inline int sw_band_route(int width) {
+  return width > 559 ? 3 : (width <= 134 ? 0 : (width <= 271 ? 1 : 2));
 }
-void launch_sw_band_route(const SwBandArgs& a, int route, int max_width, bool trace, cudaStream_t st);
+void launch_sw_band_route(const SwBandArgs& a, int route, int max_width, cudaStream_t st);
 
-struct ExactOut;
 // Width classes of the packed kernel by the widest band of a warp (the shared
 // ring holds W + 1 words per thread); each fits 3 blocks per SM but the last.
 constexpr int kSwMinWidth = 17;   // narrower bands use the exact kernel
@@ -417,6 +384,115 @@ __host__ __device__ inline uint64_t exact_scratch_bytes(uint32_t n, uint32_t m, 
 void launch_sw_exact_with_matrix(const ExactJob* jobs, uint64_t n_jobs, int gap_open, int gap_extend, bool trace,
                                  uint8_t* scratch, uint32_t* ops, ExactOut* out, const int8_t* scores625,
                                  cudaStream_t st);
+// ---- 32-bit systolic DP: traceback, and scores of any band (sw_sys.cu) --------
+// The rows of a band with a matrix cell and its diagonals clamped to the
+// matrix (i - j lies in [1 - m, n - 1] for every cell).
+struct SysGeom {
+  int rs, rows;  // rows rs .. rs + rows - 1 (rows <= 0: none)
+  int d0, d1;
+};
+__host__ __device__ inline SysGeom sys_geom(const Band& b, int m, bool row_limit) {
+  SysGeom g;
+  const int64_t n = b.n;
+  int64_t d0 = b.d0, d1 = b.d1;
+  if (d0 < -(int64_t)m) d0 = -(int64_t)m;
+  if (d1 > n) d1 = n;
+  const int64_t rs = d0 + 1 > 1 ? d0 + 1 : 1;
+  int64_t re = m + d1 < n ? m + d1 : n;
+  if (row_limit && b.pad > 0 && (int64_t)b.pad < re) re = b.pad;  // no row below the best is needed
+  g.rs = (int)rs;
+  g.rows = m > 0 && d0 <= d1 && re >= rs ? (int)(re - rs + 1) : 0;
+  g.d0 = (int)d0;
+  g.d1 = (int)d1;
+  return g;
+}
+// Widest band of the rotating kernel with R rows per lane: the lane's next
+// strip takes it over 31 (R + 1) steps after the last one started.
+__host__ __device__ constexpr int sys_rot_max(int R) { return 31 * (R + 1) - R; }
+// Turns of R + 1 steps of S strips.
+__host__ __device__ inline int sys_rot_turns(int S, int W, int R) {
+  return S > 0 ? S - 1 + (W + R - 1 + R) / (R + 1) : 0;
+}
+// Strips of 128 rows of the block kernel: strip s works on the 32-column
+// phases [b0, b1] of lane 0's columns, turns of 8 strips `stride` phases apart,
+// at most nb phases each.
+struct SysBlockPlan {
+  int stride, nb;
+  __host__ __device__ int b0(const SysGeom& g, int s) const {
+    const int j = g.rs + 128 * s - g.d1;
+    return ((j > 1 ? j : 1) - 1) >> 5;
+  }
+  __host__ __device__ int b1(const SysGeom& g, int m, int s) const {
+    const int64_t j = (int64_t)g.rs + 128 * (int64_t)s + 127 - g.d0;
+    return (int)(((j < m ? j : m) + 31) >> 5);
+  }
+};
+__host__ __device__ inline SysBlockPlan sys_block_plan(const SysGeom& g, int m) {
+  SysBlockPlan p;
+  const int W = g.d1 - g.d0 + 1, by_m = (m + 31) / 32 + 1;
+  const int span = (W + 189) / 32 + 1;          // phases of a strip (its columns: W + 127)
+  const int behind = W > 835 ? (W - 835) / 32 + 2 : 0;  // phases a strip ends after the eighth below it could start
+  p.nb = span < by_m ? span : by_m;
+  p.stride = behind < by_m ? behind : by_m;
+  if (p.stride < 16) p.stride = 16;
+  return p;
+}
+// 0, 1: rotating kernel with 4, 8 rows per lane; 2: block kernel.
+__host__ __device__ inline int sys_route(const SysGeom& g, bool trace) {
+  const int W = g.d1 - g.d0 + 1;
+  if (W <= sys_rot_max(4)) return 0;
+  return trace && W <= sys_rot_max(8) ? 1 : 2;
+}
+// Trace bytes of a band and the steps its kernel takes (a scheduling cost).
+__host__ __device__ inline uint64_t sys_trace_bytes(const SysGeom& g, int m, int route, uint64_t* steps) {
+  const int W = g.d1 - g.d0 + 1;
+  if (g.rows <= 0) {
+    *steps = 0;
+    return 0;
+  }
+  if (route < 2) {
+    const int R = route == 0 ? 4 : 8;
+    const uint64_t t = (uint64_t)sys_rot_turns((g.rows + R - 1) / R, W, R) * (uint64_t)(R + 1);
+    *steps = t;
+    return t * 32u * (uint64_t)(R / 2);
+  }
+  const SysBlockPlan p = sys_block_plan(g, m);
+  const uint64_t S = (uint64_t)((g.rows + 127) / 128);
+  *steps = S * (uint64_t)p.nb * 4;
+  return S * (uint64_t)p.nb * 2048u;
+}
+struct SysJob {
+  uint32_t band;       // index into bands
+  uint32_t pad;
+  uint64_t trace_off;  // first trace byte
+};
+constexpr unsigned kSysBlocks = 148 * 4;  // blocks of the block kernel at once
+struct SysArgs {
+  const Band* bands;
+  const SysJob* jobs;      // trace mode: jobs [lo, hi)
+  const uint32_t* list;    // score mode: bands list[0, *d_count)
+  const int64_t* d_count;
+  uint64_t lo, hi;
+  const uint8_t* q_letters;  // letters as given (codes above 24 score as 24)
+  const uint64_t* q_offsets;
+  const uint8_t* s_letters;
+  const uint64_t* s_offsets;
+  int oc, ge;              // cost of a gap's first letter, of each further one
+  int exact_below;         // the matrix's largest score + 1
+  int32_t* score;          // score mode, per band
+  int32_t* best_row;       // score mode: a bound of the first row holding the best (may be null)
+  uint8_t* trace;          // trace mode: byte trace_base of the jobs' trace
+  uint64_t trace_base;
+  const uint64_t* ops_off; // trace mode, per band: its first op slot (n + m slots)
+  uint32_t* ops;
+  ExactOut* out;
+  int2* wrap;              // block kernel: wrap_words words per block, one per subject column
+  uint64_t wrap_words;
+  int8_t scores625[628];
+};
+void launch_sys_score(SysArgs a, int route, uint64_t n_max, cudaStream_t st);
+void launch_sys_trace(SysArgs a, int route, cudaStream_t st);
+
 // ---- E-value gate (evalue.cu) ---------------------------------------------
 struct AlpDev {
   double lambda, k, ln_k, a, b, alpha, beta, sigma, tau, v_thr, c_thr;

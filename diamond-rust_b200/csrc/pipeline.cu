@@ -72,16 +72,6 @@ void select_indices_dev(drg_ctx* c, const uint8_t* flags, uint64_t n, uint32_t* 
   });
 }
 
-// Indices i < n with flags[i] != 0, in order.
-uint64_t select_indices(drg_ctx* c, const uint8_t* flags, uint64_t n, uint32_t* out, int64_t* d_count) {
-  if (n == 0) return 0;
-  thrust::counting_iterator<uint32_t> it(0);
-  cub_call(c, [&](void* t, size_t& b) {
-    return cub::DeviceSelect::Flagged(t, b, it, flags, out, d_count, (int64_t)n, c->stream);
-  });
-  return (uint64_t)fetch(c, d_count);
-}
-
 // Device time of a stage on the context's stream, added to a stats field
 // when the search's TimeLog resolves (no wait here).
 struct Timer {
@@ -302,8 +292,7 @@ __global__ void k_sw_task_flags(const uint32_t* gstart, uint64_t n, uint8_t* f, 
 }
 __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const uint64_t* keys, uint64_t n_fast,
                                 uint64_t transposed_key, const uint32_t* order, const Band* bands,
-                                const uint64_t* s_offsets, bool row_limit,
-                                SwTask* tasks, uint64_t* sort_key, uint32_t* sort_val, uint64_t* trace_size,
+                                const uint64_t* s_offsets, SwTask* tasks, uint64_t* sort_key, uint32_t* sort_val,
                                 unsigned long long* cells_gpu, const int64_t* d_n_tasks, const int64_t* d_n_fast) {
   uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (d_n_tasks) n_tasks = (uint64_t)*d_n_tasks;
@@ -322,7 +311,6 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
     int64_t m = (int64_t)(s_offsets[b.subject + 1] - s_offsets[b.subject]);
     int64_t rs, re;
     band_rows(b, m, transposed, &rs, &re);
-    if (row_limit && !transposed && b.pad > 0 && (int64_t)b.pad < re) re = b.pad;  // rows up to the best
     const uint32_t w = (uint32_t)((key >> kWidthShift) & 0x7FF);
     if (re > row_last) row_last = re;
     if (rs < row_first) row_first = rs;
@@ -347,7 +335,6 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
   // class, then longest first (a scheduling order: 21 bits of steps, saturated, suffice)
   sort_key[t] = ((uint64_t)cls << kCostBits) | (kCostMax - (steps < kCostMax ? steps : kCostMax));
   sort_val[t] = (uint32_t)t;
-  if (trace_size) trace_size[t] = steps * 32ull;
   if (cells_gpu) {
     atomicAdd(cells_gpu + 1, (unsigned long long)lane_cells);  // evaluated cells: counted by k_sw
     if (transposed) atomicAdd(cells_gpu + 3, (unsigned long long)cnt);
@@ -396,17 +383,15 @@ __global__ void k_compact_ops(const uint32_t* ops, const uint64_t* ops_off, cons
   for (uint32_t i = 0; i < out[k].n_ops; ++i) o[i] = src[i];
 }
 
-// Jobs of the one-warp-per-band kernel for the first n bands of the sorted
-// order: rows [rs, re] (re limited to the best row when known), longest first.
-// The job of sorted band k (order[k] indexes bands) and its sort key.
+// The band kernel's job of sorted band k (order[k] indexes bands): its rows,
+// and a sort key by kernel route, then longest first.
 __device__ __forceinline__ void band_job(const uint32_t* order, uint64_t k, const Band* bands,
-                                         const uint64_t* s_offsets, bool trace, SwBandJob* jobs, uint64_t* sort_key,
+                                         const uint64_t* s_offsets, SwBandJob* jobs, uint64_t* sort_key,
                                          uint32_t* sort_val, unsigned long long* max_width) {
   const uint32_t i = order[k];
   const Band b = bands[i];
   const int64_t m = (int64_t)(s_offsets[b.subject + 1] - s_offsets[b.subject]);
   int64_t re = m + b.d1 < (int64_t)b.n ? m + b.d1 : (int64_t)b.n;
-  if (b.pad > 0 && (int64_t)b.pad < re) re = b.pad;  // the traceback needs no row below the best
   const int64_t rs = band_first_row(b);
   if (re < rs) re = rs;
   const uint32_t W = (uint32_t)(b.d1 - b.d0 + 1);
@@ -415,21 +400,14 @@ __device__ __forceinline__ void band_job(const uint32_t* order, uint64_t k, cons
   j.row_first = (uint32_t)rs;
   j.n_strips = (uint32_t)((re - rs + 16) / 16);
   j.pad = W;
-  j.trace_off = 0;
   jobs[k] = j;
   // by kernel route (sw_band_route), then longest first
-  const int route = sw_band_route((int)W, trace);
+  const int route = sw_band_route((int)W);
   const uint64_t cost = (uint64_t)(j.n_strips - 1) * 19ull + W + 16ull;
   sort_key[k] = ((uint64_t)route << kCostBits) | (kCostMax - (cost < kCostMax ? cost : kCostMax));
   sort_val[k] = (uint32_t)k;
   atomicMax(max_width, (unsigned long long)W);
   atomicAdd(max_width + 1 + route, 1ull);
-}
-__global__ void k_band_jobs(const uint32_t* order, const uint64_t* keys, uint64_t n, const Band* bands,
-                            const uint64_t* s_offsets, bool trace, SwBandJob* jobs, uint64_t* sort_key,
-                            uint32_t* sort_val, unsigned long long* max_width) {
-  uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (k < n) band_job(order, k, bands, s_offsets, trace, jobs, sort_key, sort_val, max_width);
 }
 // Score pass on device counts: the wide bands are sorted positions
 // [cnt[1], cnt[0]) (after the narrow ones); n bounds their count, which is
@@ -440,58 +418,71 @@ __global__ void k_band_jobs_dev(const uint32_t* order, int64_t* cnt, uint64_t n,
   uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const uint64_t n_wide = (uint64_t)(cnt[0] - cnt[1]);
   if (k == 0) cnt[15] = (int64_t)n_wide;
-  if (k < n && k < n_wide) band_job(order + cnt[1], k, bands, s_offsets, false, jobs, sort_key, sort_val, max_width);
+  if (k < n && k < n_wide) band_job(order + cnt[1], k, bands, s_offsets, jobs, sort_key, sort_val, max_width);
 }
 __global__ void k_gather_band_jobs(const SwBandJob* in, const uint32_t* idx, uint64_t n, SwBandJob* out,
-                                   uint64_t* size, const int64_t* d_n = nullptr) {
+                                   const int64_t* d_n) {
   uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (d_n) {  // device count: no sizes
-    if (k < n && k < (uint64_t)*d_n) out[k] = in[idx[k]];
+  if (k < n && k < (uint64_t)*d_n) out[k] = in[idx[k]];
+}
+
+// Bands that the packed kernels did not settle, listed for the 32-bit kernel:
+// positions [lo, hi) of the sorted order, every one (not packed) or those
+// whose packed best is not above the matrix's largest score (exact_below =
+// that + 1: only then can the reference's clamped column past row m + d1 hold
+// the best).  lists[r]: bands of route r, *counts[r] of them, in no fixed
+// order (each band's score is its own).
+__global__ void k_sys_lists(const uint32_t* order, uint64_t lo, uint64_t hi, const int32_t* score, int exact_below,
+                            const Band* bands, const uint64_t* s_offsets, uint32_t* list0, uint32_t* list1,
+                            int64_t* counts, unsigned long long* total) {
+  const uint64_t k = lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (k >= hi) return;
+  const uint32_t i = order[k];
+  if (score && score[i] >= exact_below) return;
+  const Band b = bands[i];
+  const int m = (int)(s_offsets[b.subject + 1] - s_offsets[b.subject]);
+  const int route = sys_route(sys_geom(b, m, false), false);
+  const unsigned long long at =
+      atomicAdd(reinterpret_cast<unsigned long long*>(counts) + (route == 0 ? 0 : 1), 1ull);
+  (route == 0 ? list0 : list1)[at] = i;
+  if (total) atomicAdd(total, 1ull);
+}
+
+// Traceback jobs: by kernel route, then longest first; count[r] = jobs of
+// route r.
+__global__ void k_sys_jobs(const Band* bands, uint64_t n, const uint64_t* s_offsets, uint64_t* sort_key,
+                           uint32_t* sort_val, unsigned long long* count) {
+  const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const Band b = bands[k];
+  const int m = (int)(s_offsets[b.subject + 1] - s_offsets[b.subject]);
+  const SysGeom g = sys_geom(b, m, true);
+  const int route = sys_route(g, true);
+  uint64_t steps;
+  sys_trace_bytes(g, m, route, &steps);
+  sort_key[k] = ((uint64_t)route << kCostBits) | (kCostMax - (steps < kCostMax ? steps : kCostMax));
+  sort_val[k] = (uint32_t)k;
+  atomicAdd(count + route, 1ull);
+}
+__global__ void k_sys_sizes(const uint32_t* idx, uint64_t n, const Band* bands, const uint64_t* s_offsets,
+                            SysJob* jobs, uint64_t* size) {
+  const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (k > n) return;
+  if (k == n) {
+    size[k] = 0;
     return;
   }
-  if (k < n) {
-    const SwBandJob j = in[idx[k]];
-    out[k] = j;
-    size[k] = (uint64_t)j.n_strips * (j.pad + 16ull);
-  } else if (k == n) {
-    size[k] = 0;
-  }
+  const uint32_t i = idx[k];
+  const Band b = bands[i];
+  const int m = (int)(s_offsets[b.subject + 1] - s_offsets[b.subject]);
+  const SysGeom g = sys_geom(b, m, true);
+  uint64_t steps;
+  jobs[k] = SysJob{i, 0, 0};
+  size[k] = sys_trace_bytes(g, m, sys_route(g, true), &steps);
 }
-__global__ void k_set_band_trace_off(SwBandJob* jobs, const uint64_t* off, uint64_t n) {
-  uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+__global__ void k_sys_offsets(SysJob* jobs, const uint64_t* off, uint64_t n) {
+  const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (k < n) jobs[k].trace_off = off[k];
-}
-
-// Bands the packed kernel did not take, or whose best is not above the
-// matrix's largest score (exact_below = that + 1): only then can a cell the
-// packed kernels skip (the reference's clamped column past row m + d1) hold
-// the best.
-__global__ void k_exact_flags(const uint32_t* order, uint64_t n_fast, uint64_t n, const int32_t* score,
-                              const TraceBand* tband, int exact_below, uint8_t* f) {
-  uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  uint32_t i = order[s];
-  int v = tband ? tband[i].score : score[i];
-  f[s] = (s >= n_fast || v < exact_below) ? 1 : 0;
-}
-
-__global__ void k_gather_positions(const uint32_t* pos, const uint32_t* order, uint64_t n, const Band* bands,
-                                   uint32_t* idx, Band* out) {
-  uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  uint32_t i = order[pos[k]];
-  idx[k] = i;
-  out[k] = bands[i];
-}
-
-__global__ void k_scatter_scores(const uint32_t* idx, const ExactOut* out, uint64_t n, int32_t* score) {
-  uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (k < n) score[idx[k]] = out[k].score;
-}
-
-__global__ void k_scatter_exact(const uint32_t* idx, const ExactOut* src, uint64_t n, ExactOut* dst) {
-  uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (k < n) dst[idx[k]] = src[k];
 }
 
 __global__ void k_state_flags(const uint8_t* state, uint64_t n, uint8_t* f) {
@@ -515,69 +506,22 @@ __global__ void k_gather_bands_dev(const uint32_t* idx, uint64_t n, const int64_
 
 }  // namespace
 
-// The banded DP of n_bands bands (any order).  The packed kernel takes the
-// bands whose width it supports (by width class) and whose best cannot
-// overflow 16 bits; the exact kernel takes the rest and every band whose
-// packed best is not above the matrix's largest score.
-//  score mode (trace == false): scores[i] = best score (0 = None).
-//  trace mode: out[i] and the band's ops at h_ops_off[i] in ops (n + m slots
-//  per band), the same records the exact kernel produces.
 namespace {
 
-// Jobs of the one-warp-per-band kernel for n bands (order[k] indexes bands),
-// longest first, with their trace offsets when trace is set.
+// Jobs of the band kernel by route.
 struct BandJobs {
   SwBandJob* jobs = nullptr;
   uint64_t n = 0;
   int max_width = 0;
-  uint64_t trace_words = 0;
   uint64_t route_lo[5] = {0, 0, 0, 0, 0};  // jobs [route_lo[r], route_lo[r + 1]) take route r
 };
-BandJobs make_band_jobs(drg_ctx* c, const uint32_t* order, const uint64_t* keys, uint64_t n, const Band* bc,
-                        const uint64_t* s_offsets, bool trace) {
-  BandJobs r;
-  r.n = n;
-  if (n == 0) return r;
-  SwBandJob* jobs_u = c->band_jobs_u.as<SwBandJob>(n);
-  r.jobs = c->band_jobs.as<SwBandJob>(n);
-  uint64_t* key = c->bj_key.as<uint64_t>(n);
-  uint64_t* key_s = c->bj_key_s.as<uint64_t>(n);
-  uint32_t* val = c->bj_val.as<uint32_t>(n);
-  uint32_t* val_s = c->bj_val_s.as<uint32_t>(n);
-  unsigned long long* dmaxw = c->bj_max.as<unsigned long long>(5);  // max width, jobs per route
-  DRG_CUDA(cudaMemsetAsync(dmaxw, 0, 5 * sizeof(unsigned long long), c->stream));
-  count_launch();
-  k_band_jobs<<<ceil_div(n, 256), 256, 0, c->stream>>>(order, keys, n, bc, s_offsets, trace, jobs_u, key, val,
-                                                       dmaxw);
-  const uint32_t* val_sorted = dsort(c, key, key_s, val, val_s, n, 0, kCostBits + 3).vals;
-  uint64_t* size = c->bj_size.as<uint64_t>(n + 1);
-  uint64_t* off = c->bj_off.as<uint64_t>(n + 1);
-  count_launch();
-  k_gather_band_jobs<<<ceil_div(n + 1, 256), 256, 0, c->stream>>>(jobs_u, val_sorted, n, r.jobs, size);
-  if (trace) {
-    cub_call(c, [&](void* t, size_t& b) {
-      return cub::DeviceScan::ExclusiveSum(t, b, size, off, (int64_t)n + 1, c->stream);
-    });
-    count_launch();
-    k_set_band_trace_off<<<ceil_div(n, 256), 256, 0, c->stream>>>(r.jobs, off, n);
-  }
-  // max width, jobs per route and (trace) the trace size, in one wait
-  unsigned long long* h = c->h_stage.as<unsigned long long>(6);
-  DRG_CUDA(cudaMemcpyAsync(h, dmaxw, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-  if (trace) DRG_CUDA(cudaMemcpyAsync(h + 5, off + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
-  DRG_CUDA(cudaStreamSynchronize(c->stream));
-  r.max_width = (int)h[0];
-  for (int k = 0; k < 4; ++k) r.route_lo[k + 1] = r.route_lo[k] + h[1 + k];
-  if (trace) r.trace_words = h[5];
-  return r;
-}
 
 // The band kernels of jobs bj, one launch per route.
-void launch_band_routes(SwBandArgs ba, const BandJobs& bj, bool trace, cudaStream_t st) {
+void launch_band_routes(SwBandArgs ba, const BandJobs& bj, cudaStream_t st) {
   for (int k = 0; k < 4; ++k) {
     ba.lo = bj.route_lo[k];
     ba.hi = bj.route_lo[k + 1];
-    launch_sw_band_route(ba, k, bj.max_width, trace, st);
+    launch_sw_band_route(ba, k, bj.max_width, st);
   }
 }
 
@@ -597,12 +541,59 @@ SwBandArgs band_args(const Band* bc, const BandJobs& bj, const DevSeqs& qs, cons
   return ba;
 }
 
+SysArgs sys_args(const Band* bc, const DevSeqs& qs, const DevSeqs& s, const Scoring& scr) {
+  SysArgs a{};
+  a.bands = bc;
+  a.q_letters = qs.letters;
+  a.q_offsets = qs.offsets;
+  a.s_letters = s.letters;
+  a.s_offsets = s.offsets;
+  a.oc = scr.gap_open + scr.gap_extend;
+  a.ge = scr.gap_extend;
+  a.exact_below = scr.max_score + 1;
+  std::memcpy(a.scores625, scr.scores, 625);
+  return a;
+}
+// The block kernel's rows of the subject columns, for as many blocks as
+// 256 MB hold (one at least).
+unsigned sys_wrap(drg_ctx* c, SysArgs& a, uint64_t max_m) {
+  a.wrap_words = max_m + 1;
+  const uint64_t fit = (256ull << 20) / (a.wrap_words * sizeof(int2));
+  const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(fit, kSysBlocks));
+  a.wrap = c->sys_wrap.as<int2>(a.wrap_words * blocks);
+  return blocks;
+}
+
+// Scores of the bands at positions [lo, hi) of the sorted order through the
+// 32-bit kernel: all of them, or those below exact_below.  No host wait.
+void sys_scores(drg_ctx* c, SysArgs a, DevBuf& lists, const uint32_t* order, uint64_t lo, uint64_t hi,
+                const int32_t* below, int64_t* counts, unsigned long long* total, uint64_t max_m, cudaStream_t st) {
+  if (hi <= lo) return;
+  uint32_t* l0 = lists.as<uint32_t>(2 * (hi - lo));
+  uint32_t* l1 = l0 + (hi - lo);
+  count_launch();
+  k_sys_lists<<<ceil_div(hi - lo, 256), 256, 0, st>>>(order, lo, hi, below, a.exact_below, a.bands, a.s_offsets, l0,
+                                                       l1, counts, total);
+  DRG_CUDA(cudaGetLastError());
+  const unsigned blocks = sys_wrap(c, a, max_m);
+  a.list = l1;
+  a.d_count = counts + 1;
+  launch_sys_score(a, 2, std::min<uint64_t>(hi - lo, blocks), st);
+  a.list = l0;
+  a.d_count = counts;
+  launch_sys_score(a, 0, hi - lo, st);
+}
+
 }  // namespace
 
-void run_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs, const DevSeqs& s,
-               const Scoring& scr, bool trace, int32_t* scores, int32_t* best_row, ExactOut* out, uint32_t* ops,
-               const uint64_t* d_ops_off, const std::vector<uint64_t>* h_ops_off, drg_run_stats& st,
-               int64_t* d_count, unsigned long long* cells_gpu, TimeLog* times) {
+// Best scores of n_bands bands (any order): scores[i] (0 = None), and a bound
+// of the row that holds it.  The packed kernel takes the bands whose width it
+// supports (by width class) and whose best cannot overflow 16 bits; the
+// 32-bit kernel takes the rest and every band whose packed best is not above
+// the matrix's largest score.
+void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs, const DevSeqs& s,
+                 const Scoring& scr, int32_t* scores, int32_t* best_row, drg_run_stats& st,
+                 unsigned long long* cells_gpu, TimeLog* times) {
   if (n_bands == 0) return;
   TimeLog own;
   TimeLog* log = times ? times : &own;
@@ -615,16 +606,12 @@ void run_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs, 
   uint32_t* rows_s = c->sw_rows_s.as<uint32_t>(n_bands);
   uint64_t* swk_r = c->sw_keys_r.as<uint64_t>(n_bands);
   uint32_t* swo_r = c->sw_order_r.as<uint32_t>(n_bands);
-  // the score pass may transpose bands; the traceback runs them as they are
-  uint32_t* tr_count = nullptr;
-  if (!trace) {
-    const uint64_t n_subjects = s.h_offsets->size() - 1;
-    tr_count = c->tr_count.as<uint32_t>(n_subjects);
-    DRG_CUDA(cudaMemsetAsync(tr_count, 0, n_subjects * sizeof(uint32_t), c->stream));
-    count_launch();
-    k_sw_tr_count<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(bc, n_bands, s.offsets, scr.max_score,
-                                                                  sw_tune(c, scr), tr_count, rows);
-  }
+  const uint64_t n_subjects = s.h_offsets->size() - 1;
+  uint32_t* tr_count = c->tr_count.as<uint32_t>(n_subjects);
+  DRG_CUDA(cudaMemsetAsync(tr_count, 0, n_subjects * sizeof(uint32_t), c->stream));
+  count_launch();
+  k_sw_tr_count<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(bc, n_bands, s.offsets, scr.max_score,
+                                                                sw_tune(c, scr), tr_count, rows);
   count_launch();
   // group field: target << 16 | window start, or the subject (transposed)
   SwKeyBits kb;
@@ -651,221 +638,245 @@ void run_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs, 
   // score pass counts, on the device until the one wait before the launches:
   //   [0] fast bands  [1] narrow bands  [2] tasks  [3..5] class bounds
   //   [6] wide max width  [7..10] wide jobs per route  [11..14] longest warp
-  //   per class  [15] wide bands
-  int64_t* cnt = c->sw_counts.as<int64_t>(16);
-  DRG_CUDA(cudaMemsetAsync(cnt, 0, 16 * sizeof(int64_t), c->stream));
+  //   per class  [15] wide bands  [16..19] bands listed for the 32-bit kernel
+  int64_t* cnt = c->sw_counts.as<int64_t>(20);
+  DRG_CUDA(cudaMemsetAsync(cnt, 0, 20 * sizeof(int64_t), c->stream));
   count_launch();
   k_count_fast_narrow<<<1, 1, 0, c->stream>>>(swks, n_bands, kb.wide, cnt);
-  TraceBand* tb = nullptr;
-  if (trace) {
-    int64_t* h = c->h_stage.as<int64_t>(2);
-    DRG_CUDA(cudaMemcpyAsync(h, cnt, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-    DRG_CUDA(cudaStreamSynchronize(c->stream));
-    n_fast = (uint64_t)h[0];
-    n_narrow = (uint64_t)h[1];
-    tb = c->tband.as<TraceBand>(n_bands);
-    DRG_CUDA(cudaMemsetAsync(tb, 0xFF, n_bands * sizeof(TraceBand), c->stream));  // score -1: not traced
-    if (n_fast > 0) {
-      // traceback: one warp per band (few, long bands)
-      const BandJobs bj = make_band_jobs(c, swos, swks, n_fast, bc, s.offsets, true);
-      SwBandArgs ba = band_args(bc, bj, qs, s, scr);
-      ba.trace = c->trace.as<uint2>(bj.trace_words + 8);  // the walk reads 8-word windows
-      ba.tband = tb;
-      cudaEvent_t e0 = log->event(), e1 = log->event();
-      DRG_CUDA(cudaEventRecord(e0, c->stream));
-      // each band's walk (gapped.rs:205-279) runs in the band kernel right
-      // after its DP
-      ba.walk.trace = ba.trace;
-      ba.walk.q_letters = qs.letters;
-      ba.walk.q_offsets = qs.offsets;
-      ba.walk.s_letters = s.letters;
-      ba.walk.s_offsets = s.offsets;
-      ba.walk.ops_off = d_ops_off;
-      ba.walk.rev = c->rev.as<uint8_t>((*h_ops_off)[n_bands] + 16);
-      ba.walk.ops = ops;
-      ba.walk.out = out;
-      ba.walk.exact_below = scr.max_score + 1;
-      launch_band_routes(ba, bj, true, c->stream);
-      DRG_CUDA(cudaEventRecord(e1, c->stream));
-      log->span(e0, e1, &st.ms_trace_kernel);
+  // ---- wide bands (positions [narrow, fast) of the sorted order): band-
+  // kernel jobs by route, then longest first
+  SwBandJob* jobs_u = c->band_jobs_u.as<SwBandJob>(n_bands);
+  SwBandJob* wjobs = c->band_jobs.as<SwBandJob>(n_bands);
+  uint64_t* jkey = c->bj_key.as<uint64_t>(n_bands);
+  uint64_t* jkey_s = c->bj_key_s.as<uint64_t>(n_bands);
+  uint32_t* jval = c->bj_val.as<uint32_t>(n_bands);
+  uint32_t* jval_s = c->bj_val_s.as<uint32_t>(n_bands);
+  count_launch();
+  k_band_jobs_dev<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(
+      swos, cnt, n_bands, bc, s.offsets, jobs_u, jkey, jval, reinterpret_cast<unsigned long long*>(cnt + 6));
+  const uint32_t* jorder =
+      dsort(c, jkey, jkey_s, jval, jval_s, n_bands, 0, kCostBits + 3, reinterpret_cast<const uint64_t*>(cnt + 15))
+          .vals;
+  count_launch();
+  k_gather_band_jobs<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(jobs_u, jorder, n_bands, wjobs,
+                                                                      cnt + 15);
+  // ---- narrow bands: warps of up to 32 bands of one group
+  uint32_t* gstart = c->idx.as<uint32_t>(n_bands + 1);
+  count_launch();
+  k_sw_group_start<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(swks, n_bands, gstart, cnt + 1);
+  cub_call(c, [&](void* t, size_t& b) {
+    return cub::DeviceScan::InclusiveScan(t, b, gstart, gstart, cub::Max(), (int64_t)n_bands, c->stream);
+  });
+  count_launch();
+  k_sw_task_flags<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(gstart, n_bands, flags, cnt + 1);
+  uint32_t* tstart = c->sel_idx.as<uint32_t>(n_bands + 1);
+  select_indices_dev(c, flags, n_bands, tstart, cnt + 2);
+  SwTask* tasks_u = c->sw_tasks_u.as<SwTask>(n_bands);
+  SwTask* tasks = c->sw_tasks.as<SwTask>(n_bands);
+  uint64_t* tkey = c->task_key.as<uint64_t>(n_bands);
+  uint64_t* tkey_s = c->task_key_s.as<uint64_t>(n_bands);
+  uint32_t* tval = c->task_val.as<uint32_t>(n_bands);
+  uint32_t* tval_s = c->task_val_s.as<uint32_t>(n_bands);
+  count_launch();
+  k_sw_fill_tasks<<<ceil_div(n_bands, 128), 128, 0, c->stream>>>(tstart, n_bands, swks, n_bands, kb.transposed,
+                                                                  swos, bc, s.offsets, tasks_u, tkey, tval,
+                                                                  cells_gpu, cnt + 2, cnt + 1);
+  // by width class, longest warps first within a class
+  const uint32_t* task_order =
+      dsort(c, tkey, tkey_s, tval, tval_s, n_bands, 0, kCostBits + 2, reinterpret_cast<const uint64_t*>(cnt + 2))
+          .vals;
+  count_launch();
+  k_gather_tasks<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(tasks_u, task_order, n_bands, tasks, cnt + 2);
+  count_launch();
+  k_task_bounds<<<1, 1, 0, c->stream>>>(tasks, n_bands, cnt + 3, cnt + 2);
+  count_launch();
+  k_task_steps<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(tasks, n_bands,
+                                                               reinterpret_cast<unsigned long long*>(cnt + 11),
+                                                               cnt + 2);
+  // ---- the one wait: every count the launches need
+  int64_t* h = c->h_stage.as<int64_t>(16);
+  DRG_CUDA(cudaMemcpyAsync(h, cnt, 16 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+  DRG_CUDA(cudaStreamSynchronize(c->stream));
+  n_fast = (uint64_t)h[0];
+  n_narrow = (uint64_t)h[1];
+  const uint64_t n_tasks = (uint64_t)h[2];
+  int64_t bounds[kSwClasses - 1] = {h[3], h[4], h[5]};
+  unsigned long long hmax[kSwClasses];
+  for (int k = 0; k < kSwClasses; ++k) hmax[k] = (unsigned long long)h[11 + k];
+  BandJobs wide;
+  wide.jobs = wjobs;
+  wide.n = n_fast - n_narrow;
+  wide.max_width = (int)h[6];
+  for (int k = 0; k < 4; ++k) wide.route_lo[k + 1] = wide.route_lo[k] + (uint64_t)h[7 + k];
+  // bands the packed kernels do not take, in the 32-bit kernel: the longest
+  // chains of the pass, so first, beside the packed classes
+  SysArgs xa = sys_args(bc, qs, s, scr);
+  xa.score = scores;
+  xa.best_row = best_row;
+  unsigned long long* n_sys = cells_gpu ? cells_gpu + 5 : nullptr;
+  if (n_fast == 0)
+    sys_scores(c, xa, c->sys_list, swos, 0, n_bands, nullptr, cnt + 16, n_sys, s.max_len, c->stream);
+  if (n_fast > 0) {
+    SwScoreArgs sa{};
+    sa.bands = bc;
+    sa.order = swos;
+    sa.tasks = tasks;
+    sa.q_letters = qs.dp_letters();
+    sa.q_offsets = qs.offsets;
+    sa.s_letters = s.dp_letters();
+    sa.s_offsets = s.offsets;
+    sa.gap_open = scr.gap_open;
+    sa.gap_extend = scr.gap_extend;
+    sa.score = scores;
+    sa.best_row = best_row;
+    sa.cells_eval = cells_gpu;
+    std::memcpy(sa.scores625, scr.scores, 625);
+    uint64_t lo[kSwClasses], hi[kSwClasses];
+    for (int k = 0; k < kSwClasses; ++k) {
+      lo[k] = k == 0 ? 0 : (uint64_t)bounds[k - 1];
+      hi[k] = k == kSwClasses - 1 ? n_tasks : (uint64_t)bounds[k];
     }
-  } else {
-    // ---- wide bands (positions [narrow, fast) of the sorted order): band-
-    // kernel jobs by route, then longest first
-    SwBandJob* jobs_u = c->band_jobs_u.as<SwBandJob>(n_bands);
-    SwBandJob* wjobs = c->band_jobs.as<SwBandJob>(n_bands);
-    uint64_t* jkey = c->bj_key.as<uint64_t>(n_bands);
-    uint64_t* jkey_s = c->bj_key_s.as<uint64_t>(n_bands);
-    uint32_t* jval = c->bj_val.as<uint32_t>(n_bands);
-    uint32_t* jval_s = c->bj_val_s.as<uint32_t>(n_bands);
-    count_launch();
-    k_band_jobs_dev<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(
-        swos, cnt, n_bands, bc, s.offsets, jobs_u, jkey, jval, reinterpret_cast<unsigned long long*>(cnt + 6));
-    const uint32_t* jorder =
-        dsort(c, jkey, jkey_s, jval, jval_s, n_bands, 0, kCostBits + 3, reinterpret_cast<const uint64_t*>(cnt + 15))
-            .vals;
-    count_launch();
-    k_gather_band_jobs<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(jobs_u, jorder, n_bands, wjobs, nullptr,
-                                                                        cnt + 15);
-    // ---- narrow bands: warps of up to 32 bands of one group
-    uint32_t* gstart = c->idx.as<uint32_t>(n_bands + 1);
-    count_launch();
-    k_sw_group_start<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(swks, n_bands, gstart, cnt + 1);
-    cub_call(c, [&](void* t, size_t& b) {
-      return cub::DeviceScan::InclusiveScan(t, b, gstart, gstart, cub::Max(), (int64_t)n_bands, c->stream);
-    });
-    count_launch();
-    k_sw_task_flags<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(gstart, n_bands, flags, cnt + 1);
-    uint32_t* tstart = c->sel_idx.as<uint32_t>(n_bands + 1);
-    select_indices_dev(c, flags, n_bands, tstart, cnt + 2);
-    SwTask* tasks_u = c->sw_tasks_u.as<SwTask>(n_bands);
-    SwTask* tasks = c->sw_tasks.as<SwTask>(n_bands);
-    uint64_t* tkey = c->task_key.as<uint64_t>(n_bands);
-    uint64_t* tkey_s = c->task_key_s.as<uint64_t>(n_bands);
-    uint32_t* tval = c->task_val.as<uint32_t>(n_bands);
-    uint32_t* tval_s = c->task_val_s.as<uint32_t>(n_bands);
-    count_launch();
-    k_sw_fill_tasks<<<ceil_div(n_bands, 128), 128, 0, c->stream>>>(tstart, n_bands, swks, n_bands, kb.transposed,
-                                                                    swos, bc, s.offsets, false, tasks_u, tkey, tval,
-                                                                    nullptr, cells_gpu, cnt + 2, cnt + 1);
-    // by width class, longest warps first within a class
-    const uint32_t* task_order =
-        dsort(c, tkey, tkey_s, tval, tval_s, n_bands, 0, kCostBits + 2, reinterpret_cast<const uint64_t*>(cnt + 2))
-            .vals;
-    count_launch();
-    k_gather_tasks<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(tasks_u, task_order, n_bands, tasks, cnt + 2);
-    count_launch();
-    k_task_bounds<<<1, 1, 0, c->stream>>>(tasks, n_bands, cnt + 3, cnt + 2);
-    count_launch();
-    k_task_steps<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(tasks, n_bands,
-                                                                 reinterpret_cast<unsigned long long*>(cnt + 11),
-                                                                 cnt + 2);
-    // ---- the one wait: every count the launches need
-    int64_t* h = c->h_stage.as<int64_t>(16);
-    DRG_CUDA(cudaMemcpyAsync(h, cnt, 16 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-    DRG_CUDA(cudaStreamSynchronize(c->stream));
-    n_fast = (uint64_t)h[0];
-    n_narrow = (uint64_t)h[1];
-    const uint64_t n_tasks = (uint64_t)h[2];
-    int64_t bounds[kSwClasses - 1] = {h[3], h[4], h[5]};
-    unsigned long long hmax[kSwClasses];
-    for (int k = 0; k < kSwClasses; ++k) hmax[k] = (unsigned long long)h[11 + k];
-    BandJobs wide;
-    wide.jobs = wjobs;
-    wide.n = n_fast - n_narrow;
-    wide.max_width = (int)h[6];
-    for (int k = 0; k < 4; ++k) wide.route_lo[k + 1] = wide.route_lo[k] + (uint64_t)h[7 + k];
-    if (n_fast > 0) {
-      SwScoreArgs sa{};
-      sa.bands = bc;
-      sa.order = swos;
-      sa.tasks = tasks;
-      sa.q_letters = qs.dp_letters();
-      sa.q_offsets = qs.offsets;
-      sa.s_letters = s.dp_letters();
-      sa.s_offsets = s.offsets;
-      sa.gap_open = scr.gap_open;
-      sa.gap_extend = scr.gap_extend;
-      sa.score = scores;
-      sa.best_row = best_row;
-      sa.cells_eval = cells_gpu;
-      std::memcpy(sa.scores625, scr.scores, 625);
-      uint64_t lo[kSwClasses], hi[kSwClasses];
-      for (int k = 0; k < kSwClasses; ++k) {
-        lo[k] = k == 0 ? 0 : (uint64_t)bounds[k - 1];
-        hi[k] = k == kSwClasses - 1 ? n_tasks : (uint64_t)bounds[k];
-      }
-      // The bulk class runs on the main stream; the wider classes and the wide
-      // bands run on the side stream, queued first so that the long warps start
-      // early and the pass ends on the bulk class's shortest tasks.
-      std::array<cudaEvent_t, 2 * kSwClasses + 3> ev;
-      for (auto& e : ev) e = log->event();
-      const int fork = 2 * kSwClasses, wide0 = fork + 1, wide1 = fork + 2;
-      DRG_CUDA(cudaEventRecord(ev[fork], c->stream));
-      DRG_CUDA(cudaStreamWaitEvent(c->side, ev[fork], 0));
-      auto launch_cls = [&](int cls) {
-        cudaStream_t sc = cls == 0 ? c->stream : c->side;
-        sa.task_lo = lo[cls];
-        sa.task_hi = hi[cls];
-        DRG_CUDA(cudaEventRecord(ev[2 * cls], sc));
-        if (hi[cls] > lo[cls]) {
-          launch_sw_class(sa, cls, sc);
-          st.sw_launches += 1;
-        }
-        DRG_CUDA(cudaEventRecord(ev[2 * cls + 1], sc));
-      };
-      DRG_CUDA(cudaEventRecord(ev[wide0], c->side));
-      if (wide.n > 0) {
-        SwBandArgs ba = band_args(bc, wide, qs, s, scr);
-        ba.score = scores;
-        ba.best_row = best_row;
-        launch_band_routes(ba, wide, false, c->side);
+    // The bulk class runs on the main stream; the wider classes and the wide
+    // bands run on the side stream, queued first so that the long warps start
+    // early and the pass ends on the bulk class's shortest tasks.
+    std::array<cudaEvent_t, 2 * kSwClasses + 3> ev;
+    for (auto& e : ev) e = log->event();
+    const int fork = 2 * kSwClasses, wide0 = fork + 1, wide1 = fork + 2;
+    DRG_CUDA(cudaEventRecord(ev[fork], c->stream));
+    DRG_CUDA(cudaStreamWaitEvent(c->side, ev[fork], 0));
+    auto launch_cls = [&](int cls) {
+      cudaStream_t sc = cls == 0 ? c->stream : c->side;
+      sa.task_lo = lo[cls];
+      sa.task_hi = hi[cls];
+      DRG_CUDA(cudaEventRecord(ev[2 * cls], sc));
+      if (hi[cls] > lo[cls]) {
+        launch_sw_class(sa, cls, sc);
         st.sw_launches += 1;
       }
-      DRG_CUDA(cudaEventRecord(ev[wide1], c->side));
-      for (int cls = kSwClasses - 1; cls >= 1; --cls) launch_cls(cls);
-      launch_cls(0);
-      const int side_end = 2 * 1 + 1;  // class 1 is the side stream's last launch
-      DRG_CUDA(cudaStreamWaitEvent(c->stream, ev[side_end], 0));
-      for (int k = 0; k < kSwClasses; ++k) {
-        st.sw_class_tasks[k] += hi[k] - lo[k];
-        if (hmax[k] > st.sw_class_max_steps[k]) st.sw_class_max_steps[k] = hmax[k];
-      }
-      st.sw_wide_bands += wide.n;
-      drg_run_stats* stp = &st;
-      log->later([ev, fork, wide0, wide1, side_end, stp] {
-        float cls_ms[kSwClasses], side_span = 0, wide_ms = 0;
-        for (int k = 0; k < kSwClasses; ++k) DRG_CUDA(cudaEventElapsedTime(&cls_ms[k], ev[2 * k], ev[2 * k + 1]));
-        DRG_CUDA(cudaEventElapsedTime(&side_span, ev[fork], ev[side_end]));
-        DRG_CUDA(cudaEventElapsedTime(&wide_ms, ev[wide0], ev[wide1]));
-        stp->ms_sw_kernel += cls_ms[0] > side_span ? cls_ms[0] : side_span;  // wall of the concurrent launches
-        for (int k = 0; k < kSwClasses; ++k) stp->ms_sw_class[k] += cls_ms[k];
-        stp->ms_sw_wide += wide_ms;
-      });
+      DRG_CUDA(cudaEventRecord(ev[2 * cls + 1], sc));
+    };
+    sys_scores(c, xa, c->sys_list, swos, n_fast, n_bands, nullptr, cnt + 16, n_sys, s.max_len, c->side);
+    DRG_CUDA(cudaEventRecord(ev[wide0], c->side));
+    if (wide.n > 0) {
+      SwBandArgs ba = band_args(bc, wide, qs, s, scr);
+      ba.score = scores;
+      ba.best_row = best_row;
+      launch_band_routes(ba, wide, c->side);
+      st.sw_launches += 1;
     }
+    DRG_CUDA(cudaEventRecord(ev[wide1], c->side));
+    for (int cls = kSwClasses - 1; cls >= 1; --cls) launch_cls(cls);
+    launch_cls(0);
+    const int side_end = 2 * 1 + 1;  // class 1 is the side stream's last launch
+    DRG_CUDA(cudaStreamWaitEvent(c->stream, ev[side_end], 0));
+    for (int k = 0; k < kSwClasses; ++k) {
+      st.sw_class_tasks[k] += hi[k] - lo[k];
+      if (hmax[k] > st.sw_class_max_steps[k]) st.sw_class_max_steps[k] = hmax[k];
+    }
+    st.sw_wide_bands += wide.n;
+    drg_run_stats* stp = &st;
+    log->later([ev, fork, wide0, wide1, side_end, stp] {
+      float cls_ms[kSwClasses], side_span = 0, wide_ms = 0;
+      for (int k = 0; k < kSwClasses; ++k) DRG_CUDA(cudaEventElapsedTime(&cls_ms[k], ev[2 * k], ev[2 * k + 1]));
+      DRG_CUDA(cudaEventElapsedTime(&side_span, ev[fork], ev[side_end]));
+      DRG_CUDA(cudaEventElapsedTime(&wide_ms, ev[wide0], ev[wide1]));
+      stp->ms_sw_kernel += cls_ms[0] > side_span ? cls_ms[0] : side_span;  // wall of the concurrent launches
+      for (int k = 0; k < kSwClasses; ++k) stp->ms_sw_class[k] += cls_ms[k];
+      stp->ms_sw_wide += wide_ms;
+    });
   }
-  // the exact kernel for the bands the packed kernel did not settle
+  // the bands whose packed best does not settle them
+  sys_scores(c, xa, c->sys_list_redo, swos, 0, n_fast, scores, cnt + 18, n_sys, s.max_len, c->stream);
+  if (!times) {  // a call of its own: its kernel times are read now
+    DRG_CUDA(cudaStreamSynchronize(c->stream));
+    own.resolve();
+  }
+}
+
+// Tracebacks of n bands: out[i] and band i's ops at d_ops_off[i] in ops
+// (n + m slots per band).  Every band takes the 32-bit kernel; the walk runs in
+// the band's own warp right after its DP.  The trace of as many bands as the
+// budget holds is in memory at once.
+void trace_bands(drg_ctx* c, const Band* bc, uint64_t n, const DevSeqs& qs, const DevSeqs& s, const Scoring& scr,
+                 ExactOut* out, uint32_t* ops, const uint64_t* d_ops_off, drg_run_stats& st, TimeLog* times) {
+  if (n == 0) return;
+  TimeLog own;
+  TimeLog* log = times ? times : &own;
+  uint64_t* key = c->bj_key.as<uint64_t>(n);
+  uint64_t* key_s = c->bj_key_s.as<uint64_t>(n);
+  uint32_t* val = c->bj_val.as<uint32_t>(n);
+  uint32_t* val_s = c->bj_val_s.as<uint32_t>(n);
+  SysJob* jobs = c->sys_jobs.as<SysJob>(n);
+  uint64_t* size = c->bj_size.as<uint64_t>(n + 1);
+  uint64_t* off = c->bj_off.as<uint64_t>(n + 1);
+  unsigned long long* count = c->bj_max.as<unsigned long long>(3);
+  DRG_CUDA(cudaMemsetAsync(count, 0, 3 * sizeof(unsigned long long), c->stream));
   count_launch();
-  k_exact_flags<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(swos, n_fast, n_bands, scores, tb,
-                                                                scr.max_score + 1, flags);
-  uint32_t* ex_pos = c->sel_idx.as<uint32_t>(n_bands + 1);
-  const uint64_t n_ex = select_indices(c, flags, n_bands, ex_pos, d_count);
-  st.exact_bands += n_ex;
-  if (n_ex > 0) {
-    uint32_t* ex_idx = c->idx.as<uint32_t>(n_ex);
-    Band* ex_b = c->ex_bands.as<Band>(n_ex);
-    count_launch();
-    k_gather_positions<<<ceil_div(n_ex, 256), 256, 0, c->stream>>>(ex_pos, swos, n_ex, bc, ex_idx, ex_b);
-    std::vector<uint32_t> bidx;
-    std::vector<Band> all_b;
-    fetch_n(c, bidx, ex_idx, n_ex);
-    fetch_n(c, all_b, ex_b, n_ex);
-    std::vector<ExactJob> jobs(n_ex);
-    uint64_t soff = 0;
-    for (uint64_t k = 0; k < n_ex; ++k) {
-      const Band& b = all_b[k];
-      ExactJob& j = jobs[k];
-      j.q = qs.letters + (*qs.h_offsets)[b.target] + b.q0;
-      j.s = s.letters + (*s.h_offsets)[b.subject];
-      j.n = b.n;
-      j.m = (uint32_t)((*s.h_offsets)[b.subject + 1] - (*s.h_offsets)[b.subject]);
-      j.d0 = b.d0;
-      j.d1 = b.d1;
-      j.scratch_off = soff;
-      j.ops_off = trace ? (*h_ops_off)[bidx[k]] : 0;
-      soff += exact_scratch_bytes(j.n, j.m, j.d0, j.d1, trace);
-    }
-    ExactJob* dj = c->exact_jobs.as<ExactJob>(n_ex);
-    ExactOut* dout = c->exact_out.as<ExactOut>(n_ex);
-    uint8_t* scratch = c->exact_scratch.as<uint8_t>(soff);
-    DRG_CUDA(cudaMemcpyAsync(dj, jobs.data(), n_ex * sizeof(ExactJob), cudaMemcpyHostToDevice, c->stream));
-    launch_sw_exact_with_matrix(dj, n_ex, scr.gap_open, scr.gap_extend, trace, scratch, trace ? ops : nullptr, dout,
-                                scr.scores, c->stream);
-    count_launch();
-    if (trace) k_scatter_exact<<<ceil_div(n_ex, 256), 256, 0, c->stream>>>(ex_idx, dout, n_ex, out);
-    else k_scatter_scores<<<ceil_div(n_ex, 256), 256, 0, c->stream>>>(ex_idx, dout, n_ex, scores);
-    DRG_CUDA(cudaGetLastError());
+  k_sys_jobs<<<ceil_div(n, 256), 256, 0, c->stream>>>(bc, n, s.offsets, key, val, count);
+  const uint32_t* idx = dsort(c, key, key_s, val, val_s, n, 0, kCostBits + 2).vals;
+  count_launch();
+  k_sys_sizes<<<ceil_div(n + 1, 256), 256, 0, c->stream>>>(idx, n, bc, s.offsets, jobs, size);
+  cub_call(c, [&](void* t, size_t& b) {
+    return cub::DeviceScan::ExclusiveSum(t, b, size, off, (int64_t)n + 1, c->stream);
+  });
+  count_launch();
+  k_sys_offsets<<<ceil_div(n, 256), 256, 0, c->stream>>>(jobs, off, n);
+  // jobs per route and the trace bytes, in one wait
+  unsigned long long* h = c->h_stage.as<unsigned long long>(4);
+  DRG_CUDA(cudaMemcpyAsync(h, count, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
+  DRG_CUDA(cudaMemcpyAsync(h + 3, off + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
+  DRG_CUDA(cudaStreamSynchronize(c->stream));
+  const uint64_t lo[4] = {0, h[0], h[0] + h[1], h[0] + h[1] + h[2]}, total = h[3];
+  SysArgs a = sys_args(bc, qs, s, scr);
+  a.jobs = jobs;
+  a.ops_off = d_ops_off;
+  a.ops = ops;
+  a.out = out;
+  if (h[2] > 0) sys_wrap(c, a, s.max_len);
+  constexpr uint64_t kBudget = 24ull << 30;
+  std::vector<uint64_t> hoff;
+  if (total > kBudget) fetch_n(c, hoff, off, n + 1);
+  cudaEvent_t e0 = log->event(), e1 = log->event();
+  uint8_t* base = nullptr;
+  if (hoff.empty()) base = c->trace.as<uint8_t>(total + 16);
+  DRG_CUDA(cudaEventRecord(e0, c->stream));
+  // Each route's longest band bounds its launch (its chain of rows) and the
+  // other SMs idle, so the routes run side by side: one stream each.  (One
+  // after the other: 414 + 394 + 290 us for the 4,182 bands of the 1,000-query
+  // sensitive search.)  Trace memory that is reused keeps them in order.
+  cudaStream_t streams[3] = {c->stream, c->stream, c->stream};
+  if (hoff.empty()) {
+    streams[1] = c->side2;
+    streams[2] = c->side;
   }
+  for (int r = 2; r >= 0; --r) {
+    if (lo[r + 1] == lo[r]) continue;
+    if (streams[r] != c->stream) DRG_CUDA(cudaStreamWaitEvent(streams[r], e0, 0));
+    for (uint64_t k = lo[r]; k < lo[r + 1];) {
+      uint64_t e = lo[r + 1];
+      uint64_t from = 0;
+      if (!hoff.empty()) {  // as many jobs as the budget holds, one at least
+        from = hoff[k];
+        e = k + 1;
+        while (e < lo[r + 1] && hoff[e + 1] - from <= kBudget) ++e;
+        base = c->trace.as<uint8_t>(std::max(hoff[e] - from, kBudget) + 16);
+      }
+      a.trace = base;
+      a.trace_base = from;
+      a.lo = k;
+      a.hi = e;
+      launch_sys_trace(a, r, streams[r]);
+      k = e;
+    }
+  }
+  for (int r = 1; r <= 2; ++r) {
+    if (lo[r + 1] == lo[r] || streams[r] == c->stream) continue;
+    cudaEvent_t done = log->event();
+    DRG_CUDA(cudaEventRecord(done, streams[r]));
+    DRG_CUDA(cudaStreamWaitEvent(c->stream, done, 0));
+  }
+  DRG_CUDA(cudaEventRecord(e1, c->stream));
+  log->span(e0, e1, &st.ms_trace_kernel);
   if (!times) {  // a call of its own: its kernel times are read now
     DRG_CUDA(cudaStreamSynchronize(c->stream));
     own.resolve();
@@ -904,6 +915,7 @@ struct Search {
   int64_t* d_count = nullptr;
   // [0] xdrops [1] cells_ref [2] computed [3] cells_gpu [4] lane cells [5] issued cells
   // [6] transposed bands [7] valid reference seeds of chunks enumerated without an index
+  // [8] bands scored in 32-bit lanes
   unsigned long long* d_counters = nullptr;
   TimeLog times;  // stage times, read after the search's last wait
 
@@ -1519,11 +1531,10 @@ void Search::process_hits(uint64_t pass_id) {
   // ---- banded SW scores
   tm.start();
   int32_t* scores = c->scores.as<int32_t>(n_bands);
-  DevSeqs qs{q->letters, q->offsets, &q->h_offsets, q->score_letters};
-  DevSeqs ss{db->letters, db->offsets, &db->h_offsets, db->score_letters};
+  DevSeqs qs{q->letters, q->offsets, &q->h_offsets, q->score_letters, q->max_len};
+  DevSeqs ss{db->letters, db->offsets, &db->h_offsets, db->score_letters, db->max_len};
   int32_t* best_row = c->best_row.as<int32_t>(n_bands);
-  run_bands(c, bc, n_bands, qs, ss, sc, false, scores, best_row, nullptr, nullptr, nullptr, nullptr, st, d_count,
-            d_counters + 3, &times);
+  score_bands(c, bc, n_bands, qs, ss, sc, scores, best_row, st, d_counters + 3, &times);
   tm.stop(&st.ms_sw);
   flags = c->flags.as<uint8_t>(n_bands + 1);  // scratch buffers may have been regrown
   // ---- E-value gate and band walk
@@ -1555,7 +1566,7 @@ void Search::process_hits(uint64_t pass_id) {
   int64_t* dsel = c->pass_counts.as<int64_t>(8) + 6;
   select_indices_dev(c, flags, n_bands, sel, dsel);
   Band* gb = c->sel_bands.as<Band>(n_bands);
-  int32_t* gs = reinterpret_cast<int32_t*>(c->exact_out.as<uint8_t>(n_bands * 5 + 16));
+  int32_t* gs = reinterpret_cast<int32_t*>(c->sel_records.as<uint8_t>(n_bands * 5 + 16));
   uint8_t* gst = reinterpret_cast<uint8_t*>(gs + n_bands);
   count_launch();
   k_gather_bands_dev<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(sel, n_bands, dsel, bc, scores, best_row, state,
@@ -1700,13 +1711,12 @@ void Search::finish(drg_result* out) {
     Band* db_ = c->sel_bands.as<Band>(nj);
     uint64_t* doff = c->ops_off.as<uint64_t>(nj + 1);
     ExactOut* dout = c->trace_out.as<ExactOut>(nj);
-    uint32_t* dops = c->exact_ops.as<uint32_t>(ops_off[nj] + 1);
+    uint32_t* dops = c->trace_ops.as<uint32_t>(ops_off[nj] + 1);
     DRG_CUDA(cudaMemcpyAsync(db_, sb.data(), nj * sizeof(Band), cudaMemcpyHostToDevice, c->stream));
     DRG_CUDA(cudaMemcpyAsync(doff, ops_off.data(), (nj + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, c->stream));
-    DevSeqs qs{q->letters, q->offsets, &q->h_offsets, q->score_letters};
-    DevSeqs ss{db->letters, db->offsets, &db->h_offsets, db->score_letters};
-    run_bands(c, db_, nj, qs, ss, sc, true, nullptr, nullptr, dout, dops, doff, &ops_off, st, d_count,
-              nullptr, &times);
+    DevSeqs qs{q->letters, q->offsets, &q->h_offsets, q->score_letters, q->max_len};
+    DevSeqs ss{db->letters, db->offsets, &db->h_offsets, db->score_letters, db->max_len};
+    trace_bands(c, db_, nj, qs, ss, sc, dout, dops, doff, st, &times);
     // only the ops the alignments use come back (each band has n + m slots)
     uint64_t* cnt = c->ops_cnt.as<uint64_t>(nj + 1);
     uint64_t* coff = c->ops_coff.as<uint64_t>(nj + 1);
@@ -1817,7 +1827,7 @@ void Search::run(drg_result* out) {
   }
   finish(out);
   total.stop(&st.ms_total);
-  unsigned long long cnt[8];
+  unsigned long long cnt[9];
   uint32_t sort_err = 0;
   DRG_CUDA(cudaMemcpyAsync(cnt, d_counters, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream));
   DRG_CUDA(cudaMemcpyAsync(&sort_err, c->sort_err.as<uint32_t>(1), sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
@@ -1831,6 +1841,7 @@ void Search::run(drg_result* out) {
   st.dp_cells_lane = cnt[4];
   st.dp_cells_issued = cnt[5];
   st.sw_transposed_bands = cnt[6];
+  st.exact_bands = cnt[8];
   st.ref_seeds += cnt[7];  // valid reference seeds counted on the device
   st.seed_shapes = shapes.size();
   st.query_blocks = query_blocks;

@@ -32,11 +32,6 @@ __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
   asm("max.s16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
-__device__ __forceinline__ uint32_t max2_relu(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("max.s16x2.relu %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
 // Maximum of two pairs of non-negative 16-bit integers below 0x7C00 on the
 // FMA pipe: such bit patterns are zero, subnormal or finite positive halves,
 // ordered like the integers, and max.f16x2 (no flush to zero) returns one of
@@ -75,14 +70,12 @@ __device__ __forceinline__ uint32_t next_residue(Lane& L, int c) {
   return res;
 }
 
-template <bool TR>
 struct Regs {
   uint32_t H[kPairs], Hm[kPairs], F[kPairs];
   uint32_t E7;        // E of pair 7 at the previous step
   uint32_t htop_old;  // top H of the previous step (D operand of pair 0)
   uint32_t res_prev;  // subject residue of the previous column
   uint32_t rowmax[kPairs];            // per row of the strip: max H so far
-  uint32_t rowcol[TR ? kPairs : 1];   // trace mode: first column of that max
 };
 
 __device__ __forceinline__ int lo16(uint32_t x) { return (int)(int16_t)(x & 0xFFFFu); }

@@ -4,9 +4,8 @@
 // out-of-band H counting as 0 on the diagonal step and E/F starting at the
 // band edges, strict comparisons for every tie -- so scores, the first
 // row-major maximum, trace bits and the traceback walk are the reference's.
-// It runs on the HSPs that survive the E-value gate and the per-query cut,
-// and on the rare bands the packed score kernel does not take (width < 17,
-// possible 16-bit overflow, best score not above the matrix's largest).
+// The no-allocation entry point uses it: its scratch per job is what callers
+// size their calls by (searches and the other entry points run sw_sys.cu).
 #include "kernels.h"
 
 namespace drg {

@@ -41,8 +41,7 @@
 // exactly.  Cells left or right of the band in the first/last 16 steps of
 // a strip are masked: their H does not count and they pass -inf-like E/F.
 //
-// The traceback of the HSPs that pass the gate runs in sw_band.cu (one warp
-// per band) and sw_walk.cuh.
+// The traceback of the HSPs that pass the gate runs in sw_sys.cu.
 #include "kernels.h"
 #include "sw_common.cuh"
 
