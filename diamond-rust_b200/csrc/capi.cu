@@ -52,7 +52,40 @@ namespace {
   }                                                    \
   return DRG_OK;
 
-// Device copy of a sequence set with its letter -> sequence map.
+// Device memory of one stage call, from the context's stream-ordered pool: a
+// cudaMalloc / cudaFree pair of a few MB takes 0.1-10 ms here (it maps memory
+// and waits for the device), more than most calls compute.  A call of 400,000
+// X-drop jobs spent 2.7 of its 4.6 ms there, 3,000 tracebacks 2.1 of 4.8.
+// The pool keeps freed blocks for the next call; a call gives back what it
+// holds beyond kPoolKeep (PoolTrim).
+template <typename T>
+T* call_alloc(drg_ctx* c, size_t n) {
+  void* p = nullptr;
+  DRG_CUDA(cudaMallocFromPoolAsync(&p, n * sizeof(T), c->pool, c->stream));
+  return static_cast<T*>(p);
+}
+void call_free(drg_ctx* c, void* p) {
+  if (p) cudaFreeAsync(p, c->stream);
+}
+constexpr uint64_t kPoolKeep = 2ull << 30;
+// Declared before a call's arrays, so that it runs after they are freed (the
+// call has waited for its work by then).
+struct PoolTrim {
+  drg_ctx* ctx;
+  explicit PoolTrim(drg_ctx* c) : ctx(c) {}
+  ~PoolTrim() {
+    uint64_t held = 0, used = 0;
+    if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        held <= kPoolKeep)
+      return;
+    cudaStreamSynchronize(ctx->stream);  // the frees of this call
+    if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+        held > used + kPoolKeep)
+      cudaMemPoolTrimTo(ctx->pool, used + kPoolKeep);
+  }
+};
+
+// Device copy of a sequence set.
 struct Seqs {
   uint8_t* letters = nullptr;
   uint8_t* score_letters = nullptr;  // clamped to 24 for the DP kernels, when some code is above 24
@@ -63,12 +96,12 @@ struct Seqs {
   Seqs() = default;
   Seqs(const Seqs&) = delete;
   ~Seqs() {
-    cudaFree(letters);
-    cudaFree(score_letters);
-    cudaFree(offsets);
-    cudaFree(owner);
+    for (void* p : {(void*)letters, (void*)score_letters, (void*)offsets, (void*)owner}) call_free(ctx, p);
   }
-  void upload(drg_ctx* c, const uint8_t* l, const uint64_t* off, uint64_t count) {
+  drg_ctx* ctx = nullptr;
+  // with_owner: the letter -> sequence map too (seed enumeration reads it)
+  void upload(drg_ctx* c, const uint8_t* l, const uint64_t* off, uint64_t count, bool with_owner = false) {
+    ctx = c;
     n = count;
     h_offsets.assign(off, off + n + 1);
     total = off[n];
@@ -76,15 +109,17 @@ struct Seqs {
       if (off[i + 1] < off[i]) throw Error(DRG_ERR_INVALID, "offsets must be non-decreasing");
       max_len = std::max(max_len, off[i + 1] - off[i]);
     }
-    DRG_CUDA(cudaMalloc(&letters, total + 64));
-    DRG_CUDA(cudaMalloc(&offsets, (n + 1) * sizeof(uint64_t)));
-    DRG_CUDA(cudaMalloc(&owner, (total + 1) * sizeof(uint32_t)));
+    letters = call_alloc<uint8_t>(c, total + 64);
+    offsets = call_alloc<uint64_t>(c, n + 1);
     DRG_CUDA(cudaMemsetAsync(letters + total, 25, 64, c->stream));
     if (total) DRG_CUDA(cudaMemcpyAsync(letters, l, total, cudaMemcpyHostToDevice, c->stream));
     DRG_CUDA(cudaMemcpyAsync(offsets, off, (n + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, c->stream));
-    launch_letter_owner(offsets, n, 0, total, owner, c->stream);
+    if (with_owner) {
+      owner = call_alloc<uint32_t>(c, total + 1);
+      launch_letter_owner(offsets, n, 0, total, owner, c->stream);
+    }
     if (letters_above_24(c, letters, total)) {
-      DRG_CUDA(cudaMalloc(&score_letters, total + 64));
+      score_letters = call_alloc<uint8_t>(c, total + 64);
       DRG_CUDA(cudaMemsetAsync(score_letters + total, 25, 64, c->stream));
       launch_clamp_letters(letters, total, score_letters, c->stream);
     }
@@ -95,10 +130,10 @@ struct Seqs {
 template <typename T>
 struct DevArr {
   T* p = nullptr;
-  DevArr() = default;
-  explicit DevArr(size_t n) { DRG_CUDA(cudaMalloc(&p, (n ? n : 1) * sizeof(T))); }
+  drg_ctx* ctx = nullptr;
+  DevArr(drg_ctx* c, size_t n) : p(call_alloc<T>(c, n ? n : 1)), ctx(c) {}
   DevArr(const DevArr&) = delete;
-  ~DevArr() { cudaFree(p); }
+  ~DevArr() { call_free(ctx, p); }
 };
 
 template <typename F>
@@ -257,14 +292,15 @@ int drg_radix_sort(drg_ctx* c, void* keys, int32_t key_bytes, uint32_t* vals, ui
       end_bit > 8 * key_bytes)
     return DRG_ERR_INVALID;
   API_BEGIN(c)
+  PoolTrim trim(c);
   if (n >= (1ull << 32)) throw Error(DRG_ERR_INVALID, "radix sort: at most 2^32 - 1 keys");
   // with the count on the device, the buffers hold a larger capacity (tiles
   // past the count are never taken), as when a sort follows the kernel that
   // counted its input
   const uint64_t cap = count_on_device ? 2 * n + 5000 : n;
-  DevArr<uint8_t> k(cap * key_bytes), ka(cap * key_bytes);
-  DevArr<uint32_t> v(vals ? cap : 0), va(vals ? cap : 0);
-  DevArr<uint64_t> dn(1);
+  DevArr<uint8_t> k(c, cap * key_bytes), ka(c, cap * key_bytes);
+  DevArr<uint32_t> v(c, vals ? cap : 0), va(c, vals ? cap : 0);
+  DevArr<uint64_t> dn(c, 1);
   if (n) DRG_CUDA(cudaMemcpyAsync(k.p, keys, n * key_bytes, cudaMemcpyHostToDevice, c->stream));
   if (n && vals) DRG_CUDA(cudaMemcpyAsync(v.p, vals, n * 4, cudaMemcpyHostToDevice, c->stream));
   DRG_CUDA(cudaMemcpyAsync(dn.p, &n, sizeof(uint64_t), cudaMemcpyHostToDevice, c->stream));
@@ -295,6 +331,7 @@ int drg_seed_build(drg_ctx* c, const uint8_t* letters, const uint64_t* offsets, 
                    drg_seed_entry** out, uint64_t* n_out) {
   if (!c || !offsets || !shape_code || !out || !n_out) return DRG_ERR_INVALID;
   API_BEGIN(c)
+  PoolTrim trim(c);
   ShapeCode sh;
   if (!parse_shape(shape_code, &sh))
     throw Error(DRG_ERR_INVALID, std::string("invalid seed shape \"") + shape_code + "\": expected only 0/1");
@@ -316,11 +353,11 @@ int drg_seed_build(drg_ctx* c, const uint8_t* letters, const uint64_t* offsets, 
   p.shape_shift = 48;  // one shape: the key is the shape's packed key
   p.request_shift = 56;
   Seqs s;
-  s.upload(c, letters, offsets, n_seqs);
+  s.upload(c, letters, offsets, n_seqs, true);
   upload_seed_params(t, p, c->slot, c->stream);
   const uint64_t N = s.total;
-  DevArr<uint64_t> k(N), ks(N);
-  DevArr<uint32_t> v(N), vs(N);
+  DevArr<uint64_t> k(c, N), ks(c, N);
+  DevArr<uint32_t> v(c, N), vs(c, N);
   launch_seed_enum(s.letters, s.offsets, s.owner, 0, s.total, 1, k.p, v.p, c->slot, c->stream);
   const SortResult<uint64_t> sr = radix_sort<uint64_t>(k.p, ks.p, v.p, vs.p, N, nullptr, 0, 64, c->sort_tmp,
                                                        c->sort_err.as<uint32_t>(1), c->stream);
@@ -352,6 +389,7 @@ int drg_seed_join(drg_ctx* c, const drg_seed_entry* q, uint64_t nq, const drg_se
                   uint64_t n_targets, uint64_t max_expand, drg_seed_hit** out, uint64_t* n_out) {
   if (!c || !out || !n_out || (nq && !q) || (nr && !r)) return DRG_ERR_INVALID;
   API_BEGIN(c)
+  PoolTrim trim(c);
   *out = nullptr;
   *n_out = 0;
   for (uint64_t i = 0; i < nq; ++i)
@@ -370,11 +408,11 @@ int drg_seed_join(drg_ctx* c, const drg_seed_entry* q, uint64_t nq, const drg_se
     rpos[i] = r[i].pos;
     rid[i] = (uint32_t)i;
   }
-  DevArr<uint64_t> dqk(nq), drk(nr), ukeys(nq + 1);
-  DevArr<uint32_t> dqseq(nq), dqpos(nq), drseq(nr), drpos(nr), dqid(nq), drid(nr), ucount(nq + 1), ustart(nq + 1),
-      rlo(nq + 1), rcnt(nq + 1);
-  DevArr<uint64_t> uhits(nq + 2), uoff(nq + 2);
-  DevArr<int64_t> cnt(2);
+  DevArr<uint64_t> dqk(c, nq), drk(c, nr), ukeys(c, nq + 1);
+  DevArr<uint32_t> dqseq(c, nq), dqpos(c, nq), drseq(c, nr), drpos(c, nr), dqid(c, nq), drid(c, nr), ucount(c, nq + 1), ustart(c, nq + 1),
+      rlo(c, nq + 1), rcnt(c, nq + 1);
+  DevArr<uint64_t> uhits(c, nq + 2), uoff(c, nq + 2);
+  DevArr<int64_t> cnt(c, 2);
   auto up = [&](void* d, const void* h, size_t bytes) {
     if (bytes) DRG_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c->stream));
   };
@@ -407,7 +445,7 @@ int drg_seed_join(drg_ctx* c, const drg_seed_entry* q, uint64_t nq, const drg_se
     uint64_t n_hits = 0;
     DRG_CUDA(cudaMemcpyAsync(&n_hits, uoff.p + n_runs, 8, cudaMemcpyDeviceToHost, c->stream));
     sync(c);
-    DevArr<uint32_t> h4(4 * n_hits);
+    DevArr<uint32_t> h4(c, 4 * n_hits);
     JoinExpandArgs a{};
     a.run_hit_off = uoff.p;
     a.run_qstart = ustart.p;
@@ -447,6 +485,7 @@ int drg_xdrop_batch(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, uint64_t 
                     int32_t xdrop, drg_segment* out) {
   if (!c || !qo || !so || (n && (!jobs || !out))) return DRG_ERR_INVALID;
   API_BEGIN(c)
+  PoolTrim trim(c);
   Scoring sc;
   std::string err;
   if (!make_scoring(matrix, -1, -1, &sc, &err)) throw Error(DRG_ERR_INVALID, err);
@@ -459,8 +498,8 @@ int drg_xdrop_batch(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, uint64_t 
   qs.upload(c, ql, qo, nq);
   ss.upload(c, sl, so, ns);
   upload_score_matrix(sc.scores, c->slot, c->stream);
-  DevArr<drg_xdrop_job> dj(n);
-  DevArr<drg_segment> dout(n);
+  DevArr<drg_xdrop_job> dj(c, n);
+  DevArr<drg_segment> dout(c, n);
   if (n) DRG_CUDA(cudaMemcpyAsync(dj.p, jobs, n * sizeof(drg_xdrop_job), cudaMemcpyHostToDevice, c->stream));
   launch_xdrop_jobs(dj.p, n, qs.letters, qs.offsets, ss.letters, ss.offsets, xdrop, dout.p, c->slot, c->stream);
   if (n) DRG_CUDA(cudaMemcpyAsync(out, dout.p, n * sizeof(drg_segment), cudaMemcpyDeviceToHost, c->stream));
@@ -473,6 +512,7 @@ int drg_extend_span_batch(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, uin
                           int32_t go, int32_t ge, drg_aligned* out, uint32_t** ops, uint64_t* n_ops) {
   if (!c || !qo || !so || !ops || !n_ops || (n && (!jobs || !out))) return DRG_ERR_INVALID;
   API_BEGIN(c)
+  PoolTrim trim(c);
   Scoring sc;
   std::string err;
   if (!make_scoring(matrix, go, ge, &sc, &err)) throw Error(DRG_ERR_INVALID, err);
@@ -497,10 +537,10 @@ int drg_extend_span_batch(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, uin
     ops_off[i + 1] = ops_off[i] + b.n + (so[j.subject + 1] - so[j.subject]);
   }
   const uint64_t ooff = ops_off[n];
-  DevArr<Band> db_(n);
-  DevArr<ExactOut> dout(n);
-  DevArr<uint32_t> dops(ooff + 1);
-  DevArr<uint64_t> doff(n + 1);
+  DevArr<Band> db_(c, n);
+  DevArr<ExactOut> dout(c, n);
+  DevArr<uint32_t> dops(c, ooff + 1);
+  DevArr<uint64_t> doff(c, n + 1);
   if (n) {
     DRG_CUDA(cudaMemcpyAsync(db_.p, hb.data(), n * sizeof(Band), cudaMemcpyHostToDevice, c->stream));
     DRG_CUDA(cudaMemsetAsync(dout.p, 0, n * sizeof(ExactOut), c->stream));
@@ -508,15 +548,22 @@ int drg_extend_span_batch(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, uin
   DRG_CUDA(cudaMemcpyAsync(doff.p, ops_off.data(), (n + 1) * 8, cudaMemcpyHostToDevice, c->stream));
   drg_run_stats st{};
   trace_bands(c, db_.p, n, qs.view(), ss.view(), sc, dout.p, dops.p, doff.p, st);
+  // only the ops in use come back (each job has n + m slots), in job order
   std::vector<ExactOut> eo(n);
-  std::vector<uint32_t> hops(ooff);
-  if (n) DRG_CUDA(cudaMemcpyAsync(eo.data(), dout.p, n * sizeof(ExactOut), cudaMemcpyDeviceToHost, c->stream));
-  if (ooff) DRG_CUDA(cudaMemcpyAsync(hops.data(), dops.p, ooff * 4, cudaMemcpyDeviceToHost, c->stream));
-  sync(c);
+  const CompactOps co = compact_ops(c, dops.p, doff.p, dout.p, n, ooff);
   uint64_t total = 0;
-  for (auto& e : eo) total += e.score > 0 ? e.n_ops : 0;
+  if (n) DRG_CUDA(cudaMemcpyAsync(eo.data(), dout.p, n * sizeof(ExactOut), cudaMemcpyDeviceToHost, c->stream));
+  if (n) DRG_CUDA(cudaMemcpyAsync(&total, co.off + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
+  sync(c);
   uint32_t* o = (uint32_t*)std::malloc(sizeof(uint32_t) * (total + 1));
   if (!o) throw Error(DRG_ERR_OOM, "host allocation failed");
+  try {
+    if (total) DRG_CUDA(cudaMemcpyAsync(o, co.ops, total * 4, cudaMemcpyDeviceToHost, c->stream));
+    sync(c);
+  } catch (...) {
+    std::free(o);
+    throw;
+  }
   uint64_t k = 0;
   for (uint64_t i = 0; i < n; ++i) {
     drg_aligned& a = out[i];
@@ -542,7 +589,6 @@ int drg_extend_span_batch(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, uin
     a.gaps = eo[i].gaps;
     a.length = eo[i].length;
     a.n_ops = eo[i].n_ops;
-    std::memcpy(o + k, hops.data() + ops_off[i], eo[i].n_ops * 4);
     k += eo[i].n_ops;
   }
   *ops = o;
@@ -555,6 +601,7 @@ int drg_extend_span_scores(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, ui
                            int32_t go, int32_t ge, int32_t* scores, drg_run_stats* stats) {
   if (!c || !qo || !so || (n && (!jobs || !scores))) return DRG_ERR_INVALID;
   API_BEGIN(c)
+  PoolTrim trim(c);
   Scoring sc;
   std::string err;
   if (!make_scoring(matrix, go, ge, &sc, &err)) throw Error(DRG_ERR_INVALID, err);
@@ -576,10 +623,10 @@ int drg_extend_span_scores(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, ui
     b.q0 = 0;
     b.n = (uint32_t)(qo[j.query + 1] - qo[j.query]);
   }
-  DevArr<Band> db_(n);
-  DevArr<int32_t> ds(n);
+  DevArr<Band> db_(c, n);
+  DevArr<int32_t> ds(c, n);
   // evaluated, lane, issued cells, transposed bands, -, bands in 32-bit lanes
-  DevArr<unsigned long long> cells(6);
+  DevArr<unsigned long long> cells(c, 6);
   DRG_CUDA(cudaMemsetAsync(cells.p, 0, 6 * sizeof(unsigned long long), c->stream));
   if (n) DRG_CUDA(cudaMemcpyAsync(db_.p, hb.data(), n * sizeof(Band), cudaMemcpyHostToDevice, c->stream));
   drg_run_stats st{};

@@ -142,6 +142,15 @@ void score_bands(drg_ctx* c, const Band* bands, uint64_t n_bands, const DevSeqs&
 void trace_bands(drg_ctx* c, const Band* bands, uint64_t n, const DevSeqs& q, const DevSeqs& s, const Scoring& sc,
                  ExactOut* out, uint32_t* ops, const uint64_t* d_ops_off, drg_run_stats& st,
                  TimeLog* times = nullptr);
+// The ops that n traced bands use (band k's n_ops from its slots at ops_off[k]
+// of ops, `slots` in all), back to back in band order, and their offsets
+// (n + 1).  No wait; the context owns the arrays until its next call.
+struct CompactOps {
+  const uint32_t* ops = nullptr;
+  const uint64_t* off = nullptr;
+};
+CompactOps compact_ops(drg_ctx* c, const uint32_t* ops, const uint64_t* ops_off, const ExactOut* out, uint64_t n,
+                       uint64_t slots);
 // Whole-path search over resident inputs (pipeline.cu).
 void search(drg_ctx* ctx, const drg_db* db, const drg_batch* b, const drg_search_config* cfg, drg_result* out);
 // Whether n device letters hold a code above 24; syncs the context's stream.

@@ -793,6 +793,27 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   }
 }
 
+CompactOps compact_ops(drg_ctx* c, const uint32_t* ops, const uint64_t* ops_off, const ExactOut* out, uint64_t n,
+                       uint64_t slots) {
+  CompactOps r;
+  if (n == 0) return r;
+  uint64_t* cnt = c->ops_cnt.as<uint64_t>(n + 1);
+  uint64_t* off = c->ops_coff.as<uint64_t>(n + 1);
+  count_launch();
+  k_ops_count<<<ceil_div(n + 1, 256), 256, 0, c->stream>>>(out, n, cnt);
+  cub_call(c, [&](void* t, size_t& b) {
+    return cub::DeviceScan::ExclusiveSum(t, b, cnt, off, (int64_t)n + 1, c->stream);
+  });
+  // (the slot total bounds the ops in use)
+  uint32_t* dst = c->ops_compact.as<uint32_t>(slots + 1);
+  count_launch();
+  k_compact_ops<<<ceil_div(n, 128), 128, 0, c->stream>>>(ops, ops_off, out, off, n, dst);
+  DRG_CUDA(cudaGetLastError());
+  r.ops = dst;
+  r.off = off;
+  return r;
+}
+
 // Tracebacks of n bands: out[i] and band i's ops at d_ops_off[i] in ops
 // (n + m slots per band).  Every band takes the 32-bit kernel; the walk runs in
 // the band's own warp right after its DP.  The trace of as many bands as the
@@ -1717,28 +1738,18 @@ void Search::finish(drg_result* out) {
     DevSeqs qs{q->letters, q->offsets, &q->h_offsets, q->score_letters, q->max_len};
     DevSeqs ss{db->letters, db->offsets, &db->h_offsets, db->score_letters, db->max_len};
     trace_bands(c, db_, nj, qs, ss, sc, dout, dops, doff, st, &times);
-    // only the ops the alignments use come back (each band has n + m slots)
-    uint64_t* cnt = c->ops_cnt.as<uint64_t>(nj + 1);
-    uint64_t* coff = c->ops_coff.as<uint64_t>(nj + 1);
-    count_launch();
-    k_ops_count<<<ceil_div(nj + 1, 256), 256, 0, c->stream>>>(dout, nj, cnt);
-    cub_call(c, [&](void* t, size_t& b) {
-      return cub::DeviceScan::ExclusiveSum(t, b, cnt, coff, (int64_t)nj + 1, c->stream);
-    });
-    // compacted into a buffer of the bands' slot total (an upper bound of the
-    // ops used); the records and the used count come back in one wait
-    uint32_t* cops = c->ops_compact.as<uint32_t>(ops_off[nj] + 1);
-    count_launch();
-    k_compact_ops<<<ceil_div(nj, 128), 128, 0, c->stream>>>(dops, doff, dout, coff, nj, cops);
+    // only the ops the alignments use come back (each band has n + m slots);
+    // the records and the used count in one wait
+    const CompactOps co = compact_ops(c, dops, doff, dout, nj, ops_off[nj]);
     uint8_t* hst = c->h_stage.as<uint8_t>(nj * sizeof(ExactOut) + 16);
     DRG_CUDA(cudaMemcpyAsync(hst, dout, nj * sizeof(ExactOut), cudaMemcpyDeviceToHost, c->stream));
-    DRG_CUDA(cudaMemcpyAsync(hst + nj * sizeof(ExactOut), coff + nj, sizeof(uint64_t), cudaMemcpyDeviceToHost,
+    DRG_CUDA(cudaMemcpyAsync(hst + nj * sizeof(ExactOut), co.off + nj, sizeof(uint64_t), cudaMemcpyDeviceToHost,
                              c->stream));
     DRG_CUDA(cudaStreamSynchronize(c->stream));
     eo.assign(reinterpret_cast<const ExactOut*>(hst), reinterpret_cast<const ExactOut*>(hst) + nj);
     uint64_t n_used = 0;
     std::memcpy(&n_used, hst + nj * sizeof(ExactOut), sizeof(uint64_t));
-    fetch_n(c, ops_all, cops, n_used);
+    fetch_n(c, ops_all, co.ops, n_used);
     tm.stop(&st.ms_trace);
   }
   auto t1 = std::chrono::steady_clock::now();
