@@ -10,7 +10,10 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <unordered_map>
+
+#include <sys/mman.h>
 
 #include "context.h"
 #include "kernels.h"
@@ -154,6 +157,32 @@ void sync(drg_ctx* c) {
   if (*h) {
     DRG_CUDA(cudaMemsetAsync(d_err, 0, sizeof(uint32_t), c->stream));
     throw Error(DRG_ERR_TIMEOUT, "radix sort: a tile's bounded wait for an earlier tile gave up");
+  }
+}
+
+// Host memory of a result (released with std::free).  Results of tens of MB
+// are new pages on every call: on huge pages the copy into them faults once
+// per 2 MB instead of once per 4 KB.
+void* result_alloc(size_t bytes) {
+  constexpr size_t kHuge = 2 << 20;
+  void* p = nullptr;
+  if (bytes >= 4 * kHuge) {
+    p = std::aligned_alloc(kHuge, (bytes + kHuge - 1) / kHuge * kHuge);
+    if (p) madvise(p, bytes, MADV_HUGEPAGE);
+  } else {
+    p = std::malloc(bytes);
+  }
+  if (!p) throw Error(DRG_ERR_OOM, "host allocation failed");
+  return p;
+}
+// Waits for `bytes` at d copied into a result, which is freed if that fails.
+void fetch_result(drg_ctx* c, void* o, const void* d, size_t bytes) {
+  try {
+    if (bytes) DRG_CUDA(cudaMemcpyAsync(o, d, bytes, cudaMemcpyDeviceToHost, c->stream));
+    sync(c);
+  } catch (...) {
+    std::free(o);
+    throw;
   }
 }
 
@@ -356,30 +385,35 @@ int drg_seed_build(drg_ctx* c, const uint8_t* letters, const uint64_t* offsets, 
   s.upload(c, letters, offsets, n_seqs, true);
   upload_seed_params(t, p, c->slot, c->stream);
   const uint64_t N = s.total;
-  DevArr<uint64_t> k(c, N), ks(c, N);
+  // The sort covers the bits of the shape's largest key and one more, so that
+  // "no seed" (all ones) sorts last; keys that then fit 32 bits are sorted as
+  // 32-bit words (2.26M letters, weight 8: 255 -> 110 us).
+  double mx = 1.0;
+  for (int k = 0; k < sh.weight; ++k) mx *= (double)red.size;
+  int bits = 64;
+  if (mx < 4.0e18) {
+    uint64_t top = 1;
+    for (int k = 0; k < sh.weight; ++k) top *= (uint64_t)red.size;
+    bits = bits_for(top - 1) + 1;
+  }
+  DevArr<drg_seed_entry> entries(c, N);
+  DevArr<uint64_t> n_valid(c, 1);
+  DevArr<uint64_t> k(c, bits <= 32 ? (N + 1) / 2 : N), ks(c, bits <= 32 ? (N + 1) / 2 : N);
   DevArr<uint32_t> v(c, N), vs(c, N);
-  launch_seed_enum(s.letters, s.offsets, s.owner, 0, s.total, 1, k.p, v.p, c->slot, c->stream);
-  const SortResult<uint64_t> sr = radix_sort<uint64_t>(k.p, ks.p, v.p, vs.p, N, nullptr, 0, 64, c->sort_tmp,
-                                                       c->sort_err.as<uint32_t>(1), c->stream);
-  std::vector<uint64_t> hk(N);
-  std::vector<uint32_t> hv(N);
-  if (N) {
-    DRG_CUDA(cudaMemcpyAsync(hk.data(), sr.keys, N * 8, cudaMemcpyDeviceToHost, c->stream));
-    DRG_CUDA(cudaMemcpyAsync(hv.data(), sr.vals, N * 4, cudaMemcpyDeviceToHost, c->stream));
-  }
-  sync(c);
+  auto build = [&](auto* keys, auto* keys_alt) {
+    using K = std::remove_pointer_t<decltype(keys)>;
+    launch_seed_enum(s.letters, s.offsets, s.owner, 0, s.total, 1, keys, v.p, c->slot, c->stream);
+    const SortResult<K> r = radix_sort<K>(keys, keys_alt, v.p, vs.p, N, nullptr, 0, bits, c->sort_tmp,
+                                          c->sort_err.as<uint32_t>(1), c->stream);
+    launch_seed_entries(r.keys, r.vals, N, s.owner, s.offsets, base, entries.p, n_valid.p, c->stream);
+  };
+  if (bits <= 32) build(reinterpret_cast<uint32_t*>(k.p), reinterpret_cast<uint32_t*>(ks.p));
+  else build(k.p, ks.p);
   uint64_t nv = 0;
-  while (nv < N && hk[nv] != kNoSeed) ++nv;
-  drg_seed_entry* o = (drg_seed_entry*)std::malloc(sizeof(drg_seed_entry) * (nv + 1));
-  if (!o) throw Error(DRG_ERR_OOM, "host allocation failed");
-  for (uint64_t i = 0; i < nv; ++i) {
-    uint64_t g = hv[i];
-    uint64_t seq = (uint64_t)(std::upper_bound(s.h_offsets.begin(), s.h_offsets.end(), g) - s.h_offsets.begin()) - 1;
-    while (seq + 1 < s.h_offsets.size() && s.h_offsets[seq + 1] <= g) ++seq;  // empty sequences
-    o[i].key = hk[i];
-    o[i].seq = base + (uint32_t)seq;
-    o[i].pos = (uint32_t)(g - s.h_offsets[seq]);
-  }
+  if (N) DRG_CUDA(cudaMemcpyAsync(&nv, n_valid.p, sizeof nv, cudaMemcpyDeviceToHost, c->stream));
+  sync(c);
+  drg_seed_entry* o = static_cast<drg_seed_entry*>(result_alloc(sizeof(drg_seed_entry) * (nv + 1)));
+  fetch_result(c, o, entries.p, nv * sizeof(drg_seed_entry));
   *out = o;
   *n_out = nv;
   API_END(c)
@@ -555,15 +589,8 @@ int drg_extend_span_batch(drg_ctx* c, const uint8_t* ql, const uint64_t* qo, uin
   if (n) DRG_CUDA(cudaMemcpyAsync(eo.data(), dout.p, n * sizeof(ExactOut), cudaMemcpyDeviceToHost, c->stream));
   if (n) DRG_CUDA(cudaMemcpyAsync(&total, co.off + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
   sync(c);
-  uint32_t* o = (uint32_t*)std::malloc(sizeof(uint32_t) * (total + 1));
-  if (!o) throw Error(DRG_ERR_OOM, "host allocation failed");
-  try {
-    if (total) DRG_CUDA(cudaMemcpyAsync(o, co.ops, total * 4, cudaMemcpyDeviceToHost, c->stream));
-    sync(c);
-  } catch (...) {
-    std::free(o);
-    throw;
-  }
+  uint32_t* o = static_cast<uint32_t*>(result_alloc(sizeof(uint32_t) * (total + 1)));
+  fetch_result(c, o, co.ops, total * 4);
   uint64_t k = 0;
   for (uint64_t i = 0; i < n; ++i) {
     drg_aligned& a = out[i];

@@ -49,6 +49,13 @@ void launch_seed_enum_filtered(const uint8_t* letters, const uint64_t* offsets, 
                                int log2_bits, uint32_t* keys, uint32_t* vals, unsigned long long* counts, int slot,
                                cudaStream_t st);
 constexpr uint64_t kNoSeed = ~0ull;
+// Sorted seeds to seed::build's records; *n_valid = the valid ones (n > 0).
+void launch_seed_entries(const uint64_t* keys, const uint32_t* vals, uint64_t n, const uint32_t* owner,
+                         const uint64_t* offsets, uint32_t base, drg_seed_entry* out, uint64_t* n_valid,
+                         cudaStream_t st);
+void launch_seed_entries(const uint32_t* keys, const uint32_t* vals, uint64_t n, const uint32_t* owner,
+                         const uint64_t* offsets, uint32_t base, drg_seed_entry* out, uint64_t* n_valid,
+                         cudaStream_t st);
 constexpr uint32_t kMaxRequests = 65535;  // request ids of one batch
 
 // A block of the query batch: the targets whose letters lie in [lo, hi).  A
