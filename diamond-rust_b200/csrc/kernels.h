@@ -135,13 +135,20 @@ struct JoinExpandArgs {
   const uint64_t* r_offsets;    // subject offsets
   HitKeyLayout layout;
   uint64_t* hit_keys;
-  // entries mode: payloads index seq/pos arrays
-  const uint32_t* q_seq;
-  const uint32_t* q_pos;
-  const uint32_t* r_seq;
-  const uint32_t* r_pos;
-  uint32_t* hits4;  // 4 x u32 per hit
+  // entries mode (q_entries set; no q_vals / r_vals): hit_keys when set, else
+  // hits4, 4 x u32 per hit
+  const drg_seed_entry* q_entries;
+  const drg_seed_entry* r_entries;
+  uint32_t* hits4;
 };
+// Largest sequence index and position of a list of seed entries.
+struct EntryMax {
+  uint32_t seq, pos;
+};
+// The entries' keys, and their maxima (*top zeroed by the caller).
+void launch_split_entries(const drg_seed_entry* e, uint64_t n, uint64_t* keys, EntryMax* top, cudaStream_t st);
+// Hit keys back to (query, qpos, subject, spos) records.
+void launch_unpack_hits(const uint64_t* keys, uint64_t n, const HitKeyLayout& L, uint32_t* hits4, cudaStream_t st);
 void launch_join_expand(const JoinExpandArgs& a, cudaStream_t st);
 // coarse[j] (j in [0, ceil(n_hits >> shift)]) = the run holding hit j << shift
 // (the last run for j past the hits): narrows each hit's run search.

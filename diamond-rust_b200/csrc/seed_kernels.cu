@@ -597,26 +597,76 @@ __global__ void k_join_expand(JoinExpandArgs a) {
   uint32_t rc = a.run_rcount[u];
   uint64_t qi = a.run_qstart[u] + k / rc;
   uint64_t ri = a.run_rlo[u] + k % rc;
-  if (a.hit_keys) {
-    uint32_t qg = a.q_vals[qi], rg = a.r_vals[ri];
-    uint32_t t = a.q_owner[qg];
-    uint32_t s = a.r_owner[rg];
-    int64_t qpos = (int64_t)qg - (int64_t)a.q_offsets[t];
-    int64_t spos = (int64_t)rg - (int64_t)a.r_offsets[s];
-    const HitKeyLayout& L = a.layout;
-    uint64_t key = (uint64_t)(t - L.t_base);
-    key = (key << L.sb) | (uint64_t)s;
-    key = (key << L.db) | (uint64_t)(qpos - spos + L.doff);
-    key = (key << L.pb) | (uint64_t)spos;
-    a.hit_keys[h] = key;
+  uint32_t t, s;
+  int64_t qpos, spos;
+  if (a.q_entries) {
+    const drg_seed_entry qe = a.q_entries[qi], re = a.r_entries[ri];
+    t = qe.seq;
+    s = re.seq;
+    qpos = qe.pos;
+    spos = re.pos;
+    if (!a.hit_keys) {
+      reinterpret_cast<uint4*>(a.hits4)[h] = make_uint4(qe.seq, qe.pos, re.seq, re.pos);
+      return;
+    }
   } else {
-    uint32_t qe = a.q_vals[qi], re = a.r_vals[ri];
-    uint32_t* o = a.hits4 + 4 * h;
-    o[0] = a.q_seq[qe];
-    o[1] = a.q_pos[qe];
-    o[2] = a.r_seq[re];
-    o[3] = a.r_pos[re];
+    const uint32_t qg = a.q_vals[qi], rg = a.r_vals[ri];
+    t = a.q_owner[qg];
+    s = a.r_owner[rg];
+    qpos = (int64_t)qg - (int64_t)a.q_offsets[t];
+    spos = (int64_t)rg - (int64_t)a.r_offsets[s];
   }
+  const HitKeyLayout& L = a.layout;
+  uint64_t key = (uint64_t)(t - L.t_base);
+  key = (key << L.sb) | (uint64_t)s;
+  key = (key << L.db) | (uint64_t)(qpos - spos + L.doff);
+  key = (key << L.pb) | (uint64_t)spos;
+  a.hit_keys[h] = key;
+}
+
+// One thread per entry: a 16-byte load, its key stored, the maxima folded per
+// warp.
+__global__ void k_split_entries(const drg_seed_entry* __restrict__ e, uint64_t n, uint64_t* __restrict__ keys,
+                                EntryMax* __restrict__ top) {
+  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  uint32_t seq = 0, pos = 0;
+  if (i < n) {
+    const uint4 v = reinterpret_cast<const uint4*>(e)[i];
+    keys[i] = (uint64_t)v.y << 32 | v.x;
+    seq = v.z;
+    pos = v.w;
+  }
+  seq = __reduce_max_sync(0xFFFFFFFFu, seq);
+  pos = __reduce_max_sync(0xFFFFFFFFu, pos);
+  if ((threadIdx.x & 31) == 0) {  // most warps read a maximum already reached
+    if (seq > *(volatile uint32_t*)&top->seq) atomicMax(&top->seq, seq);
+    if (pos > *(volatile uint32_t*)&top->pos) atomicMax(&top->pos, pos);
+  }
+}
+void launch_split_entries(const drg_seed_entry* e, uint64_t n, uint64_t* keys, EntryMax* top, cudaStream_t st) {
+  if (n == 0) return;
+  count_launch();
+  k_split_entries<<<ceil_div(n, 256), 256, 0, st>>>(e, n, keys, top);
+  DRG_CUDA(cudaGetLastError());
+}
+
+__global__ void k_unpack_hits(const uint64_t* __restrict__ keys, uint64_t n, HitKeyLayout L,
+                              uint32_t* __restrict__ hits4) {
+  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint64_t key = keys[i];
+  // (every field's width is below 64)
+  const uint64_t spos = key & ((1ull << L.pb) - 1);
+  const int64_t diag = (int64_t)((key >> L.pb) & ((1ull << L.db) - 1)) - L.doff;
+  const uint32_t s = (uint32_t)((key >> (L.pb + L.db)) & ((1ull << L.sb) - 1));
+  const uint32_t t = (uint32_t)(key >> (L.pb + L.db + L.sb));
+  reinterpret_cast<uint4*>(hits4)[i] = make_uint4(t, (uint32_t)(diag + (int64_t)spos), s, (uint32_t)spos);
+}
+void launch_unpack_hits(const uint64_t* keys, uint64_t n, const HitKeyLayout& L, uint32_t* hits4, cudaStream_t st) {
+  if (n == 0) return;
+  count_launch();
+  k_unpack_hits<<<ceil_div(n, 256), 256, 0, st>>>(keys, n, L, hits4);
+  DRG_CUDA(cudaGetLastError());
 }
 
 void launch_join_expand(const JoinExpandArgs& a, cudaStream_t st) {

@@ -26,3 +26,37 @@ def test_seed_entries(ctx, orc, shape, reduction):
 @pytest.mark.parametrize("seqs", [[], [np.zeros(0, np.uint8)] * 3, [np.full(2, 3, np.uint8)]])
 def test_no_seeds(ctx, seqs):
     assert len(ctx.seed_build(seqs, "1111", 0, base=0, cut=0.0)) == 0
+
+
+def _entries(r, keys, n, seqs, poss):
+    e = np.zeros(n, dtype=[("key", "u8"), ("seq", "u4"), ("pos", "u4")])
+    e["key"] = np.sort(r.choice(keys, n))
+    e["seq"] = r.choice(seqs, n)
+    e["pos"] = r.choice(poss, n)
+    return e
+
+
+@pytest.mark.parametrize("seqs,poss", [
+    ([0], [0]),                                    # every field zero bits wide
+    ([0, 1, 70], [0, 1, 5, 1000]),
+    ([3, 2 ** 20], [0, 2 ** 20 - 1]),              # exactly 64 bits: 2 + 21 + 21 + 20
+    ([3, 2 ** 20], [0, 2 ** 20]),                  # 66
+    ([7, 2 ** 32 - 1], [0, 2 ** 31, 2 ** 32 - 1]),  # 99
+])
+def test_join_records(ctx, orc, seqs, poss):
+    r = np.random.Generator(np.random.PCG64(len(seqs) + len(poss)))
+    keys = np.array([0, 3, 4, 2 ** 40, 2 ** 64 - 1], np.uint64)
+    q = _entries(r, keys, 40, [0, 2, 3], poss)
+    e = _entries(r, keys, 90, seqs, poss)
+    for cap in (4096, 150):
+        assert ctx.seed_join(q, e, 4, cap) == orc.seed_join(q, e, 4, cap)
+
+
+def test_join_rejects_a_target_out_of_range(ctx):
+    import drgpu
+    r = np.random.Generator(np.random.PCG64(1))
+    q = _entries(r, np.array([1], np.uint64), 3, [4], [0])
+    with pytest.raises(drgpu.DrgError) as e:
+        ctx.seed_join(q, q, 4)
+    assert e.value.code == 1
+    assert ctx.seed_join(q[:0], q, 4) == [] and ctx.seed_join(q, q[:0], 5) == []
