@@ -244,12 +244,16 @@ int drg_ctx_create(int device, drg_ctx** out) {
       // the side stream carries the long warps of the score pass: its blocks
       // are dispatched ahead of the bulk class's whenever an SM frees up
       cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
-      cudaStreamCreateWithPriority(&c->side2, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
+      std::any_of(std::begin(c->lanes), std::end(c->lanes),
+                  [&](cudaStream_t& s) {
+                    return cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, prio_high) != cudaSuccess;
+                  }) ||
       cudaMemPoolCreate(&c->pool, &props) != cudaSuccess ||
       cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, (void*)&keep) != cudaSuccess) {
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->side) cudaStreamDestroy(c->side);
-    if (c->side2) cudaStreamDestroy(c->side2);
+    for (cudaStream_t s : c->lanes)
+      if (s) cudaStreamDestroy(s);
     if (c->pool) cudaMemPoolDestroy(c->pool);
     release_slot(c->slot);
     delete c;
@@ -273,10 +277,10 @@ void drg_ctx_destroy(drg_ctx* c) {
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
   cudaStreamSynchronize(c->side);
-  cudaStreamSynchronize(c->side2);
+  for (cudaStream_t s : c->lanes) cudaStreamSynchronize(s);
   cudaStreamDestroy(c->stream);
   cudaStreamDestroy(c->side);
-  cudaStreamDestroy(c->side2);
+  for (cudaStream_t s : c->lanes) cudaStreamDestroy(s);
   cudaMemPoolDestroy(c->pool);  // released once the last resident buffer is freed
   release_slot(c->slot);
   delete c;

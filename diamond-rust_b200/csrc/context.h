@@ -20,7 +20,9 @@ struct drg_ctx {
   int slot = -1;                // constant-memory bank of this context (kConstSlots of them)
   cudaStream_t stream = nullptr;
   cudaStream_t side = nullptr;  // concurrent launches (wide-band classes)
-  cudaStream_t side2 = nullptr;  // a third one (traceback routes)
+  // more of them: each route of the score and traceback passes has its own, so
+  // that the launches' longest bands run beside one another
+  cudaStream_t lanes[5] = {};
   cudaMemPool_t pool = nullptr;  // resident databases and batches (kept across calls)
   std::string err;
   // seed stage

@@ -298,11 +298,13 @@ struct SwBandArgs {
 };
 size_t sw_band_smem(int max_width);
 void launch_sw_band(SwBandArgs a, int max_width, cudaStream_t st);
-// Bands by width: route 0 (W <= 134), 1 (<= 271), 2 (<= 559) run in groups
-// of 8, 16, 32 lanes with rotating strips; route 3 (wider) in the block
-// kernel.  max_width matters for route 3 only.
+// Bands of the score pass that do not share a warp 32 at a time, by width:
+// routes 0, 1, 2 run two per warp with rotating strips of 4, 8, 16 rows per
+// lane (k_sys_pair, W <= 151, 271, 511); route 3 (wider) in the block kernel.
+// max_width matters for route 3 only.
+__host__ __device__ constexpr int sys_rot_max(int R);
 __host__ __device__ inline int sw_band_route(int width) {
-  return width > 559 ? 3 : (width <= 134 ? 0 : (width <= 271 ? 1 : 2));
+  return width <= sys_rot_max(4) ? 0 : (width <= sys_rot_max(8) ? 1 : (width <= sys_rot_max(16) ? 2 : 3));
 }
 void launch_sw_band_route(const SwBandArgs& a, int route, int max_width, cudaStream_t st);
 

@@ -143,6 +143,9 @@ struct SwKeyBits {
 // inverse orders longest first; the order only schedules, so costs saturate.
 constexpr int kCostBits = 21;  // 2M column steps: above any warp but the rarest, so the keys sort in 3 passes
 constexpr uint64_t kCostMax = (1ull << kCostBits) - 1;
+// Transposed warps (full, their rows a short subject) stay up to this chain.
+constexpr uint64_t kTransposedChain = 4096;
+constexpr uint32_t kSwNoClass = 0xFFFFFFFFu;  // width of a warp that was given up
 constexpr int kGroupShift = 24, kWidthShift = 13, kKeyLo = 13;
 
 // DP rows [rs, re] of a band with at least one in-matrix cell: rows are the
@@ -208,7 +211,7 @@ struct SwTune {
 };
 SwTune sw_tune(const drg_ctx* c, const Scoring& scr) {
   SwTune t{c->tuning.sw_wide_min_width, c->tuning.sw_min_packed_width, c->tuning.sw_transpose};
-  if (scr.gap_open + scr.gap_extend > kSwMaxOpenCost) t.wide_min = t.min_packed;  // no packed-kernel bands
+  if (scr.gap_open + scr.gap_extend > kSwMaxOpenCost) t.wide_min = t.min_packed;  // no bands 32 to a warp
   return t;
 }
 
@@ -235,15 +238,57 @@ __device__ __forceinline__ SwRoute sw_route(const Band& b, const uint64_t* s_off
          (r.te - r.ts + 16) / 16 < (r.re - r.rs + 16) / 16;
   return r;
 }
-// Bands per subject that would run with fewer strips transposed; each such
-// band draws a ticket (its arrival order, which varies from run to run: the
-// grouping of bands into warps does not change any score).
+// Which warps of the packed kernel are given up.  A warp of k_sw runs 32
+// bands, one per lane, strip after strip: steps = strips x (W + 16), over the
+// union of its bands' rows and its widest band, at the same cost for 1 band as
+// for 32.  The lane kernel (k_sys_pair) takes two bands per warp, a step per
+// row and a quarter.  A warp's bands go there
+//  - when its steps alone outlast the pass: the pass takes about sum(chain) /
+//    32 steps over 148 x 12 warps, a step 530 cycles with twelve warps on an
+//    SM and 200 to 350 with few, so steps > sum(chain) / 35,000.  (61 queries,
+//    sensitive, whole search: 3.65 / 3.58 / 3.7 / 4.1 ms at 22,000 / 30,000 /
+//    40,000 / 55,000, and 5.5 ms with every warp kept.)
+//  - when the lane kernel runs its bands in less than half its steps, as it
+//    does for a warp of fewer than some 10 bands (pair_cost, in k_sw steps,
+//    from 1.36M bands in full warps, where that kernel takes 1.53 times as
+//    long).  20,000 queries default: 34.1 ms without this rule, 32.3, 31.9,
+//    33.1 and 35.2 ms at 0.3, 0.5, 0.8 and 0.95 of the steps: beside full
+//    warps the lane kernel is slower than alone.
+constexpr uint64_t kChainShare = 35000;
+constexpr float kPairShare = 0.5f;
+__device__ __forceinline__ float pair_cost(int rows, int W) {
+  return W <= sys_rot_max(4) ? 0.26f * (1.25f * rows + W)
+                             : W <= sys_rot_max(8) ? 0.41f * (1.125f * rows + W) : 0.7f * (1.06f * rows + W);
+}
+
+__device__ __forceinline__ uint64_t sw_chain(int64_t rs, int64_t re, uint64_t W) {
+  return (uint64_t)((re - rs + 16) / 16) * (W + 16);
+}
+
+// Per subject, the bands that would run with fewer strips transposed, each
+// with a ticket (its arrival order, which varies from run to run: the grouping
+// of bands into warps does not change any score); the sum of all chains.
 __global__ void k_sw_tr_count(const Band* bands, uint64_t n, const uint64_t* s_offsets, int max_score, SwTune tn,
-                              uint32_t* count, uint32_t* ticket) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const Band b = bands[i];
-  ticket[i] = sw_route(b, s_offsets, max_score, tn).tr ? atomicAdd(count + b.subject, 1u) : 0xFFFFFFFFu;
+                              uint32_t* count, uint32_t* ticket, unsigned long long* chain_sum) {
+  __shared__ unsigned long long sums[8];
+  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  unsigned long long chain = 0;
+  if (i < n) {
+    const Band b = bands[i];
+    const SwRoute r = sw_route(b, s_offsets, max_score, tn);
+    const uint64_t W = (uint64_t)(b.d1 - b.d0 + 1);
+    if (r.fast && !r.wide) chain = r.tr ? sw_chain(r.ts, r.te, W) : sw_chain(r.rs, r.re, W);
+    ticket[i] = r.tr ? atomicAdd(count + b.subject, 1u) : 0xFFFFFFFFu;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) chain += __shfl_xor_sync(0xFFFFFFFFu, chain, o);
+  if (lane == 0) sums[threadIdx.x >> 5] = chain;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) chain += sums[w];
+    if (chain) atomicAdd(chain_sum, chain);
+  }
 }
 
 // The two sort keys of the score pass: the key above, and rows (first-row
@@ -260,7 +305,7 @@ __global__ void k_sw_keys(const Band* bands, uint64_t n, const uint64_t* s_offse
   const SwRoute r = sw_route(b, s_offsets, max_score, tn);
   // A subject's transposed bands form warps of their own: only whole warps
   // of them are transposed, the rest stay with their query windows.
-  const bool tr = r.tr && tr_count && rows[i] < (tr_count[b.subject] & ~31u);
+  const bool tr = r.tr && rows[i] < (tr_count[b.subject] & ~31u);
   const int64_t rs = tr ? r.ts : r.rs, re = tr ? r.te : r.re;
   const uint64_t group = tr ? (kb.transposed | ((uint64_t)b.subject << kGroupShift))
                             : ((((uint64_t)b.target << 16) | b.q0) << kGroupShift);
@@ -276,7 +321,29 @@ __global__ void k_gather_keys(const uint64_t* keys, const uint32_t* idx, uint64_
   uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (k < n) out[k] = keys[idx[k]];
 }
-__device__ __forceinline__ int64_t band_first_row(const Band& b) { return b.d0 + 1 > 1 ? b.d0 + 1 : 1; }
+
+// The lane kernel's job of band i in slot `at`, with its sort key: by kernel
+// route, then longest first.  Returns the route.
+__device__ __forceinline__ int band_job(uint32_t i, uint64_t at, const Band* bands, const uint64_t* s_offsets,
+                                        SwBandJob* jobs, uint64_t* sort_key, uint32_t* sort_val) {
+  const Band b = bands[i];
+  const int64_t m = (int64_t)(s_offsets[b.subject + 1] - s_offsets[b.subject]);
+  int64_t rs, re;
+  band_rows(b, m, false, &rs, &re);
+  if (re < rs) re = rs;
+  const uint32_t W = (uint32_t)(b.d1 - b.d0 + 1);
+  SwBandJob j;
+  j.band = i;
+  j.row_first = (uint32_t)rs;
+  j.n_strips = (uint32_t)((re - rs + 16) / 16);
+  j.pad = W;
+  jobs[at] = j;
+  const int route = sw_band_route((int)W);
+  const uint64_t cost = (uint64_t)(j.n_strips - 1) * 19ull + W + 16ull;
+  sort_key[at] = ((uint64_t)route << kCostBits) | (kCostMax - (cost < kCostMax ? cost : kCostMax));
+  sort_val[at] = (uint32_t)at;
+  return route;
+}
 
 // Task heads: first band of each (target, window) group and every 32nd after
 // (a group's bands are in width order, so a warp's widths are close).
@@ -293,7 +360,9 @@ __global__ void k_sw_task_flags(const uint32_t* gstart, uint64_t n, uint8_t* f, 
 __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const uint64_t* keys, uint64_t n_fast,
                                 uint64_t transposed_key, const uint32_t* order, const Band* bands,
                                 const uint64_t* s_offsets, SwTask* tasks, uint64_t* sort_key, uint32_t* sort_val,
-                                unsigned long long* cells_gpu, const int64_t* d_n_tasks, const int64_t* d_n_fast) {
+                                unsigned long long* cells_gpu, const int64_t* d_n_tasks, const int64_t* d_n_fast,
+                                const unsigned long long* chain_sum, SwBandJob* jobs, uint64_t* job_key,
+                                uint32_t* job_val, unsigned long long* n_jobs, unsigned long long* route) {
   uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (d_n_tasks) n_tasks = (uint64_t)*d_n_tasks;
   if (d_n_fast) n_fast = (uint64_t)*d_n_fast;
@@ -305,6 +374,7 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
   int64_t row_first = INT64_MAX, row_last = 0;
   uint32_t wmin = 0xFFFFFFFFu, wmax = 0;
   uint64_t lane_cells = 0;
+  float cost = 0.0f;  // the lane kernel's, in steps of this warp
   while (cnt < 32 && s + cnt < n_fast && (keys[s + cnt] >> kGroupShift) == grp) {
     const uint64_t key = keys[s + cnt];
     const Band b = bands[order[s + cnt]];
@@ -317,6 +387,7 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
     if (w < wmin) wmin = w;
     if (w > wmax) wmax = w;
     lane_cells += (uint64_t)((re - rs + 16) / 16) * 16ull * (w + 16ull);
+    cost += pair_cost((int)(re - rs + 1), (int)w);
     ++cnt;
   }
   if (row_last < row_first) row_last = row_first;
@@ -331,10 +402,30 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
   k.pad = 0;
   tasks[t] = k;
   const uint64_t steps = (uint64_t)k.n_strips * (wmax + 16ull);
+  sort_val[t] = (uint32_t)t;
+  // Given up (see kChainShare); not a transposed warp of a short subject, whose
+  // bands would have more rows there.
+  const uint64_t limit = *chain_sum / kChainShare;
+  if (transposed ? steps > (limit > kTransposedChain ? limit : kTransposedChain)
+                 : (steps > limit || cost < kPairShare * (float)steps)) {
+    const uint64_t at = atomicAdd(n_jobs, (unsigned long long)cnt);
+    uint32_t n_route[4] = {0, 0, 0, 0};
+    for (uint32_t x = 0; x < cnt; ++x) {
+      const int r = band_job(order[s + x], at + x, bands, s_offsets, jobs, job_key, job_val);
+#pragma unroll
+      for (int y = 0; y < 4; ++y) n_route[y] += r == y;
+    }
+    atomicMax(route, (unsigned long long)wmax);
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+      if (n_route[y]) atomicAdd(route + 1 + y, (unsigned long long)n_route[y]);
+    tasks[t].width = kSwNoClass;
+    sort_key[t] = (uint64_t)kSwClasses << kCostBits;  // after every class
+    return;
+  }
   const int cls = sw_class_of(wmax);
   // class, then longest first (a scheduling order: 21 bits of steps, saturated, suffice)
   sort_key[t] = ((uint64_t)cls << kCostBits) | (kCostMax - (steps < kCostMax ? steps : kCostMax));
-  sort_val[t] = (uint32_t)t;
   if (cells_gpu) {
     atomicAdd(cells_gpu + 1, (unsigned long long)lane_cells);  // evaluated cells: counted by k_sw
     if (transposed) atomicAdd(cells_gpu + 3, (unsigned long long)cnt);
@@ -346,18 +437,19 @@ __global__ void k_gather_tasks(const SwTask* in, const uint32_t* idx, uint64_t n
   if (t < n && (!d_n || t < (uint64_t)*d_n)) out[t] = in[idx[t]];
 }
 
-// First task of classes 1, 2 and 3 (tasks are sorted by class).
+// First task of classes 1, 2 and 3, and of the warps given up (tasks are
+// sorted by class).
 __global__ void k_task_bounds(const SwTask* tasks, uint64_t n, int64_t* out, const int64_t* d_n) {
   if (d_n) n = (uint64_t)*d_n;
-  for (int c = 0; c < kSwClasses - 1; ++c) {
-    uint64_t lo = 0, hi = n;
-    while (lo < hi) {
-      uint64_t m = (lo + hi) >> 1;
-      if (sw_class_of(tasks[m].width) <= c) lo = m + 1;
-      else hi = m;
-    }
-    out[c] = (int64_t)lo;
+  const int c = threadIdx.x;  // one thread per class
+  uint64_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint64_t m = (lo + hi) >> 1;
+    const uint32_t w = tasks[m].width;
+    if ((w == kSwNoClass ? kSwClasses : sw_class_of(w)) <= c) lo = m + 1;
+    else hi = m;
   }
+  out[c] = (int64_t)lo;
 }
 
 // Longest warp of each width class, in column steps (strips x (W + 16)).
@@ -365,6 +457,7 @@ __global__ void k_task_steps(const SwTask* tasks, uint64_t n, unsigned long long
   uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (t >= n || (d_n && t >= (uint64_t)*d_n)) return;
   const SwTask k = tasks[t];
+  if (k.width == kSwNoClass) return;
   atomicMax(mx + sw_class_of(k.width), (unsigned long long)k.n_strips * (k.width + 16ull));
 }
 
@@ -383,42 +476,30 @@ __global__ void k_compact_ops(const uint32_t* ops, const uint64_t* ops_off, cons
   for (uint32_t i = 0; i < out[k].n_ops; ++i) o[i] = src[i];
 }
 
-// The band kernel's job of sorted band k (order[k] indexes bands): its rows,
-// and a sort key by kernel route, then longest first.
-__device__ __forceinline__ void band_job(const uint32_t* order, uint64_t k, const Band* bands,
-                                         const uint64_t* s_offsets, SwBandJob* jobs, uint64_t* sort_key,
-                                         uint32_t* sort_val, unsigned long long* max_width) {
-  const uint32_t i = order[k];
-  const Band b = bands[i];
-  const int64_t m = (int64_t)(s_offsets[b.subject + 1] - s_offsets[b.subject]);
-  int64_t re = m + b.d1 < (int64_t)b.n ? m + b.d1 : (int64_t)b.n;
-  const int64_t rs = band_first_row(b);
-  if (re < rs) re = rs;
-  const uint32_t W = (uint32_t)(b.d1 - b.d0 + 1);
-  SwBandJob j;
-  j.band = i;
-  j.row_first = (uint32_t)rs;
-  j.n_strips = (uint32_t)((re - rs + 16) / 16);
-  j.pad = W;
-  jobs[k] = j;
-  // by kernel route (sw_band_route), then longest first
-  const int route = sw_band_route((int)W);
-  const uint64_t cost = (uint64_t)(j.n_strips - 1) * 19ull + W + 16ull;
-  sort_key[k] = ((uint64_t)route << kCostBits) | (kCostMax - (cost < kCostMax ? cost : kCostMax));
-  sort_val[k] = (uint32_t)k;
-  atomicMax(max_width, (unsigned long long)W);
-  atomicAdd(max_width + 1 + route, 1ull);
-}
 // Score pass on device counts: the wide bands are sorted positions
-// [cnt[1], cnt[0]) (after the narrow ones); n bounds their count, which is
-// also written to cnt[15] for the job sort.
+// [cnt[1], cnt[0]) (after the narrow ones); n bounds their count, which starts
+// the count of jobs cnt[15].  route[0] = widest, route[1 + r] = jobs of route r.
 __global__ void k_band_jobs_dev(const uint32_t* order, int64_t* cnt, uint64_t n, const Band* bands,
                                 const uint64_t* s_offsets, SwBandJob* jobs, uint64_t* sort_key, uint32_t* sort_val,
-                                unsigned long long* max_width) {
-  uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+                                unsigned long long* route) {
+  const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const uint64_t n_wide = (uint64_t)(cnt[0] - cnt[1]);
   if (k == 0) cnt[15] = (int64_t)n_wide;
-  if (k < n && k < n_wide) band_job(order + cnt[1], k, bands, s_offsets, jobs, sort_key, sort_val, max_width);
+  if ((k & ~31ull) >= n_wide) return;  // warp-uniform
+  int r = -1;
+  uint32_t W = 0;
+  if (k < n && k < n_wide) {
+    r = band_job(order[cnt[1] + k], k, bands, s_offsets, jobs, sort_key, sort_val);
+    W = jobs[k].pad;
+  }
+  W = __reduce_max_sync(0xFFFFFFFFu, W);
+  const bool head = (threadIdx.x & 31) == 0;
+  if (head) atomicMax(route, (unsigned long long)W);
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const uint32_t in = __ballot_sync(0xFFFFFFFFu, r == x);
+    if (head && in) atomicAdd(route + 1 + x, (unsigned long long)__popc(in));
+  }
 }
 __global__ void k_gather_band_jobs(const SwBandJob* in, const uint32_t* idx, uint64_t n, SwBandJob* out,
                                    const int64_t* d_n) {
@@ -516,15 +597,6 @@ struct BandJobs {
   uint64_t route_lo[5] = {0, 0, 0, 0, 0};  // jobs [route_lo[r], route_lo[r + 1]) take route r
 };
 
-// The band kernels of jobs bj, one launch per route.
-void launch_band_routes(SwBandArgs ba, const BandJobs& bj, cudaStream_t st) {
-  for (int k = 0; k < 4; ++k) {
-    ba.lo = bj.route_lo[k];
-    ba.hi = bj.route_lo[k + 1];
-    launch_sw_band_route(ba, k, bj.max_width, st);
-  }
-}
-
 SwBandArgs band_args(const Band* bc, const BandJobs& bj, const DevSeqs& qs, const DevSeqs& s, const Scoring& scr) {
   SwBandArgs ba{};
   ba.bands = bc;
@@ -610,8 +682,17 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   uint32_t* tr_count = c->tr_count.as<uint32_t>(n_subjects);
   DRG_CUDA(cudaMemsetAsync(tr_count, 0, n_subjects * sizeof(uint32_t), c->stream));
   count_launch();
+  // score pass counts, on the device until the one wait before the launches:
+  //   [0] fast bands  [1] narrow bands  [2] tasks  [6] widest job  [7..10]
+  //   jobs per route  [11..14] longest warp per class  [15] jobs  [16..19]
+  //   bands listed for the 32-bit kernel  [20] sum of the packed kernel's
+  //   chains  [21..24] tasks up to each class's end
+  int64_t* cnt = c->sw_counts.as<int64_t>(25);
+  DRG_CUDA(cudaMemsetAsync(cnt, 0, 25 * sizeof(int64_t), c->stream));
+  unsigned long long* chain_sum = reinterpret_cast<unsigned long long*>(cnt + 20);
   k_sw_tr_count<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(bc, n_bands, s.offsets, scr.max_score,
-                                                                sw_tune(c, scr), tr_count, rows);
+                                                                sw_tune(c, scr), tr_count, rows,
+                                                                chain_sum);
   count_launch();
   // group field: target << 16 | window start, or the subject (transposed)
   SwKeyBits kb;
@@ -634,13 +715,6 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
     swks = r.keys;
     swos = r.vals;
   }
-  uint64_t n_fast = 0, n_narrow = 0;
-  // score pass counts, on the device until the one wait before the launches:
-  //   [0] fast bands  [1] narrow bands  [2] tasks  [3..5] class bounds
-  //   [6] wide max width  [7..10] wide jobs per route  [11..14] longest warp
-  //   per class  [15] wide bands  [16..19] bands listed for the 32-bit kernel
-  int64_t* cnt = c->sw_counts.as<int64_t>(20);
-  DRG_CUDA(cudaMemsetAsync(cnt, 0, 20 * sizeof(int64_t), c->stream));
   count_launch();
   k_count_fast_narrow<<<1, 1, 0, c->stream>>>(swks, n_bands, kb.wide, cnt);
   // ---- wide bands (positions [narrow, fast) of the sorted order): band-
@@ -654,12 +728,6 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   count_launch();
   k_band_jobs_dev<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(
       swos, cnt, n_bands, bc, s.offsets, jobs_u, jkey, jval, reinterpret_cast<unsigned long long*>(cnt + 6));
-  const uint32_t* jorder =
-      dsort(c, jkey, jkey_s, jval, jval_s, n_bands, 0, kCostBits + 3, reinterpret_cast<const uint64_t*>(cnt + 15))
-          .vals;
-  count_launch();
-  k_gather_band_jobs<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(jobs_u, jorder, n_bands, wjobs,
-                                                                      cnt + 15);
   // ---- narrow bands: warps of up to 32 bands of one group
   uint32_t* gstart = c->idx.as<uint32_t>(n_bands + 1);
   count_launch();
@@ -678,34 +746,39 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   uint32_t* tval = c->task_val.as<uint32_t>(n_bands);
   uint32_t* tval_s = c->task_val_s.as<uint32_t>(n_bands);
   count_launch();
-  k_sw_fill_tasks<<<ceil_div(n_bands, 128), 128, 0, c->stream>>>(tstart, n_bands, swks, n_bands, kb.transposed,
-                                                                  swos, bc, s.offsets, tasks_u, tkey, tval,
-                                                                  cells_gpu, cnt + 2, cnt + 1);
+  k_sw_fill_tasks<<<ceil_div(n_bands, 128), 128, 0, c->stream>>>(
+      tstart, n_bands, swks, n_bands, kb.transposed, swos, bc, s.offsets, tasks_u, tkey, tval, cells_gpu, cnt + 2,
+      cnt + 1, chain_sum, jobs_u, jkey, jval,
+      reinterpret_cast<unsigned long long*>(cnt + 15), reinterpret_cast<unsigned long long*>(cnt + 6));
+  const uint32_t* jorder =
+      dsort(c, jkey, jkey_s, jval, jval_s, n_bands, 0, kCostBits + 3, reinterpret_cast<const uint64_t*>(cnt + 15))
+          .vals;
+  count_launch();
+  k_gather_band_jobs<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(jobs_u, jorder, n_bands, wjobs,
+                                                                      cnt + 15);
   // by width class, longest warps first within a class
   const uint32_t* task_order =
-      dsort(c, tkey, tkey_s, tval, tval_s, n_bands, 0, kCostBits + 2, reinterpret_cast<const uint64_t*>(cnt + 2))
+      dsort(c, tkey, tkey_s, tval, tval_s, n_bands, 0, kCostBits + 3, reinterpret_cast<const uint64_t*>(cnt + 2))
           .vals;
   count_launch();
   k_gather_tasks<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(tasks_u, task_order, n_bands, tasks, cnt + 2);
   count_launch();
-  k_task_bounds<<<1, 1, 0, c->stream>>>(tasks, n_bands, cnt + 3, cnt + 2);
+  k_task_bounds<<<1, kSwClasses, 0, c->stream>>>(tasks, n_bands, cnt + 21, cnt + 2);
   count_launch();
   k_task_steps<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(tasks, n_bands,
                                                                reinterpret_cast<unsigned long long*>(cnt + 11),
                                                                cnt + 2);
   // ---- the one wait: every count the launches need
-  int64_t* h = c->h_stage.as<int64_t>(16);
-  DRG_CUDA(cudaMemcpyAsync(h, cnt, 16 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+  int64_t* h = c->h_stage.as<int64_t>(25);
+  DRG_CUDA(cudaMemcpyAsync(h, cnt, 25 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
   DRG_CUDA(cudaStreamSynchronize(c->stream));
-  n_fast = (uint64_t)h[0];
-  n_narrow = (uint64_t)h[1];
-  const uint64_t n_tasks = (uint64_t)h[2];
-  int64_t bounds[kSwClasses - 1] = {h[3], h[4], h[5]};
+  const uint64_t n_fast = (uint64_t)h[0];
+  const int64_t* bounds = h + 21;  // ends of the classes
   unsigned long long hmax[kSwClasses];
   for (int k = 0; k < kSwClasses; ++k) hmax[k] = (unsigned long long)h[11 + k];
   BandJobs wide;
   wide.jobs = wjobs;
-  wide.n = n_fast - n_narrow;
+  wide.n = (uint64_t)h[15];
   wide.max_width = (int)h[6];
   for (int k = 0; k < 4; ++k) wide.route_lo[k + 1] = wide.route_lo[k] + (uint64_t)h[7 + k];
   // bands the packed kernels do not take, in the 32-bit kernel: the longest
@@ -734,54 +807,79 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
     uint64_t lo[kSwClasses], hi[kSwClasses];
     for (int k = 0; k < kSwClasses; ++k) {
       lo[k] = k == 0 ? 0 : (uint64_t)bounds[k - 1];
-      hi[k] = k == kSwClasses - 1 ? n_tasks : (uint64_t)bounds[k];
+      hi[k] = (uint64_t)bounds[k];
     }
-    // The bulk class runs on the main stream; the wider classes and the wide
-    // bands run on the side stream, queued first so that the long warps start
-    // early and the pass ends on the bulk class's shortest tasks.
-    std::array<cudaEvent_t, 2 * kSwClasses + 3> ev;
-    for (auto& e : ev) e = log->event();
-    const int fork = 2 * kSwClasses, wide0 = fork + 1, wide1 = fork + 2;
-    DRG_CUDA(cudaEventRecord(ev[fork], c->stream));
-    DRG_CUDA(cudaStreamWaitEvent(c->side, ev[fork], 0));
-    auto launch_cls = [&](int cls) {
-      cudaStream_t sc = cls == 0 ? c->stream : c->side;
+    // The bulk class runs on the main stream, the wider classes on the side
+    // stream, and the lane kernel's routes and the unpacked bands on a stream
+    // each, queued first: every launch ends on its longest chain, and one
+    // after the other those ends add up (61 queries, sensitive: 6.4 ms against
+    // 4.9 ms side by side).  The pass then ends on the bulk class's shortest
+    // tasks.
+    cudaEvent_t fork = log->event();
+    DRG_CUDA(cudaEventRecord(fork, c->stream));
+    std::vector<cudaEvent_t> ends;  // of the other streams
+    auto on = [&](cudaStream_t s2, auto&& launch) {
+      DRG_CUDA(cudaStreamWaitEvent(s2, fork, 0));
+      launch(s2);
+      cudaEvent_t e = log->event();
+      DRG_CUDA(cudaEventRecord(e, s2));
+      ends.push_back(e);
+      return e;
+    };
+    if (n_bands > n_fast)
+      on(c->lanes[4], [&](cudaStream_t s2) {
+        sys_scores(c, xa, c->sys_list, swos, n_fast, n_bands, nullptr, cnt + 16, n_sys, s.max_len, s2);
+      });
+    std::vector<cudaEvent_t> wide_ends;
+    SwBandArgs ba = band_args(bc, wide, qs, s, scr);
+    ba.score = scores;
+    ba.best_row = best_row;
+    for (int k = 3; k >= 0; --k) {
+      ba.lo = wide.route_lo[k];
+      ba.hi = wide.route_lo[k + 1];
+      if (ba.hi == ba.lo) continue;
+      wide_ends.push_back(on(c->lanes[k], [&](cudaStream_t s2) { launch_sw_band_route(ba, k, wide.max_width, s2); }));
+      st.sw_launches += 1;
+    }
+    std::array<cudaEvent_t, 2 * kSwClasses> ev{};
+    auto launch_cls = [&](int cls, cudaStream_t sc) {
+      if (hi[cls] == lo[cls]) return;
+      ev[2 * cls] = log->event();
+      ev[2 * cls + 1] = log->event();
       sa.task_lo = lo[cls];
       sa.task_hi = hi[cls];
       DRG_CUDA(cudaEventRecord(ev[2 * cls], sc));
-      if (hi[cls] > lo[cls]) {
-        launch_sw_class(sa, cls, sc);
-        st.sw_launches += 1;
-      }
+      launch_sw_class(sa, cls, sc);
+      st.sw_launches += 1;
       DRG_CUDA(cudaEventRecord(ev[2 * cls + 1], sc));
     };
-    sys_scores(c, xa, c->sys_list, swos, n_fast, n_bands, nullptr, cnt + 16, n_sys, s.max_len, c->side);
-    DRG_CUDA(cudaEventRecord(ev[wide0], c->side));
-    if (wide.n > 0) {
-      SwBandArgs ba = band_args(bc, wide, qs, s, scr);
-      ba.score = scores;
-      ba.best_row = best_row;
-      launch_band_routes(ba, wide, c->side);
-      st.sw_launches += 1;
-    }
-    DRG_CUDA(cudaEventRecord(ev[wide1], c->side));
-    for (int cls = kSwClasses - 1; cls >= 1; --cls) launch_cls(cls);
-    launch_cls(0);
-    const int side_end = 2 * 1 + 1;  // class 1 is the side stream's last launch
-    DRG_CUDA(cudaStreamWaitEvent(c->stream, ev[side_end], 0));
+    if (hi[kSwClasses - 1] > lo[1])
+      on(c->side, [&](cudaStream_t s2) {
+        for (int cls = kSwClasses - 1; cls >= 1; --cls) launch_cls(cls, s2);
+      });
+    launch_cls(0, c->stream);
+    for (cudaEvent_t e : ends) DRG_CUDA(cudaStreamWaitEvent(c->stream, e, 0));
+    cudaEvent_t joined = log->event();
+    DRG_CUDA(cudaEventRecord(joined, c->stream));
     for (int k = 0; k < kSwClasses; ++k) {
       st.sw_class_tasks[k] += hi[k] - lo[k];
       if (hmax[k] > st.sw_class_max_steps[k]) st.sw_class_max_steps[k] = hmax[k];
     }
     st.sw_wide_bands += wide.n;
     drg_run_stats* stp = &st;
-    log->later([ev, fork, wide0, wide1, side_end, stp] {
-      float cls_ms[kSwClasses], side_span = 0, wide_ms = 0;
-      for (int k = 0; k < kSwClasses; ++k) DRG_CUDA(cudaEventElapsedTime(&cls_ms[k], ev[2 * k], ev[2 * k + 1]));
-      DRG_CUDA(cudaEventElapsedTime(&side_span, ev[fork], ev[side_end]));
-      DRG_CUDA(cudaEventElapsedTime(&wide_ms, ev[wide0], ev[wide1]));
-      stp->ms_sw_kernel += cls_ms[0] > side_span ? cls_ms[0] : side_span;  // wall of the concurrent launches
-      for (int k = 0; k < kSwClasses; ++k) stp->ms_sw_class[k] += cls_ms[k];
+    log->later([ev, fork, joined, wide_ends, stp] {
+      float ms = 0, wide_ms = 0;
+      DRG_CUDA(cudaEventElapsedTime(&ms, fork, joined));
+      stp->ms_sw_kernel += ms;  // wall of the concurrent launches
+      for (int k = 0; k < kSwClasses; ++k) {
+        if (!ev[2 * k]) continue;
+        DRG_CUDA(cudaEventElapsedTime(&ms, ev[2 * k], ev[2 * k + 1]));
+        stp->ms_sw_class[k] += ms;
+      }
+      for (cudaEvent_t e : wide_ends) {
+        DRG_CUDA(cudaEventElapsedTime(&ms, fork, e));
+        wide_ms = std::max(wide_ms, ms);
+      }
       stp->ms_sw_wide += wide_ms;
     });
   }
@@ -867,8 +965,8 @@ void trace_bands(drg_ctx* c, const Band* bc, uint64_t n, const DevSeqs& qs, cons
   // sensitive search.)  Trace memory that is reused keeps them in order.
   cudaStream_t streams[3] = {c->stream, c->stream, c->stream};
   if (hoff.empty()) {
-    streams[1] = c->side2;
-    streams[2] = c->side;
+    streams[1] = c->lanes[1];
+    streams[2] = c->lanes[2];
   }
   for (int r = 2; r >= 0; --r) {
     if (lo[r + 1] == lo[r]) continue;

@@ -1,6 +1,8 @@
-// Banded affine Smith-Waterman in 32-bit lanes, systolic: the traceback of the
-// HSPs that survive the E-value gate, and the exact score of the bands that
-// the packed 16-bit kernels do not settle (gapped.rs:67-280).
+// Banded affine Smith-Waterman, systolic: the traceback of the HSPs that
+// survive the E-value gate and the exact score of the bands that the packed
+// 16-bit kernels do not settle, in 32-bit lanes (gapped.rs:67-280); and, two
+// bands per warp in 16-bit halves (k_sys_pair), the bands of the score pass
+// that do not fill a warp of the packed kernel or would outlast it.
 //
 // What bounds these bands is the dependency chain of one band, not the chip:
 // there are few of them (4,000 of 1.4M bands of a search of 1,000 queries) and
@@ -57,6 +59,7 @@
 // on the ALU pipe at two cycles each (ncu: 0.39 instructions per cycle for a
 // lone warp, stalled on fixed latencies); its chain is shorter than that.
 #include "kernels.h"
+#include "sw_common.cuh"
 
 namespace drg {
 
@@ -489,6 +492,222 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
   }
 }
 
+// ---- rotating strips, two bands per warp (score pass) ----------------------------
+// The same strips with a band in each 16-bit half: lane and step of a strip
+// depend on its number only, so two bands run in step, each with its own
+// letters, profile and right edge.  Jobs are sorted by route and length, so
+// that a pair's bands end together.  For bands whose best stays below 2^15
+// (the packed kernels' bound); H counts only inside the band and the matrix,
+// and is below 0x7C00 there, so its maximum folds as half-precision bit
+// patterns (max2_pos_f16).
+// A step of 4 rows is about 75 warp instructions for the two bands (8 rows
+// 118, 16 rows 206), ALU-bound like the forms above; 22 bands of a 497-aa
+// query take 156 us (one band per lane: 758 us).  16 rows per lane replace
+// the 16-row groups of lanes on one band each (2,000 bands of 272-559 columns:
+// 708 -> 676 us) up to 511 columns.
+using sw::add2;
+using sw::kNeg2;
+using sw::max2;
+using sw::max2_pos_f16;
+using sw::pick_sel;
+using sw::prmt;
+using sw::sel2;
+
+template <int R>
+constexpr size_t pair_smem() {
+  return (size_t)kRotWarpsPerBlock * 2 * (R / 4) * kResidues * 32 * sizeof(uint32_t);
+}
+
+template <int R>
+__global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs a) {
+  constexpr int kLag = R + 1, kWords = R / 4;
+  extern __shared__ __align__(16) uint32_t pair_prof[];
+  __shared__ int8_t mat[kResidues * 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  stage_scores(mat, a.scores625);
+  const uint64_t t0 = a.lo + 2 * ((uint64_t)blockIdx.x * kRotWarpsPerBlock + warp);
+  if (t0 >= a.hi) return;  // warp-uniform
+  uint32_t* prof = pair_prof + (size_t)warp * 2 * kWords * kResidues * 32;  // [half][word][residue][lane]
+  // per half: geometry and letters (an odd last job runs twice, written once)
+  SysGeom g[2];
+  uint32_t band[2];
+  const uint8_t *q[2], *sl[2];
+  int n[2], m[2], W[2], S[2];
+  int turns = 0;
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    band[x] = a.jobs[t0 + x < a.hi ? t0 + x : t0].band;
+    const Band b = a.bands[band[x]];
+    q[x] = a.q_letters + a.q_offsets[b.target] + b.q0;
+    sl[x] = a.s_letters + a.s_offsets[b.subject];
+    m[x] = (int)(a.s_offsets[b.subject + 1] - a.s_offsets[b.subject]);
+    n[x] = (int)b.n;
+    g[x] = sys_geom(b, m[x], false);
+    W[x] = g[x].d1 - g[x].d0 + 1;
+    S[x] = g[x].rows > 0 ? (g[x].rows + R - 1) / R : 0;
+    turns = max(turns, sys_rot_turns(S[x], W[x], R));
+  }
+  const uint32_t noc2 = (uint32_t)(uint16_t)(-(a.gap_open + a.gap_extend)) * 0x10001u;
+  const uint32_t nge2 = (uint32_t)(uint16_t)(-a.gap_extend) * 0x10001u;
+  uint32_t hl[R], f[R];
+  uint32_t top = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    hl[r] = 0;
+    f[r] = kNeg2;
+  }
+  int best[2] = {0, 0}, bi[2] = {0x7FFFFFFF, 0x7FFFFFFF};
+  int s = lane, c = -kLag * lane;
+  constexpr int kPast = 0x3FFF;  // c - (W - 1) of a lane without a strip: right of the band
+  auto cw_of = [&](int x) { return (uint32_t)(uint16_t)(s < S[x] ? c - (W[x] - 1) : kPast); };
+  uint32_t cw2 = cw_of(0) | cw_of(1) << 16;
+  int p[2] = {g[0].rs - g[0].d1 - 1 - lane, g[1].rs - g[1].d1 - 1 - lane};
+  auto letter = [&](int x, int at) -> uint32_t {
+    return (unsigned)at < (unsigned)m[x] ? (uint32_t)__ldg(sl[x] + at) : (uint32_t)kSentinel;
+  };
+  auto load_rows = [&](int x, int k, uint32_t (&v)[kWords]) {
+#pragma unroll
+    for (int w = 0; w < kWords; ++w) {
+      uint32_t y = 0;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int64_t i = (int64_t)g[x].rs + (int64_t)R * k + 4 * w + r;
+        y |= (k < S[x] && i <= n[x] ? min((uint32_t)__ldg(q[x] + i - 1), 24u) : (uint32_t)kSentinel) << (8 * r);
+      }
+      v[w] = y;
+    }
+  };
+  uint32_t qv[2][kWords], qn[2][kWords];
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    load_rows(x, lane, qv[x]);
+    load_rows(x, 32 + lane, qn[x]);
+  }
+  auto build = [&](int k) {
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+#pragma unroll
+      for (int w = 0; w < kWords; ++w) {
+        const uint32_t ql = __shfl_sync(kAll, qv[x][w], k & 31);
+        uint32_t y = 0;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) y |= (uint32_t)(uint8_t)mat[((ql >> (8 * r)) & 0xFFu) * 32 + lane] << (8 * r);
+        if (lane < kResidues) prof[((x * kWords + w) * kResidues + lane) * 32 + (k & 31)] = y;
+      }
+    }
+  };
+  auto fold = [&]() {
+    const int t2[2] = {(int)(top & 0xFFFFu), (int)(top >> 16)};
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      if (t2[x] > best[x]) {
+        best[x] = t2[x];
+        bi[x] = g[x].rs + R * s + R - 1;  // a bound of the best's row
+      }
+    }
+    top = 0;
+  };
+  __syncwarp();
+  build(0);
+  __syncwarp();
+  uint32_t l1[2], wn[2][kWords];
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    const uint32_t l0 = letter(x, p[x]);
+    l1[x] = letter(x, p[x] + 1);
+#pragma unroll
+    for (int w = 0; w < kWords; ++w) wn[x][w] = prof[((x * kWords + w) * kResidues + l0) * 32 + lane];
+  }
+  uint32_t hup = 0, h_out = 0, e_out = kNeg2;
+  const int src = (lane + 31) & 31;
+  for (int k = 0; k < turns; ++k) {
+    if (((k + 1) & 31) == 0) {
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+#pragma unroll
+        for (int w = 0; w < kWords; ++w) qv[x][w] = qn[x][w];
+        load_rows(x, k + 33 + lane, qn[x]);
+      }
+    }
+    if (k + 1 < max(S[0], S[1])) build(k + 1);
+    if (k >= 31 && lane == ((k + 1) & 31)) {
+      fold();
+      s += 32;
+      c -= 32 * kLag;
+      p[0] -= 32;
+      p[1] -= 32;
+      cw2 = cw_of(0) | cw_of(1) << 16;
+    }
+    const bool starts = lane == (k & 31);
+    if (starts) {
+      top = 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        hl[r] = 0;
+        f[r] = kNeg2;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kLag; ++u) {
+      uint32_t hu = __shfl_sync(kAll, h_out, src), eu = __shfl_sync(kAll, e_out, src);
+      if (s == 0) {
+        hu = 0;
+        eu = kNeg2;
+      }
+      uint32_t w[2][kWords];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+#pragma unroll
+        for (int y = 0; y < kWords; ++y) {
+          w[x][y] = wn[x][y];
+          wn[x][y] = prof[((x * kWords + y) * kResidues + l1[x]) * 32 + lane];
+        }
+        l1[x] = letter(x, p[x] + 2);
+      }
+      uint32_t hd = hup;
+      hup = hu;
+      uint32_t t = 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint32_t sc = prmt(w[0][r >> 2], w[1][r >> 2], pick_sel(r & 3));
+        const uint32_t in = prmt(add2(cw2, (uint32_t)(uint16_t)(-(r + 1)) * 0x10001u), 0u, 0xBB99u);
+        uint32_t e = __viaddmax_s16x2(eu, nge2, add2(hu, noc2));
+        uint32_t fn = __viaddmax_s16x2(f[r], nge2, add2(hl[r], noc2));
+        const uint32_t x = __viaddmax_s16x2_relu(hd, sc, fn);
+        uint32_t h = max2(x, e) & in;
+        e = sel2(e, in, kNeg2);
+        if (u < R - 1 && r > u && starts) {  // left of the band
+          h = 0;
+          fn = kNeg2;
+        }
+        t = max2_pos_f16(t, h);
+        hd = hl[r];
+        hl[r] = h;
+        f[r] = fn;
+        hu = h;
+        eu = e;
+      }
+      top = max2_pos_f16(top, t);
+      h_out = hu;
+      e_out = eu;
+      cw2 = add2(cw2, 0x00010001u);
+      ++c;
+      ++p[0];
+      ++p[1];
+    }
+  }
+  fold();
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    const CellOut b = warp_best(CellOut{best[x], bi[x], 0});
+    if (lane == 0 && t0 + x < a.hi) {
+      a.score[band[x]] = b.best;
+      if (a.best_row) a.best_row[band[x]] = b.best > 0 ? min(b.bi, n[x]) : 0;
+    }
+  }
+}
+
 // ---- any width: one block per band ----------------------------------------------
 template <bool TR>
 __global__ void __launch_bounds__(kBlkWarps * 32) k_sys_block(SysArgs a) {
@@ -660,6 +879,30 @@ void launch_sys_score(SysArgs a, int route, uint64_t n_max, cudaStream_t st) {
     k_sys_block<false><<<(unsigned)(n_max < kSysBlocks ? n_max : kSysBlocks), kBlkWarps * 32, 0, st>>>(a);
   }
   DRG_CUDA(cudaGetLastError());
+}
+
+template <int R>
+static void launch_pair(const SwBandArgs& a, cudaStream_t st) {
+  static bool configured = false;
+  if (!configured) {
+    DRG_CUDA(cudaFuncSetAttribute(k_sys_pair<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem<R>()));
+    configured = true;
+  }
+  const uint64_t warps = (a.hi - a.lo + 1) / 2;
+  count_launch();
+  k_sys_pair<R><<<(unsigned)((warps + kRotWarpsPerBlock - 1) / kRotWarpsPerBlock), kRotWarpsPerBlock * 32,
+                  pair_smem<R>(), st>>>(a);
+  DRG_CUDA(cudaGetLastError());
+}
+
+void launch_sw_band_route(const SwBandArgs& a, int route, int max_width, cudaStream_t st) {
+  if (a.hi <= a.lo) return;
+  switch (route) {
+    case 0: launch_pair<4>(a, st); break;
+    case 1: launch_pair<8>(a, st); break;
+    case 2: launch_pair<16>(a, st); break;
+    default: launch_sw_band(a, max_width, st); break;
+  }
 }
 
 void launch_sys_trace(SysArgs a, int route, cudaStream_t st) {

@@ -66,3 +66,17 @@ def test_many_bands_of_mixed_routes(ctx, orc):
     jobs = [(k % 24, k % 24, int(c) - int(w) // 2, int(c) - int(w) // 2 + int(w) - 1)
             for k, (w, c) in enumerate(zip(r.integers(1, 420, 240), r.integers(-300, 200, 240)))]
     _check(ctx, orc, list(qs), list(ss), jobs, "PAM70")
+
+
+def test_two_bands_per_warp(ctx, orc):
+    # the score pass's lane kernel: the edges of its three widths, an odd count,
+    # halves of a warp of very different lengths, a best just below 0x7C00
+    r = np.random.Generator(np.random.PCG64(77))
+    qs, ss = zip(*[_related(r, n, m) for n, m in ((1, 30), (3, 60), (33, 40), (300, 280), (640, 600), (1100, 1500))])
+    qs, ss = list(qs), list(ss)
+    jobs = [(k, k, -w // 2, -w // 2 + w - 1) for w in (17, 18, 31, 136, 137, 151, 152, 271, 272, 273, 511, 512)
+            for k in range(6)]
+    jobs.append((5, 5, -60, 60))
+    _check(ctx, orc, qs, ss, jobs)
+    q = np.full(2885, 17, np.uint8)  # W scores 11: 31,735
+    _check(ctx, orc, [q, qs[2]], [q.copy(), ss[2]], [(0, 0, -10, 10), (1, 1, -10, 10), (0, 0, -250, 250)])
