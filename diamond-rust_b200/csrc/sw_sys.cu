@@ -502,16 +502,13 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
 // patterns (max2_pos_f16).
 // A step of 4 rows is about 75 warp instructions for the two bands (8 rows
 // 118, 16 rows 206), ALU-bound like the forms above; 22 bands of a 497-aa
-// query take 156 us (one band per lane: 758 us).  16 rows per lane replace
+// query take 142 us (one band per lane: 758 us).  16 rows per lane replace
 // the 16-row groups of lanes on one band each (2,000 bands of 272-559 columns:
 // 708 -> 676 us) up to 511 columns.
 using sw::add2;
-using sw::kNeg2;
-using sw::max2;
 using sw::max2_pos_f16;
 using sw::pick_sel;
 using sw::prmt;
-using sw::sel2;
 
 template <int R>
 constexpr size_t pair_smem() {
@@ -554,7 +551,7 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs 
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     hl[r] = 0;
-    f[r] = kNeg2;
+    f[r] = 0;
   }
   int best[2] = {0, 0}, bi[2] = {0x7FFFFFFF, 0x7FFFFFFF};
   int s = lane, c = -kLag * lane;
@@ -618,7 +615,7 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs 
 #pragma unroll
     for (int w = 0; w < kWords; ++w) wn[x][w] = prof[((x * kWords + w) * kResidues + l0) * 32 + lane];
   }
-  uint32_t hup = 0, h_out = 0, e_out = kNeg2;
+  uint32_t hup = 0, h_out = 0, e_out = 0;
   const int src = (lane + 31) & 31;
   for (int k = 0; k < turns; ++k) {
     if (((k + 1) & 31) == 0) {
@@ -644,7 +641,7 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs 
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         hl[r] = 0;
-        f[r] = kNeg2;
+        f[r] = 0;
       }
     }
     __syncwarp();
@@ -653,7 +650,7 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs 
       uint32_t hu = __shfl_sync(kAll, h_out, src), eu = __shfl_sync(kAll, e_out, src);
       if (s == 0) {
         hu = 0;
-        eu = kNeg2;
+        eu = 0;
       }
       uint32_t w[2][kWords];
 #pragma unroll
@@ -672,14 +669,18 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs 
       for (int r = 0; r < R; ++r) {
         const uint32_t sc = prmt(w[0][r >> 2], w[1][r >> 2], pick_sel(r & 3));
         const uint32_t in = prmt(add2(cw2, (uint32_t)(uint16_t)(-(r + 1)) * 0x10001u), 0u, 0xBB99u);
-        uint32_t e = __viaddmax_s16x2(eu, nge2, add2(hu, noc2));
-        uint32_t fn = __viaddmax_s16x2(f[r], nge2, add2(hl[r], noc2));
-        const uint32_t x = __viaddmax_s16x2_relu(hd, sc, fn);
-        uint32_t h = max2(x, e) & in;
-        e = sel2(e, in, kNeg2);
+        // e, fn: E and F with the open cost added back, so that E' = max(E' -
+        // ge, H) above, F' = max(F' - ge, H) to the left and H = max(0, D,
+        // max(E', F') - oc): all at least 0, a dead cell plain 0, and two adds
+        // per pair less than with H - oc (22 bands of a 497-aa query: 156 ->
+        // 142 us)
+        uint32_t e = __viaddmax_s16x2(eu, nge2, hu);
+        uint32_t fn = __viaddmax_s16x2(f[r], nge2, hl[r]);
+        uint32_t h = __viaddmax_s16x2_relu(max2_pos_f16(e, fn), noc2, add2(hd, sc)) & in;
+        e &= in;
         if (u < R - 1 && r > u && starts) {  // left of the band
           h = 0;
-          fn = kNeg2;
+          fn = 0;
         }
         t = max2_pos_f16(t, h);
         hd = hl[r];
