@@ -312,6 +312,72 @@ int onesweep_resident_blocks() {
   return r;
 }
 
+// Up to kSmallSort keys: one block, one launch.  Each key's bits [begin_bit,
+// end_bit) and its index make one 64-bit word (so equal keys keep their
+// order), sorted by a bitonic network: stages whose pairs lie 32 words apart
+// or less run in a warp's registers (64 words, shuffles), the others in shared
+// memory between block barriers.  What bounds such a sort is launches: TIMES
+constexpr int kSmallSort = 4096, kSmallBits = 52, kSmallThreads = 1024;
+template <typename K>
+__global__ void __launch_bounds__(kSmallThreads) k_sort_small(const K* __restrict__ kin, K* __restrict__ kout,
+                                                              const uint32_t* __restrict__ vin,
+                                                              uint32_t* __restrict__ vout, const uint64_t* d_n,
+                                                              uint32_t n_max, int begin_bit, int bits) {
+  __shared__ uint64_t w[kSmallSort];
+  const uint32_t n = d_n ? (uint32_t)(*d_n < n_max ? *d_n : n_max) : n_max;
+  uint32_t size = 64;  // words of the network
+  while (size < n) size <<= 1;
+  const uint64_t mask = (1ull << bits) - 1;
+  for (uint32_t i = threadIdx.x; i < size; i += kSmallThreads)
+    w[i] = i < n ? (((uint64_t)kin[i] >> begin_bit & mask) << 12) | i : ~0ull;
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31;
+  // the stages of 2^k from pairs j <= 32 apart on, for each warp's 64 words
+  auto in_warp = [&](uint32_t k_first, uint32_t k_last) {
+    for (uint32_t base = 2 * (threadIdx.x & ~31u); base < size; base += 2 * kSmallThreads) {
+      uint64_t lo = w[base + lane], hi = w[base + 32 + lane];
+      for (uint32_t k = k_first; k <= k_last; k <<= 1) {
+        if (k >= 64 && (lo > hi) == (((base + lane) & k) == 0)) {
+          const uint64_t x = lo;
+          lo = hi;
+          hi = x;
+        }
+        for (uint32_t j = k >= 64 ? 16 : k >> 1; j > 0; j >>= 1) {
+          const uint64_t a = __shfl_xor_sync(0xFFFFFFFFu, lo, j), b = __shfl_xor_sync(0xFFFFFFFFu, hi, j);
+          const bool first = (lane & j) == 0;
+          const bool up_lo = ((base + lane) & k) == 0, up_hi = ((base + 32 + lane) & k) == 0;
+          if ((lo > a) == (first == up_lo)) lo = a;
+          if ((hi > b) == (first == up_hi)) hi = b;
+        }
+      }
+      w[base + lane] = lo;
+      w[base + 32 + lane] = hi;
+    }
+  };
+  in_warp(2, 64);
+  for (uint32_t k = 128; k <= size; k <<= 1) {
+    __syncthreads();
+    for (uint32_t j = k >> 1; j > 32; j >>= 1) {
+      for (uint32_t t = threadIdx.x; t < size / 2; t += kSmallThreads) {
+        const uint32_t a = 2 * t - (t & (j - 1)), b = a + j;  // pair t of this stage
+        const uint64_t x = w[a], y = w[b];
+        if ((x > y) == ((a & k) == 0)) {
+          w[a] = y;
+          w[b] = x;
+        }
+      }
+      __syncthreads();
+    }
+    in_warp(k, k);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < n; i += kSmallThreads) {
+    const uint32_t from = (uint32_t)w[i] & 0xFFFu;
+    kout[i] = kin[from];
+    if (vin) vout[i] = vin[from];
+  }
+}
+
 constexpr int kMaxPasses = 8;  // 64-bit keys in 8-bit digits
 
 struct SortPlan {
@@ -352,6 +418,15 @@ SortResult<K> radix_sort(K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_al
   if (end_bit > (int)(8 * sizeof(K))) end_bit = 8 * sizeof(K);
   const SortPlan p = plan<K>(n_max, begin_bit, end_bit, small_tiles);
   if (p.passes == 0 || (n_max == 0 && !d_n)) return r;
+  if (n_max <= (uint64_t)kSmallSort && end_bit - begin_bit <= kSmallBits) {
+    count_launch();
+    k_sort_small<K><<<1, kSmallThreads, 0, st>>>(keys, keys_alt, vals, vals_alt, d_n, (uint32_t)n_max, begin_bit,
+                                                 end_bit - begin_bit);
+    DRG_CUDA(cudaGetLastError());
+    r.keys = keys_alt;
+    r.vals = vals ? vals_alt : nullptr;
+    return r;
+  }
   // (a reallocation shows in the capacity: the new block may start at the
   // old address, holding another buffer's stale words)
   const size_t cap_before = temp.buf.cap;
