@@ -37,17 +37,17 @@ void launch_seed_enum(const uint8_t* letters, const uint64_t* offsets, const uin
 void launch_key_filter(const uint64_t* run_keys, uint64_t n, uint64_t key_mask, uint32_t* filter, int log2_bits,
                        cudaStream_t st);
 // Reference seeds of letters [letter_lo, letter_hi) whose key's bit is set
-// in the filter, appended in no fixed order: counts[0] += kept, counts[1] +=
-// valid seeds (kept or not).  keys / vals need room for every seed of the
-// range; 32-bit keys for a seed key of at most 32 bits.
+// in the filter, appended in no fixed order at *kept, which counts them;
+// *valid += valid seeds (kept or not).  keys / vals need room for every seed of
+// the range; 32-bit keys for a seed key of at most 32 bits.
 void launch_seed_enum_filtered(const uint8_t* letters, const uint64_t* offsets, const uint32_t* owner,
                                uint64_t letter_lo, uint64_t letter_hi, int n_shapes, const uint32_t* filter,
-                               int log2_bits, uint64_t* keys, uint32_t* vals, unsigned long long* counts, int slot,
-                               cudaStream_t st);
+                               int log2_bits, uint64_t* keys, uint32_t* vals, unsigned long long* kept,
+                               unsigned long long* valid, int slot, cudaStream_t st);
 void launch_seed_enum_filtered(const uint8_t* letters, const uint64_t* offsets, const uint32_t* owner,
                                uint64_t letter_lo, uint64_t letter_hi, int n_shapes, const uint32_t* filter,
-                               int log2_bits, uint32_t* keys, uint32_t* vals, unsigned long long* counts, int slot,
-                               cudaStream_t st);
+                               int log2_bits, uint32_t* keys, uint32_t* vals, unsigned long long* kept,
+                               unsigned long long* valid, int slot, cudaStream_t st);
 constexpr uint64_t kNoSeed = ~0ull;
 // Sorted seeds to seed::build's records; *n_valid = the valid ones (n > 0).
 void launch_seed_entries(const uint64_t* keys, const uint32_t* vals, uint64_t n, const uint32_t* owner,
@@ -114,6 +114,23 @@ struct HitKeyLayout {
   int total() const { return tb + sb + db + pb; }
 };
 
+// Index chunks joined together: (chunk, run) entries chunk * n_runs + run.
+constexpr int kJoinChunks = 16;
+struct JoinChunks {
+  int n;                              // 0: one chunk, entries are the runs
+  uint32_t n_runs;
+  uint64_t end[kJoinChunks];          // letters before the end of each chunk
+  const uint32_t* vals[kJoinChunks];  // each chunk's reference payloads
+};
+// launch_join_count for jc.n chunks whose seeds are sorted together, equal keys
+// in chunk order: n x n_runs entries.
+void launch_join_count_chunks(const uint64_t* run_keys, const uint32_t* run_counts, const uint64_t* ref_keys,
+                              const JoinChunks& jc, uint64_t max_expand, uint32_t* run_rlo, uint32_t* run_rcount,
+                              uint64_t* run_hits, uint64_t key_mask, cudaStream_t st, const uint32_t* first, int shift);
+void launch_join_count_chunks(const uint64_t* run_keys, const uint32_t* run_counts, const uint32_t* ref_keys,
+                              const JoinChunks& jc, uint64_t max_expand, uint32_t* run_rlo, uint32_t* run_rcount,
+                              uint64_t* run_hits, uint64_t key_mask, cudaStream_t st, const uint32_t* first, int shift);
+
 // Expand every counted run into hits.  Writes hit_keys[h] (packed) when
 // keys_mode, otherwise hits[h] = {query seq, qpos, subject seq, spos} taken
 // straight from the entries' (seq, pos).
@@ -125,6 +142,7 @@ struct JoinExpandArgs {
   const uint32_t* run_rlo;
   const uint32_t* run_rcount;
   uint64_t n_runs;
+  JoinChunks chunks;       // chunks.n > 0: the runs are (chunk, run) entries, payloads per chunk
   const uint32_t* q_vals;  // query entry payloads
   const uint32_t* r_vals;  // reference entry payloads
   uint64_t n_hits;

@@ -112,7 +112,6 @@ int64_t count_valid(drg_ctx* c, const K* keys, uint64_t n, int64_t* d_tmp) {
 }
 
 __global__ void k_set_u64(uint64_t* p, uint64_t v) { *p = v; }
-__global__ void k_add_u64(unsigned long long* p, const unsigned long long* v) { *p += *v; }
 
 // flags of each pair's first band, over a bound n of the device count *d_n
 // (0 past the count)
@@ -1012,6 +1011,11 @@ struct Candidate {
   double evalue, bits;
 };
 
+// Limits of the join of all index chunks together: its (chunk, query run)
+// arrays of 24 bytes an entry, its seed positions (16 or 24 bytes each), and a
+// hit budget below which a search is meant to go in small pieces.
+constexpr uint64_t kMergeRuns = 1ull << 28, kMergePositions = 1ull << 28, kMergeHits = 1ull << 24;
+
 struct Search {
   drg_ctx* c;
   const drg_db* db;
@@ -1129,26 +1133,44 @@ struct Search {
 
   void run(drg_result* out);
   void query_seeds(uint64_t* n_runs);
-  // The join of index chunk [c0, c1): its hits are appended to acc.
-  void join_chunk(uint64_t c0, uint64_t c1, uint64_t n_runs);
+  // The join of index chunk k: its hits are appended to acc.
+  void join_chunk(size_t k, uint64_t n_runs);
   // bitmap of the query's seed keys (built on the first chunk that needs it)
   uint32_t* key_filter = nullptr;
   int key_filter_log2 = 0;
   void build_key_filter(uint64_t n_runs);
-  // The first index chunk's reference side (key bitmap, filtered reference
-  // seeds, their sort) on the side stream while the query seeds sort: no
-  // index cache, no request ids, 32-bit seed keys.  The query enumeration
-  // sets the bitmap; ev_qkeys: it is done; ev_ref: the chunk's sorted
-  // reference seeds are ready.
+  // Sorted reference seeds of one or several index chunks.
+  struct RefSeeds {
+    const uint64_t* keys = nullptr;    // or
+    const uint32_t* keys32 = nullptr;  // when the seed key fits 32 bits
+    const uint32_t* vals = nullptr;
+    int64_t nr = 0;                  // their count, or a bound of it when
+    const uint64_t* d_nr = nullptr;  // it is on the device only
+  };
+  // The seeds of chunks [k0, k1) whose key the query holds, equal keys in
+  // chunk order, sorted on `stream`.
+  RefSeeds filtered_seeds(size_t k0, size_t k1, cudaStream_t stream, SortScratch& scratch);
+  // The reference side of the first index chunk (of all, when they are joined
+  // together) on the side stream while the query seeds sort: no index cache,
+  // no request ids, 32-bit seed keys.  The query enumeration sets the bitmap;
+  // ev_qkeys: it is done; ev_ref: the sorted reference seeds are ready.
   bool early_possible() const;
   void start_early_ref();
   bool early_ref = false;
-  uint64_t early_c0 = 0, early_c1 = 0;
-  const uint32_t* early_keys32_s = nullptr;
-  const uint32_t* early_vals_s = nullptr;
-  int64_t early_nr = 0;
-  const uint64_t* early_d_nr = nullptr;
+  size_t early_chunks = 0;  // chunks [0, early_chunks)
+  RefSeeds early;
   cudaEvent_t ev_ref = nullptr, ev_qkeys = nullptr;
+  std::vector<std::pair<uint64_t, uint64_t>> chunks;
+  // Seed positions of chunks [k0, k1) over all shapes.
+  uint64_t positions(size_t k0, size_t k1) const {
+    return (db->h_offsets[chunks[k1 - 1].second] - db->h_offsets[chunks[k0].first]) * (uint64_t)shapes.size();
+  }
+  bool cached() const { return db->cache && db->cache->budget() > 0; }
+  // All chunks joined together (see join_all).
+  bool merge = false;
+  bool join_all(uint64_t n_runs);
+  std::vector<std::shared_ptr<SeedIndex>> held;  // join_all's look-ups in the index cache, per chunk
+  size_t looked_up = 0;
   // X-drop, bands, score pass and gate over the accumulated hits.
   void process_hits(uint64_t pass_id);
   // Hits of the chunks joined since the last process_hits (device, from the
@@ -1156,6 +1178,8 @@ struct Search {
   uint64_t* acc = nullptr;
   uint64_t acc_n = 0, acc_cap = 0;
   void acc_reserve(uint64_t n);
+  void expand_hits(uint64_t n_hits, uint64_t n_runs, const uint64_t* roff, const uint32_t* qstart, const uint32_t* rlo,
+                   const uint32_t* rcnt, const uint32_t* r_vals, const JoinChunks* jc);
   ~Search() {
     if (early_ref) cudaStreamSynchronize(c->side);  // unconsumed side-stream work (a search that stopped early)
     if (acc) cudaFreeAsync(acc, c->stream);
@@ -1265,12 +1289,62 @@ void Search::acc_reserve(uint64_t n) {
 // of the keys that no query holds pass, and the bitmap stays resident in L2
 // while the reference seeds probe it.
 bool Search::early_possible() const {
-  const bool cached = db->cache && db->cache->budget() > 0;
-  if (cached || q->request || seed_key_bits > 32 || db->n == 0) return false;
-  const auto ch = split_chunks(db->n, index_chunks);
-  if (ch.empty()) return false;
-  const uint64_t n_pos = (db->h_offsets[ch[0].second] - db->h_offsets[ch[0].first]) * (uint64_t)shapes.size();
-  return n_pos < (1ull << 32);
+  if (cached() || q->request || seed_key_bits > 32 || chunks.empty()) return false;
+  return positions(0, merge ? chunks.size() : 1) < (1ull << 32);
+}
+
+Search::RefSeeds Search::filtered_seeds(size_t k0, size_t k1, cudaStream_t stream, SortScratch& scratch) {
+  const int S = (int)shapes.size();
+  const uint64_t N = positions(k0, k1);
+  const bool key32 = seed_key_bits <= 32;
+  // every buffer first, on the host (a reallocation would wait for the device)
+  unsigned long long* cnt = c->seed_counts.as<unsigned long long>(1);
+  uint32_t* vals = c->r_vals.as<uint32_t>(N);
+  uint32_t* vals_alt = c->r_vals_s.as<uint32_t>(N);
+  void* keys = key32 ? (void*)c->r_keys.as<uint32_t>(N) : (void*)c->r_keys.as<uint64_t>(N);
+  void* keys_alt = key32 ? (void*)c->r_keys_s.as<uint32_t>(N) : (void*)c->r_keys_s.as<uint64_t>(N);
+  uint32_t* err = c->sort_err.as<uint32_t>(1);
+  if (stream != c->stream) {  // the query seeds are enumerated and the bitmap set
+    DRG_CUDA(cudaEventRecord(ev_qkeys, c->stream));
+    DRG_CUDA(cudaStreamWaitEvent(stream, ev_qkeys, 0));
+  }
+  DRG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), stream));
+  // chunk after chunk: the kept seeds of one follow those of the one before
+  for (size_t k = k0; k < k1; ++k) {
+    const uint64_t lo = db->h_offsets[chunks[k].first], hi = db->h_offsets[chunks[k].second];
+    if (key32)
+      launch_seed_enum_filtered(db->letters, db->offsets, db->owner + lo, lo, hi, S, key_filter, key_filter_log2,
+                                (uint32_t*)keys, vals, cnt, d_counters + 7, c->slot, stream);
+    else
+      launch_seed_enum_filtered(db->letters, db->offsets, db->owner + lo, lo, hi, S, key_filter, key_filter_log2,
+                                (uint64_t*)keys, vals, cnt, d_counters + 7, c->slot, stream);
+  }
+  // the kept count stays on the device: the sort, the bucket starts and the
+  // join read it there (no host wait).  More seed positions than one sort
+  // takes (2^32 - 1): the kept count is read first (the kept seeds are the ones
+  // its queries can join).
+  RefSeeds r;
+  uint64_t n_sort = N;
+  if (N < (1ull << 32)) {
+    r.d_nr = reinterpret_cast<const uint64_t*>(cnt);
+    r.nr = (int64_t)N;  // capacity
+  } else {
+    r.nr = (int64_t)fetch(c, cnt);
+    n_sort = (uint64_t)r.nr;
+  }
+  const bool small = c->tuning.sort_small_tiles != 0;
+  if (key32) {
+    const SortResult<uint32_t> x = radix_sort<uint32_t>((uint32_t*)keys, (uint32_t*)keys_alt, vals, vals_alt, n_sort,
+                                                        r.d_nr, 0, seed_key_bits, scratch, err, stream, small);
+    r.keys32 = x.keys;
+    r.vals = x.vals;
+  } else {
+    const SortResult<uint64_t> x = radix_sort<uint64_t>((uint64_t*)keys, (uint64_t*)keys_alt, vals, vals_alt, n_sort,
+                                                        r.d_nr, 0, seed_key_bits, scratch, err, stream, small);
+    r.keys = x.keys;
+    r.vals = x.vals;
+  }
+  return r;
 }
 
 void Search::start_early_ref() {
@@ -1278,37 +1352,9 @@ void Search::start_early_ref() {
     DRG_CUDA(cudaEventCreateWithFlags(&ev_qkeys, cudaEventDisableTiming));
     DRG_CUDA(cudaEventCreateWithFlags(&ev_ref, cudaEventDisableTiming));
   }
-  const auto ch = split_chunks(db->n, index_chunks);
-  early_c0 = ch[0].first;
-  early_c1 = ch[0].second;
-  const int S = (int)shapes.size();
-  const uint64_t lo = db->h_offsets[early_c0], hi = db->h_offsets[early_c1];
-  const uint64_t N = (hi - lo) * (uint64_t)S;
-  // every buffer first, on the host (a reallocation would wait for the device)
-  unsigned long long* cnt = c->seed_counts.as<unsigned long long>(2);
-  uint32_t* vals = c->r_vals.as<uint32_t>(N);
-  uint32_t* vs = c->r_vals_s.as<uint32_t>(N);
-  uint32_t* k32 = c->r_keys.as<uint32_t>(N);
-  uint32_t* ks32 = c->r_keys_s.as<uint32_t>(N);
-  uint32_t* err = c->sort_err.as<uint32_t>(1);
-  // the query seeds are enumerated and the bitmap set
-  DRG_CUDA(cudaEventRecord(ev_qkeys, c->stream));
-  DRG_CUDA(cudaStreamWaitEvent(c->side, ev_qkeys, 0));
-  // the first chunk's reference seeds the queries can join, sorted on their
-  // device-side count with the side stream's sort scratch
-  DRG_CUDA(cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), c->side));
-  launch_seed_enum_filtered(db->letters, db->offsets, db->owner + lo, lo, hi, S, key_filter, key_filter_log2, k32, vals,
-                            cnt, c->slot, c->side);
-  count_launch();
-  k_add_u64<<<1, 1, 0, c->side>>>(d_counters + 7, cnt + 1);
-  const uint64_t* d_nr = reinterpret_cast<const uint64_t*>(cnt);
-  const SortResult<uint32_t> r = radix_sort<uint32_t>(k32, ks32, vals, vs, N, d_nr, 0, seed_key_bits, c->sort_tmp_side,
-                                                      err, c->side, c->tuning.sort_small_tiles != 0);
+  early_chunks = merge ? chunks.size() : 1;
+  early = filtered_seeds(0, early_chunks, c->side, c->sort_tmp_side);
   DRG_CUDA(cudaEventRecord(ev_ref, c->side));
-  early_keys32_s = r.keys;
-  early_vals_s = r.vals;
-  early_nr = (int64_t)N;  // capacity; the count is d_nr
-  early_d_nr = d_nr;
   early_ref = true;
 }
 
@@ -1322,16 +1368,143 @@ void Search::build_key_filter(uint64_t n_runs) {
   key_filter_log2 = lg;
 }
 
-void Search::join_chunk(uint64_t c0, uint64_t c1, uint64_t n_runs) {
+// The join of all index chunks together: one sort, one count and one expansion
+// instead of one per chunk.  The expansion cap counts reference occurrences per
+// chunk (search.rs:127-131), so every (chunk, query run) has a range, a count
+// and hits of its own; equal keys lie in chunk order in the one sorted array
+// (or each chunk has its cached index).  The kernels of a small search wait on
+// launches: with the presets' four chunks 100 of 190 launches were the chunks'
+// (one query: 1.47 -> 1.11 ms; 20,000 short reads 6.0 -> 5.3 ms; 61 queries on a
+// cached index 3.65 -> 3.29 ms).  Falls back to one chunk after the other when the hits pass the budget, or a chunk's index is not
+// cached yet.
+bool Search::join_all(uint64_t n_runs) {
+  const size_t nc = chunks.size();
+  const bool from_cache = cached();
+  if (merge && from_cache) {
+    held.resize(nc);
+    for (; looked_up < nc; ++looked_up)
+      if (!(held[looked_up] = db->cache->find(index_key(chunks[looked_up].first, chunks[looked_up].second)))) {
+        ++looked_up;
+        merge = false;
+        break;
+      }
+  }
+  const uint64_t V = n_runs * nc;
+  if (!merge || V > kMergeRuns) {
+    if (early_ref && early_chunks > 1) {  // sorted for all chunks together: of no use to one
+      DRG_CUDA(cudaStreamWaitEvent(c->stream, ev_ref, 0));
+      early_ref = false;
+      DRG_CUDA(cudaMemsetAsync(d_counters + 7, 0, sizeof(unsigned long long), c->stream));
+    }
+    return false;
+  }
   Timer tm(c, &times);
+  tm.start();
+  RefSeeds ref;
+  if (early_ref) {
+    DRG_CUDA(cudaStreamWaitEvent(c->stream, ev_ref, 0));
+    early_ref = false;
+    ref = early;
+  } else if (!from_cache) {
+    if (!key_filter) build_key_filter(n_runs);
+    ref = filtered_seeds(0, nc, c->stream, c->sort_tmp);
+  }
+  uint32_t* rlo = c->run_rlo.as<uint32_t>(V + 1);
+  uint32_t* rcnt = c->run_rcount.as<uint32_t>(V + 1);
+  uint64_t* rhits = c->run_hits.as<uint64_t>(V + 1);
+  uint64_t* roff = c->run_hit_off.as<uint64_t>(V + 1);
+  const int bucket_bits = std::min(16, seed_key_bits);
+  const int shift = seed_key_bits - bucket_bits;
+  const uint32_t nb = 1u << bucket_bits;
+  const uint64_t key_mask = (1ull << seed_key_bits) - 1;
+  uint32_t* first = c->ref_first.as<uint32_t>(nb + 1);
+  const uint64_t* rk = c->run_keys.as<uint64_t>(0);
+  const uint32_t* rc = c->run_counts.as<uint32_t>(0);
+  JoinChunks jc{};
+  jc.n = (int)nc;
+  jc.n_runs = (uint32_t)n_runs;
+  for (size_t k = 0; k < nc; ++k) {
+    jc.end[k] = db->h_offsets[chunks[k].second];
+    jc.vals[k] = from_cache ? held[k]->vals : ref.vals;
+  }
+  auto count = [&](auto* keys, uint64_t nr, const uint64_t* d_nr, size_t k) {
+    launch_bucket_first(keys, nr, shift, nb, first, c->stream, d_nr);
+    if (from_cache)
+      launch_join_count(rk, rc, n_runs, keys, nr, 4096, rlo + k * n_runs, rcnt + k * n_runs, rhits + k * n_runs,
+                        key_mask, c->stream, first, shift, nullptr, d_nr);
+    else
+      launch_join_count_chunks(rk, rc, keys, jc, 4096, rlo, rcnt, rhits, key_mask, c->stream, first, shift);
+  };
+  for (size_t k = 0; k < (from_cache ? nc : 1); ++k) {
+    if (from_cache && held[k]->keys32) count(held[k]->keys32, held[k]->n, nullptr, k);
+    else if (from_cache) count(held[k]->keys, held[k]->n, nullptr, k);
+    else if (ref.keys32) count(ref.keys32, (uint64_t)ref.nr, ref.d_nr, k);
+    else count(ref.keys, (uint64_t)ref.nr, ref.d_nr, k);
+  }
+  count_launch();
+  k_set_u64<<<1, 1, 0, c->stream>>>(rhits + V, 0);
+  cub_call(c, [&](void* t, size_t& b) {
+    return cub::DeviceScan::ExclusiveSum(t, b, rhits, roff, (int64_t)V + 1, c->stream);
+  });
+  const uint64_t n_hits = fetch(c, roff + V);
+  if (n_hits > hit_budget) {
+    DRG_CUDA(cudaMemsetAsync(d_counters + 7, 0, sizeof(unsigned long long), c->stream));  // counted again per chunk
+    tm.stop(&st.ms_join);
+    return false;
+  }
+  if (from_cache) {
+    st.index_hits += nc;
+    for (const auto& h : held) st.ref_seeds += h->n;
+  }
+  expand_hits(n_hits, V, roff, c->run_qstart.as<uint32_t>(0), rlo, rcnt, nullptr, &jc);
+  query_blocks += nc;
+  tm.stop(&st.ms_join);
+  return true;
+}
+
+// Appends the hits of n_runs counted runs to acc.
+void Search::expand_hits(uint64_t n_hits, uint64_t n_runs, const uint64_t* roff, const uint32_t* qstart,
+                         const uint32_t* rlo, const uint32_t* rcnt, const uint32_t* r_vals, const JoinChunks* jc) {
+  st.hits += n_hits;
+  acc_reserve(acc_n + n_hits);
+  if (n_hits > 0) {
+    JoinExpandArgs ja{};
+    ja.run_hit_off = roff;
+    ja.coarse_shift = 7;  // one entry per 128 hits
+    uint32_t* coarse = c->hit_coarse.as<uint32_t>(((n_hits - 1) >> ja.coarse_shift) + 2);
+    launch_hit_coarse(roff, n_runs, ja.coarse_shift, n_hits, coarse, c->stream);
+    ja.coarse = coarse;
+    ja.run_qstart = qstart;
+    ja.run_rlo = rlo;
+    ja.run_rcount = rcnt;
+    ja.n_runs = n_runs;
+    ja.q_vals = c->q_vals_s.as<uint32_t>(0);
+    ja.r_vals = r_vals;
+    if (jc) ja.chunks = *jc;
+    ja.n_hits = n_hits;
+    ja.q_owner = q->owner;
+    ja.q_offsets = q->offsets;
+    ja.r_owner = db->owner;
+    ja.r_offsets = db->offsets;
+    ja.layout = layout();
+    ja.hit_keys = acc + acc_n;
+    launch_join_expand(ja, c->stream);
+  }
+  acc_n += n_hits;
+}
+
+void Search::join_chunk(size_t k, uint64_t n_runs) {
+  Timer tm(c, &times);
+  const auto [c0, c1] = chunks[k];
   const int S = (int)shapes.size();
   const uint64_t lo = db->h_offsets[c0], hi = db->h_offsets[c1];
-  const uint64_t N = (hi - lo) * (uint64_t)S;
+  const uint64_t N = positions(k, k + 1);
   // ---- reference seeds (or the database's cached index of them) + join
   tm.start();
-  IndexCache* cache = db->cache && db->cache->budget() > 0 ? db->cache.get() : nullptr;
+  IndexCache* cache = cached() ? db->cache.get() : nullptr;
   const std::string ikey = cache ? index_key(c0, c1) : std::string();
-  std::shared_ptr<SeedIndex> held = cache ? cache->find(ikey) : nullptr;  // kept until the join has read it
+  // kept until the join has read it
+  std::shared_ptr<SeedIndex> held = !cache ? nullptr : k < looked_up ? this->held[k] : cache->find(ikey);
   // A seed key of at most 32 bits is sorted as a 32-bit key: 8 bytes per
   // entry and pass instead of 12.
   const bool key32 = seed_key_bits <= 32;
@@ -1348,62 +1521,24 @@ void Search::join_chunk(uint64_t c0, uint64_t c1, uint64_t n_runs) {
     nr = (int64_t)held->n;
     n_valid = held->n;
     st.index_hits += 1;
-  } else if (!cache && early_ref && c0 == early_c0 && c1 == early_c1) {
-    // sorted on the side stream while the query seeds sorted
-    DRG_CUDA(cudaStreamWaitEvent(c->stream, ev_ref, 0));
-    early_ref = false;
-    keys32_s = early_keys32_s;
-    vals_s = early_vals_s;
-    nr = early_nr;
-    d_nr = early_d_nr;
   } else if (!cache) {
     // Nothing is kept for later searches, so only the seeds whose key the
     // query holds are sorted: the join pairs equal keys only (seed.rs:110-140),
     // so the rest cannot yield a hit or change a run's count.
-    if (!key_filter) build_key_filter(n_runs);
-    unsigned long long* cnt = c->seed_counts.as<unsigned long long>(2);
-    DRG_CUDA(cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), c->stream));
-    uint32_t* vals = c->r_vals.as<uint32_t>(N);
-    uint32_t* vs = c->r_vals_s.as<uint32_t>(N);
-    uint32_t *k32 = nullptr, *ks32 = nullptr;
-    uint64_t *k64 = nullptr, *ks64 = nullptr;
-    if (key32) {
-      k32 = c->r_keys.as<uint32_t>(N);
-      ks32 = c->r_keys_s.as<uint32_t>(N);
-      launch_seed_enum_filtered(db->letters, db->offsets, db->owner + lo, lo, hi, S, key_filter, key_filter_log2, k32,
-                                vals, cnt, c->slot, c->stream);
+    RefSeeds r;
+    if (early_ref && k == 0) {  // sorted on the side stream while the query seeds sorted
+      DRG_CUDA(cudaStreamWaitEvent(c->stream, ev_ref, 0));
+      early_ref = false;
+      r = early;
     } else {
-      k64 = c->r_keys.as<uint64_t>(N);
-      ks64 = c->r_keys_s.as<uint64_t>(N);
-      launch_seed_enum_filtered(db->letters, db->offsets, db->owner + lo, lo, hi, S, key_filter, key_filter_log2, k64,
-                                vals, cnt, c->slot, c->stream);
+      if (!key_filter) build_key_filter(n_runs);
+      r = filtered_seeds(k, k + 1, c->stream, c->sort_tmp);
     }
-    // the kept count stays on the device: the sort, the bucket starts and the
-    // join read it there (no host wait); the valid count joins the counters.
-    // A chunk with more seed positions than one sort takes (2^32 - 1) reads
-    // the kept count first (the kept seeds are the ones its queries can join).
-    count_launch();
-    k_add_u64<<<1, 1, 0, c->stream>>>(d_counters + 7, cnt + 1);
-    uint64_t n_sort = N;
-    if (N < (1ull << 32)) {
-      d_nr = reinterpret_cast<const uint64_t*>(cnt);
-      nr = (int64_t)N;  // capacity
-    } else {
-      nr = (int64_t)fetch(c, cnt);
-      n_sort = (uint64_t)nr;
-    }
-    if (key32) {
-      const SortResult<uint32_t> r = dsort(c, k32, ks32, vals, vs, n_sort, 0, seed_key_bits, d_nr);
-      ks32 = r.keys;
-      vs = r.vals;
-    } else {
-      const SortResult<uint64_t> r = dsort(c, k64, ks64, vals, vs, n_sort, 0, seed_key_bits, d_nr);
-      ks64 = r.keys;
-      vs = r.vals;
-    }
-    keys_s = ks64;
-    keys32_s = ks32;
-    vals_s = vs;
+    keys_s = r.keys;
+    keys32_s = r.keys32;
+    vals_s = r.vals;
+    nr = r.nr;
+    d_nr = r.d_nr;
   } else {
     uint32_t* vals = c->r_vals.as<uint32_t>(N);
     uint32_t* vs = c->r_vals_s.as<uint32_t>(N);
@@ -1460,31 +1595,7 @@ void Search::join_chunk(uint64_t c0, uint64_t c1, uint64_t n_runs) {
     return fetch(c, roff + n_runs);
   };
   auto expand = [&](uint64_t n_hits, const uint32_t* qstart) {
-    st.hits += n_hits;
-    acc_reserve(acc_n + n_hits);
-    if (n_hits > 0) {
-      JoinExpandArgs ja{};
-      ja.run_hit_off = roff;
-      ja.coarse_shift = 7;  // one entry per 128 hits
-      uint32_t* coarse = c->hit_coarse.as<uint32_t>(((n_hits - 1) >> ja.coarse_shift) + 2);
-      launch_hit_coarse(roff, n_runs, ja.coarse_shift, n_hits, coarse, c->stream);
-      ja.coarse = coarse;
-      ja.run_qstart = qstart;
-      ja.run_rlo = rlo;
-      ja.run_rcount = rcnt;
-      ja.n_runs = n_runs;
-      ja.q_vals = c->q_vals_s.as<uint32_t>(0);
-      ja.r_vals = vals_s;
-      ja.n_hits = n_hits;
-      ja.q_owner = q->owner;
-      ja.q_offsets = q->offsets;
-      ja.r_owner = db->owner;
-      ja.r_offsets = db->offsets;
-      ja.layout = layout();
-      ja.hit_keys = acc + acc_n;
-      launch_join_expand(ja, c->stream);
-    }
-    acc_n += n_hits;
+    expand_hits(n_hits, n_runs, roff, qstart, rlo, rcnt, vals_s, nullptr);
   };
   const uint64_t n_hits = scan_hits();
   if ((n_hits <= hit_budget || q->n == 1) && q->n <= t_window) {
@@ -1921,13 +2032,17 @@ void Search::run(drg_result* out) {
     return;
   }
   set_target_window();
+  chunks = split_chunks(db->n, index_chunks);
+  merge = chunks.size() >= 2 && chunks.size() <= (size_t)kJoinChunks && q->n <= t_window && hit_budget >= kMergeHits &&
+          (cached() || positions(0, chunks.size()) <= kMergePositions);
   Timer tm(c, &times);
   tm.start();
   uint64_t n_runs = 0;
   query_seeds(&n_runs);
   tm.stop(&st.ms_seed);
   if (n_runs > 0) {
-    for (auto [c0, c1] : split_chunks(db->n, index_chunks)) join_chunk(c0, c1, n_runs);
+    if (!join_all(n_runs))
+      for (size_t k = 0; k < chunks.size(); ++k) join_chunk(k, n_runs);
     process_hits(pass++);
   }
   if (early_ref) {  // no join read it: its buffers must not outlive this search's use of them

@@ -316,7 +316,10 @@ int onesweep_resident_blocks() {
 // end_bit) and its index make one 64-bit word (so equal keys keep their
 // order), sorted by a bitonic network: stages whose pairs lie 32 words apart
 // or less run in a warp's registers (64 words, shuffles), the others in shared
-// memory between block barriers.  What bounds such a sort is launches: TIMES
+// memory between block barriers.  What bounds such a sort is launches:
+// 22 / 1,438 / 4,096 keys of 42 bits take 2.8 / 11 / 23 us here; histogram, scan
+// and six onesweep passes over 4,097 take 60 us and seven host launches more.
+// (One query, whole search: 1.65 -> 1.47 ms.)
 constexpr int kSmallSort = 4096, kSmallBits = 52, kSmallThreads = 1024;
 template <typename K>
 __global__ void __launch_bounds__(kSmallThreads) k_sort_small(const K* __restrict__ kin, K* __restrict__ kout,

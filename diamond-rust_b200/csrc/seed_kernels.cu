@@ -323,8 +323,7 @@ void launch_key_filter(const uint64_t* run_keys, uint64_t n, uint64_t key_mask, 
 
 // One thread per letter as in k_seed_enum.  Kept seeds collect in shared
 // memory, kFilterGroup shapes at a time, and each block reserves its output
-// range with one atomic per group; counts[0] = seeds kept, counts[1] = valid
-// seeds (kept or not).  The output order depends on the blocks' timing; the
+// range with one atomic per group.  The output order depends on the blocks' timing; the
 // caller sorts by key, and the hits made from them are sorted in full later.
 constexpr int kFilterBlock = kEnumBlock, kFilterGroup = 8;
 
@@ -333,7 +332,8 @@ __global__ void __launch_bounds__(kFilterBlock)
     k_seed_enum_filtered(const uint8_t* __restrict__ letters, const uint64_t* __restrict__ offsets,
                          const uint32_t* __restrict__ owner, uint64_t lo, uint64_t hi, int n_shapes,
                          const uint32_t* __restrict__ filter, int log2_bits, K* __restrict__ keys,
-                         uint32_t* __restrict__ vals, unsigned long long* __restrict__ counts, int slot) {
+                         uint32_t* __restrict__ vals, unsigned long long* __restrict__ kept,
+                         unsigned long long* __restrict__ n_valid, int slot) {
   __shared__ EnumTables tab;
   __shared__ K s_keys[kFilterBlock * kFilterGroup];
   __shared__ uint32_t s_vals[kFilterBlock * kFilterGroup];
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kFilterBlock)
     }
     __syncthreads();
     const uint32_t n = s_n;
-    if (threadIdx.x == 0 && n > 0) s_base = atomicAdd(counts, (unsigned long long)n);
+    if (threadIdx.x == 0 && n > 0) s_base = atomicAdd(kept, (unsigned long long)n);
     __syncthreads();  // every thread has read s_n and can see s_base
     const unsigned long long base = s_base;
     if (threadIdx.x == 0) s_n = 0;
@@ -382,30 +382,30 @@ __global__ void __launch_bounds__(kFilterBlock)
   for (int o = 16; o > 0; o >>= 1) valid += __shfl_xor_sync(0xFFFFFFFFu, valid, o);
   if ((threadIdx.x & 31) == 0 && valid) atomicAdd(&s_valid, valid);
   __syncthreads();
-  if (threadIdx.x == 0 && s_valid) atomicAdd(counts + 1, s_valid);
+  if (threadIdx.x == 0 && s_valid) atomicAdd(n_valid, s_valid);
 }
 
 template <typename K>
 void seed_enum_filtered(const uint8_t* letters, const uint64_t* offsets, const uint32_t* owner, uint64_t lo,
                         uint64_t hi, int n_shapes, const uint32_t* filter, int log2_bits, K* keys, uint32_t* vals,
-                        unsigned long long* counts, int slot, cudaStream_t st) {
+                        unsigned long long* kept, unsigned long long* valid, int slot, cudaStream_t st) {
   if (hi <= lo || n_shapes == 0) return;
   count_launch();
   k_seed_enum_filtered<K><<<ceil_div(hi - lo, kFilterBlock), kFilterBlock, 0, st>>>(
-      letters, offsets, owner, lo, hi, n_shapes, filter, log2_bits, keys, vals, counts, slot);
+      letters, offsets, owner, lo, hi, n_shapes, filter, log2_bits, keys, vals, kept, valid, slot);
   DRG_CUDA(cudaGetLastError());
 }
 
 void launch_seed_enum_filtered(const uint8_t* letters, const uint64_t* offsets, const uint32_t* owner, uint64_t lo,
                                uint64_t hi, int n_shapes, const uint32_t* filter, int log2_bits, uint64_t* keys,
-                               uint32_t* vals, unsigned long long* counts, int slot, cudaStream_t st) {
-  seed_enum_filtered(letters, offsets, owner, lo, hi, n_shapes, filter, log2_bits, keys, vals, counts, slot, st);
+                               uint32_t* vals, unsigned long long* kept, unsigned long long* valid, int slot, cudaStream_t st) {
+  seed_enum_filtered(letters, offsets, owner, lo, hi, n_shapes, filter, log2_bits, keys, vals, kept, valid, slot, st);
 }
 
 void launch_seed_enum_filtered(const uint8_t* letters, const uint64_t* offsets, const uint32_t* owner, uint64_t lo,
                                uint64_t hi, int n_shapes, const uint32_t* filter, int log2_bits, uint32_t* keys,
-                               uint32_t* vals, unsigned long long* counts, int slot, cudaStream_t st) {
-  seed_enum_filtered(letters, offsets, owner, lo, hi, n_shapes, filter, log2_bits, keys, vals, counts, slot, st);
+                               uint32_t* vals, unsigned long long* kept, unsigned long long* valid, int slot, cudaStream_t st) {
+  seed_enum_filtered(letters, offsets, owner, lo, hi, n_shapes, filter, log2_bits, keys, vals, kept, valid, slot, st);
 }
 
 // first[b] = the first of n sorted keys with key >> shift >= b, for b in
@@ -498,6 +498,77 @@ __global__ void k_join_count(const uint64_t* __restrict__ run_keys, const uint32
   }
   // the cap sees the whole run's count (seed.rs:120-127)
   run_hits[u] = (rc > 0 && qc * rc <= max_expand) ? qb * rc : 0;
+}
+
+// One thread per query run: the range of its key in the bucket, then (equal
+// keys lie in chunk order) where each chunk's share of it ends.
+template <typename K>
+__global__ void k_join_count_chunks(const uint64_t* __restrict__ run_keys, const uint32_t* __restrict__ run_counts,
+                                    const K* __restrict__ ref_keys, JoinChunks jc, uint64_t max_expand,
+                                    uint32_t* __restrict__ run_rlo, uint32_t* __restrict__ run_rcount,
+                                    uint64_t* __restrict__ run_hits, uint64_t key_mask,
+                                    const uint32_t* __restrict__ first, int shift) {
+  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= jc.n_runs) return;
+  const uint64_t key = run_keys[u] & key_mask;
+  uint64_t a = first[key >> shift], b = first[(key >> shift) + 1];
+  const uint64_t end = b;
+  while (a < b) {  // lower bound
+    const uint64_t m = (a + b) >> 1;
+    if ((uint64_t)ref_keys[m] < key) a = m + 1;
+    else b = m;
+  }
+  uint64_t lo = a;
+  b = end;
+  while (a < b) {  // upper bound
+    const uint64_t m = (a + b) >> 1;
+    if ((uint64_t)ref_keys[m] <= key) a = m + 1;
+    else b = m;
+  }
+  const uint64_t hi = a, qc = run_counts[u];
+  const uint32_t* vals = jc.vals[0];
+  for (int x = 0; x < jc.n; ++x) {
+    uint64_t e = hi;
+    if (x + 1 < jc.n && lo < hi) {
+      uint64_t y = lo;
+      while (y < e) {  // first entry past the chunk
+        const uint64_t m = (y + e) >> 1;
+        if (vals[m] < jc.end[x]) y = m + 1;
+        else e = m;
+      }
+    }
+    const uint64_t rc = e - lo, v = (uint64_t)x * jc.n_runs + u;
+    run_rlo[v] = (uint32_t)lo;
+    run_rcount[v] = (uint32_t)rc;
+    run_hits[v] = (rc > 0 && qc * rc <= max_expand) ? qc * rc : 0;
+    lo = e;
+  }
+}
+template <typename K>
+static void join_count_chunks(const uint64_t* run_keys, const uint32_t* run_counts, const K* ref_keys,
+                              const JoinChunks& jc, uint64_t max_expand, uint32_t* run_rlo, uint32_t* run_rcount,
+                              uint64_t* run_hits, uint64_t key_mask, cudaStream_t st, const uint32_t* first,
+                              int shift) {
+  if (jc.n_runs == 0) return;
+  count_launch();
+  k_join_count_chunks<K><<<ceil_div(jc.n_runs, 256), 256, 0, st>>>(run_keys, run_counts, ref_keys, jc, max_expand,
+                                                                   run_rlo, run_rcount, run_hits, key_mask, first,
+                                                                   shift);
+  DRG_CUDA(cudaGetLastError());
+}
+void launch_join_count_chunks(const uint64_t* run_keys, const uint32_t* run_counts, const uint64_t* ref_keys,
+                              const JoinChunks& jc, uint64_t max_expand, uint32_t* run_rlo, uint32_t* run_rcount,
+                              uint64_t* run_hits, uint64_t key_mask, cudaStream_t st, const uint32_t* first,
+                              int shift) {
+  join_count_chunks(run_keys, run_counts, ref_keys, jc, max_expand, run_rlo, run_rcount, run_hits, key_mask, st, first,
+                    shift);
+}
+void launch_join_count_chunks(const uint64_t* run_keys, const uint32_t* run_counts, const uint32_t* ref_keys,
+                              const JoinChunks& jc, uint64_t max_expand, uint32_t* run_rlo, uint32_t* run_rcount,
+                              uint64_t* run_hits, uint64_t key_mask, cudaStream_t st, const uint32_t* first,
+                              int shift) {
+  join_count_chunks(run_keys, run_counts, ref_keys, jc, max_expand, run_rlo, run_rcount, run_hits, key_mask, st, first,
+                    shift);
 }
 
 // One thread per query run: each entry of a run that passes the cap adds
@@ -595,8 +666,15 @@ __global__ void k_join_expand(JoinExpandArgs a) {
   uint64_t u = lo;
   uint64_t k = h - a.run_hit_off[u];
   uint32_t rc = a.run_rcount[u];
-  uint64_t qi = a.run_qstart[u] + k / rc;
-  uint64_t ri = a.run_rlo[u] + k % rc;
+  uint32_t run = (uint32_t)u;
+  const uint32_t* r_vals = a.r_vals;
+  if (a.chunks.n > 0) {  // (chunk, run) entries
+    const uint32_t x = run / a.chunks.n_runs;
+    run -= x * a.chunks.n_runs;
+    r_vals = a.chunks.vals[x];
+  }
+  const uint64_t qi = a.run_qstart[run] + k / rc;
+  const uint64_t ri = a.run_rlo[u] + k % rc;
   uint32_t t, s;
   int64_t qpos, spos;
   if (a.q_entries) {
@@ -610,7 +688,7 @@ __global__ void k_join_expand(JoinExpandArgs a) {
       return;
     }
   } else {
-    const uint32_t qg = a.q_vals[qi], rg = a.r_vals[ri];
+    const uint32_t qg = a.q_vals[qi], rg = r_vals[ri];
     t = a.q_owner[qg];
     s = a.r_owner[rg];
     qpos = (int64_t)qg - (int64_t)a.q_offsets[t];
