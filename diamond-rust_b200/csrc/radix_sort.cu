@@ -9,8 +9,8 @@
 //   k_radix_scan    exclusive scan of each pass's 256 digit counts
 //   k_onesweep      one persistent launch per 8-bit digit: a tile of 256
 //                   threads x ITEMS keys is loaded with 128-bit loads through
-//                   shared memory, ranked stably (per-warp __match_any_sync,
-//                   then a scan over warps), its global position per digit
+//                   shared memory, ranked stably (ballots per warp, then a
+//                   scan over warps), its global position per digit
 //                   found by decoupled look-back over the preceding tiles
 //                   (words tagged with the pass's epoch, so the look-back
 //                   area is never cleared between passes), and
@@ -152,6 +152,27 @@ __device__ __forceinline__ void load_tile(const K* __restrict__ src, uint64_t ba
   }
 }
 
+// The lanes whose 8-bit digit equals this lane's: a ballot per bit, four
+// instructions each (the compiler's form of the same loop takes thirteen).
+// match.any runs on the ADU pipe, some 34 cycles an instruction and SM, which
+// bounded a pass (ncu: ADU 48 %, issue 19 %).  Per pass, by match.any / this, with
+// the values loaded ahead of the look-back: 5.75M u32 pairs 78.7 / 51.5 us,
+// 13.4M u64 pairs 192 / 140, 2.8M u64 keys 42.6 / 31.6.
+__device__ __forceinline__ uint32_t same_digit(uint32_t d) {
+  uint32_t peers = 0xFFFFFFFFu;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    uint32_t same;  // the lanes whose bit b equals this lane's
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tand.b32 t, %1, %2;\n\tsetp.ne.u32 p, t, 0;\n\t"
+        "vote.sync.ballot.b32 %0, p, 0xffffffff;\n\t@!p not.b32 %0, %0;\n\t}"
+        : "=r"(same)
+        : "r"(d), "r"(1u << b));
+    peers &= same;
+  }
+  return peers;
+}
+
 // One tile of one digit pass (s.warp_cnt zeroed, tile < tiles of the count).
 template <typename K, bool VALS, bool SMALL>
 __device__ __forceinline__ void onesweep_tile(OnesweepShared<K, VALS, SMALL>& s, uint32_t tile, uint64_t n,
@@ -186,7 +207,7 @@ __device__ __forceinline__ void onesweep_tile(OnesweepShared<K, VALS, SMALL>& s,
   const uint32_t lt = (1u << lane) - 1;
 #pragma unroll
   for (int j = 0; j < kItems; ++j) {
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, dig[j]);
+    const uint32_t peers = same_digit(dig[j]);
     const uint32_t before = s.warp_cnt[w][dig[j]];
     __syncwarp();
     if ((peers & lt) == 0) s.warp_cnt[w][dig[j]] = before + __popc(peers);
@@ -215,6 +236,15 @@ __device__ __forceinline__ void onesweep_tile(OnesweepShared<K, VALS, SMALL>& s,
   for (int i = 0; i < w; ++i) local_start += s.scan_tot[i];
 #pragma unroll
   for (int i = 0; i < kSortWarps; ++i) s.warp_cnt[i][t] += local_start;
+  // the values' loads are in flight during the look-back
+  uint32_t val[VALS ? kItems : 1];
+  if (VALS) {
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+      const int e = w * 32 * kItems + j * 32 + lane;
+      val[j] = e < valid ? vin[base + e] : 0u;
+    }
+  }
   // ---- decoupled look-back: this tile's count of digit t, and the counts of
   // the tiles before it
   const uint32_t mine = count - (t == kBins - 1 ? (uint32_t)(kTile - valid) : 0u);
@@ -263,7 +293,7 @@ __device__ __forceinline__ void onesweep_tile(OnesweepShared<K, VALS, SMALL>& s,
 #pragma unroll
   for (int j = 0; j < kItems; ++j) {
     const int e = w * 32 * kItems + j * 32 + lane;
-    if (e < valid) s.stage.vals[pos[j]] = vin[base + e];
+    if (e < valid) s.stage.vals[pos[j]] = val[j];
   }
   __syncthreads();
   for (int i = t; i < valid; i += kSortThreads) {
