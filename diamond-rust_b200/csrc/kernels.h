@@ -332,14 +332,10 @@ constexpr int kSwMinWidth = 17;   // narrower bands use the exact kernel
 constexpr int kSwC0 = 136, kSwC1 = 272, kSwC2 = 544, kSwC3 = 1700;
 constexpr int kSwClassMax[4] = {kSwC0, kSwC1, kSwC2, kSwC3};  // 4, 2, 1, 1 warps per block
 constexpr int kSwMaxWidth = 1700;                       // wider bands use the exact kernel
-// The packed kernel's profile bytes hold a score plus the open cost (gap open
-// + extend): with larger open costs its bands go to the band kernel.
-constexpr int kSwMaxOpenCost = 64;
 // Bands whose best can reach this bound are not packed: every H of the packed
 // kernel stays below 0x7C00 (its strip maximum folds H on the FMA pipe as
 // half-precision bit patterns) and far from the 16-bit limit.
 constexpr int kSwPackedMaxBest = 31743;
-constexpr int kSwBandMinWidth = kSwC1 + 1;  // score pass: wider bands run one warp per band
 constexpr int kSwClasses = 4;
 int sw_width_class(int width);  // 0..3, or -1 for the exact kernel
 void launch_sw_class(const SwScoreArgs& a, int cls, cudaStream_t st);  // score mode

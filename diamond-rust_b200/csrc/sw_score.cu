@@ -8,26 +8,33 @@
 // in the band for r <= c <= r + W - 1.  The 16 rows are held as 8 pairs of
 // signed 16-bit lanes (DPX s16x2 instructions): pair p holds row p at column c
 // in its low half and row p + 8 at column c - 1 in its high half.  With that
-// one-column skew every dependency of a pair is already computed:
-//   D(i,j) = H(i-1,j-1) + S                        previous step, pair above
-//   E(i,j) = max(E(i-1,j) - ge, H(i-1,j) - oc)      this step, pair above
-//   F(i,j) = max(F(i,j-1) - ge, H(i,j-1) - oc)      previous step, same pair
-//   H      = max(0, D, E, F)
+// one-column skew every dependency of a pair is already computed.  The gap
+// scores are kept with the cost of a gap's first letter added back (oc):
+//   E'(i,j) = E + oc = max(E'(i-1,j) - ge, H(i-1,j))   this step, pair above
+//   F'(i,j) = F + oc = max(F'(i,j-1) - ge, H(i,j-1))   previous step, same pair
+//   H       = max(0, H(i-1,j-1) + S, max(E', F') - oc)
 // Row 8's "pair above" is row 7, taken from the previous step; row 0's is the
 // previous strip's last row, kept in a per-thread ring in shared memory.  The
-// ring holds W + 1 words (H - oc | E << 16): a strip reads the previous
-// strip's word for column c and then overwrites the slot of column c - 1,
-// which is the word the next strip needs at its column c - 17.
+// ring holds W + 1 words (H | E' << 16): a strip reads the previous strip's
+// word for column c and then overwrites the slot of column c - 1, which is the
+// word the next strip needs at its column c - 17.
 //
-// A pair update is five half-rate DPX/PRMT operations and one full-rate max:
+// In this form all of H, E' and F' are at least 0, no H - oc is kept, and a
+// cell outside the band or the matrix is plain 0 (E' = 0 is E = -oc, which
+// raises nothing).  A pair update is six half-rate ALU operations, of which
+// only the last two wait for the pair above:
 //   sc = the pair's two scores (one byte permute)
-//   F  = max(F - ge, H - oc)            (viaddmax)
-//   X  = max(D, F, 0)                   (viaddmax.relu: D = Hdiag + sc fused)
-//   E  = max(E - ge, H - oc)            (viaddmax, the step's vertical chain)
-//   H  = max(X, E)                      (max.s16x2, full rate)
-//   H - oc                              (add, shared by the next E and F)
-// Pair 0's diagonal operand comes from the ring and row 7 in the H - oc form
-// (that is what the ring keeps), so the profile rows 0 and 8 carry + oc.
+//   X  = max(F' - oc, Hdiag + sc, 0)   (add, viaddmax.relu)
+//   E' = max(E' - ge, H of the pair above)   (viaddmax)
+//   H  = max(E' - oc, X)               (viaddmax)
+//   F' = max(F' - ge, H)               (viaddmax, for the next column)
+// ALU bound, then by the chain of E' and H down the pairs.  The residues are
+// loaded four columns ahead of their use.  Against the same cell with H - oc
+// kept beside H and residues two columns ahead: 18.05 -> 17.75 ms for the
+// 1,000-query sensitive search, 15.60 -> 15.27 for 250 very-sensitive queries.
+// One operation less on the ALU pipe, G = max(E', F') as a half-precision
+// maximum and H = max(G - oc, D, 0), is slower (17.98 ms): the maximum
+// lengthens the chain.
 //
 // Exactness: values equal the reference's int32 DP while the band's best is
 // below 31744 = 0x7C00 (bands that could reach it are not given to this
@@ -39,7 +46,7 @@
 // max(largest matrix score, band best - open), so a packed best above the
 // matrix's largest score is the reference's; smaller results are recomputed
 // exactly.  Cells left or right of the band in the first/last 16 steps of
-// a strip are masked: their H does not count and they pass -inf-like E/F.
+// a strip are masked to 0: their H does not count and they pass no gap.
 //
 // The traceback of the HSPs that pass the gate runs in sw_sys.cu.
 #include "kernels.h"
@@ -53,9 +60,9 @@ using namespace sw;
 
 // Registers of one lane's 16-row strip in the score pass.
 struct SRegs {
-  uint32_t H[kPairs], Hm[kPairs], F[kPairs];
-  uint32_t E7;        // E of pair 7 at the previous step
-  uint32_t hmtop_old; // H - oc above pair 0 at the previous step (its D operand, profile + oc)
+  uint32_t H[kPairs], F[kPairs];
+  uint32_t E7;        // E' of pair 7 at the previous step
+  uint32_t htop_old;  // H above pair 0 at the previous step (its D operand)
   const uint8_t* prow_prev;  // profile row of the previous column's residue
   uint32_t mx0, mx1;  // maximum H of the strip so far, folded over rows
 };
@@ -64,8 +71,8 @@ struct SRegs {
 // C (= c), 2: epilogue step C (= c - W) of a warp whose bands share one
 // width, 3: step past the narrowest band of a warp with mixed widths
 // (cw = c - this lane's W, masks computed at run time).  rp holds the
-// (H - oc, E) word of the row above row 0 at column c; wp receives row 15's
-// word of column c - 1.
+// (H, E') word of the row above row 0 at column c; wp receives row 15's word of
+// column c - 1.
 template <int MODE, int C>
 __device__ __forceinline__ void sw_step(SRegs& R, Lane& L, int c, const uint8_t* __restrict__ prof,
                                         const uint32_t* __restrict__ rp, uint32_t* __restrict__ wp, uint32_t noc2,
@@ -75,42 +82,39 @@ __device__ __forceinline__ void sw_step(SRegs& R, Lane& L, int c, const uint8_t*
   const uint2 lo8 = *reinterpret_cast<const uint2*>(prow);
   const uint2 hi8 = *reinterpret_cast<const uint2*>(R.prow_prev + 8);
   R.prow_prev = prow;
-  const uint32_t rw = *rp;  // (H - oc, E) of the row above row 0, column c
-  const uint32_t hm_top = prmt(rw, R.Hm[kPairs - 1], 0x5410);
-  uint32_t hm_up = hm_top;
+  const uint32_t rw = *rp;  // (H, E') of the row above row 0, column c
+  const uint32_t h_top = prmt(rw, R.H[kPairs - 1], 0x5410);
+  uint32_t h_up = h_top;
   uint32_t e_up = prmt(rw, R.E7, 0x5432);
-  uint32_t hd = R.hmtop_old;
+  uint32_t hd = R.htop_old;
 #pragma unroll
   for (int p = 0; p < kPairs; ++p) {
     // Pairs whose two halves are both outside the band at this compile-time
     // step are not computed: left of it in the prologue (C < p), right of it
     // in a one-width epilogue (C >= p + 9).  They take the values the masks
-    // below would give (H = 0, H - oc = -oc, F = -inf) and hand the next
-    // pair the same E/H the masked computation would; in the prologue every
-    // pair below is skipped too, and the E of pair 7 is first read by row 8
-    // at step 9, when pair 7 is computed again.
+    // below would give (0) and hand the next pair the same E/H the masked
+    // computation would; in the prologue every pair below is skipped too, and
+    // the E' of pair 7 is first read by row 8 at step 9, when pair 7 is
+    // computed again.
     if ((MODE == 1 && C < p) || (MODE == 2 && C >= p + 9)) {
       hd = R.H[p];
       R.H[p] = 0;
-      R.Hm[p] = noc2;
-      R.F[p] = kNeg2;
-      hm_up = noc2;
-      e_up = kNeg2;
+      R.F[p] = 0;
+      h_up = 0;
+      e_up = 0;
       continue;
     }
     const uint32_t sc = prmt(p < 4 ? lo8.x : lo8.y, p < 4 ? hi8.x : hi8.y, pick_sel(p & 3));
-    uint32_t f = __viaddmax_s16x2(R.F[p], nge2, R.Hm[p]);
-    const uint32_t x = __viaddmax_s16x2_relu(hd, sc, f);  // max(D, F, 0)
-    uint32_t e = __viaddmax_s16x2(e_up, nge2, hm_up);
-    uint32_t h = max2(x, e);
+    uint32_t f = R.F[p];
+    uint32_t e = __viaddmax_s16x2(e_up, nge2, h_up);
+    uint32_t h = __viaddmax_s16x2(e, noc2, __viaddmax_s16x2_relu(f, noc2, add2(hd, sc)));
     if (MODE == 1) {
       // left of the band: row p at column C (low), row p+8 at column C-1 (high)
       const bool lo_left = C < p;
       const bool hi_left = C <= p + 8;
       const uint32_t k = (lo_left ? 0u : 0x0000FFFFu) | (hi_left ? 0u : 0xFFFF0000u);
       if (k != 0xFFFFFFFFu) {
-        h = h & k;  // no score; H - oc = -oc toward the entry cell
-        f = sel2(f, k, kNeg2);
+        h = h & k;  // no score toward the entry cell (F' is 0 there already)
       }
     } else if (MODE == 2) {
       const bool lo_right = C >= p;
@@ -118,20 +122,18 @@ __device__ __forceinline__ void sw_step(SRegs& R, Lane& L, int c, const uint8_t*
       const uint32_t k = (lo_right ? 0u : 0x0000FFFFu) | (hi_right ? 0u : 0xFFFF0000u);
       if (k != 0xFFFFFFFFu) {
         h = h & k;
-        e = sel2(e, k, kNeg2);
+        e = e & k;
       }
     } else if (MODE == 3) {
       // right of this lane's band: row p at column c (low), row p+8 at column c-1 (high)
       const uint32_t k = (cw >= p ? 0u : 0x0000FFFFu) | (cw >= p + 9 ? 0u : 0xFFFF0000u);
       h = h & k;
-      e = sel2(e, k, kNeg2);
+      e = e & k;
     }
-    const uint32_t hm = add2(h, noc2);
     hd = R.H[p];
     R.H[p] = h;
-    R.Hm[p] = hm;
-    R.F[p] = f;
-    hm_up = hm;
+    R.F[p] = __viaddmax_s16x2(f, nge2, h);
+    h_up = h;
     e_up = e;
   }
   // the strip's maximum, two accumulators of four pairs each, on the FMA
@@ -141,8 +143,8 @@ __device__ __forceinline__ void sw_step(SRegs& R, Lane& L, int c, const uint8_t*
   R.mx0 = max2_pos_f16(R.mx0, max2_pos_f16(R.H[2], R.H[3]));
   R.mx1 = max2_pos_f16(R.mx1, max2_pos_f16(R.H[6], R.H[7]));
   R.E7 = e_up;
-  *wp = prmt(R.Hm[kPairs - 1], R.E7, 0x7632);  // (H - oc, E) of row 15 at column c - 1
-  R.hmtop_old = hm_top;
+  *wp = prmt(R.H[kPairs - 1], R.E7, 0x7632);  // (H, E') of row 15 at column c - 1
+  R.htop_old = h_top;
 }
 
 // The ring of one lane: W + 1 words at stride `stride`; rp reads column c,
@@ -211,15 +213,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
   Lane L;
   L.s = tr ? qw : sj;  // column letters
   L.m = tr ? (int)band.n : m_s;
-  const int oc = a.gap_open + a.gap_extend;  // at most kSwMaxOpenCost (profile bytes carry it)
-  const uint32_t noc2 = (uint32_t)(uint16_t)(-oc) * 0x10001u;
+  const uint32_t noc2 = (uint32_t)(uint16_t)(-(a.gap_open + a.gap_extend)) * 0x10001u;
   const uint32_t nge2 = (uint32_t)(uint16_t)(-a.gap_extend) * 0x10001u;
-  // dead cell word: H = 0 (H - oc = -oc), E = -inf
-  const uint32_t dead = 0xC0000000u | (noc2 & 0xFFFFu);
-  // the row above the first strip is row 0 of the reference: H = 0, and its
-  // E is -inf; column Wl - 1 is outside row 0's band on the right.
-  for (int g = 0; g < buf; ++g) ring[g * stride] = dead;
-  ring[(Wl - 1) * stride] = kNeg2;
+  // a dead cell's word is 0 (H = 0, E' = 0); the row above the first strip, row
+  // 0 of the reference, is dead
+  for (int g = 0; g < buf; ++g) ring[g * stride] = 0;
   RingPtr rg;
   rg.begin = ring;
   rg.end = ring + buf * stride;
@@ -231,8 +229,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
   for (uint32_t k = 0; k < task.n_strips; ++k) {
     const int i0 = (int)task.row_first + (int)(k * kRows);
     // strip profile: prof[res * stride + r] = S(query letter, subject letter)
-    // of row i0 + r against column residue res, + oc in rows 0 and 8 (their
-    // diagonal operand is H - oc)
+    // of row i0 + r against column residue res
     __syncwarp();
     for (int e = lane; e < 26 * kRows; e += 32) {
       int res = e >> 4, r = e & 15;
@@ -243,21 +240,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
         const int row = (int)min((uint32_t)q[i - 1], 24u);
         v = tr ? mat[res * 25 + row] : mat[row * 25 + res];
       }
-      if ((r & 7) == 0) v += oc;
       prof[res * kProfStride + r] = (uint8_t)(int8_t)v;
     }
     __syncwarp();
     L.jbase = i0 - d1;
-    // column c_begin - 1 of the strip: dead cells (H = 0, so H - oc = -oc,
-    // which is also pair 0's diagonal operand and row 8's E source)
+    // column c_begin - 1 of the strip: dead cells
 #pragma unroll
-    for (int p = 0; p < kPairs; ++p) {
-      R.H[p] = 0;
-      R.Hm[p] = noc2;
-      R.F[p] = kNeg2;
-    }
+    for (int p = 0; p < kPairs; ++p) R.H[p] = R.F[p] = 0;
     R.mx0 = R.mx1 = 0;
-    R.E7 = kNeg2;
+    R.E7 = 0;
     // Steps whose cells all lie off the matrix for every lane of the warp are
     // skipped: at step c a lane's cells sit at subject columns jbase + c (rows
     // 0-7) and jbase + c - 1 (rows 8-15), all j <= 0 for c <= -jbase and all
@@ -275,13 +266,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
       rg.rp = ring + slot * stride;
       rg.wp = ring + (slot == 0 ? buf - 1 : slot - 1) * stride;
     }
-    // H - oc of column c_begin - 1 of the row above; row 7 not yet computed: H = 0
-    R.hmtop_old = (*rg.wp & 0xFFFFu) | (noc2 & 0xFFFF0000u);
+    // H of column c_begin - 1 of the row above; row 7 not yet computed: 0
+    R.htop_old = *rg.wp & 0xFFFFu;
     {
       const int jm1 = L.jbase + c_begin - 2;  // column c_begin - 1
       R.prow_prev = prof + subject_residue(L, jm1) * kProfStride;
-      L.r0 = subject_residue(L, jm1 + 1);  // columns c_begin and c_begin + 1
-      L.r1 = subject_residue(L, jm1 + 2);
+#pragma unroll
+      for (int i = 0; i < kQueue; ++i) L.queue[i] = subject_residue(L, jm1 + 1 + i);
     }
     int c = c_begin;
     if (c_begin == 0) {
@@ -317,12 +308,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
     }
     // Ring words the next strip may read that this strip did not write: the
     // next strip's column x reads this strip's column x + 16.  Skipped columns
-    // on the left hold dead cells (H = 0, E = -inf); past the early stop the
-    // next strip computes only off-matrix cells, which must see -inf.
+    // on the left hold dead cells, and so do those past the early stop, where
+    // the next strip computes only off-matrix cells.
     for (int x = kRows - 1; x <= c_begin - 2; ++x) {
       int ls = base + x;
       ls = ls >= buf ? ls - buf : ls;
-      ring[ls * stride] = dead;
+      ring[ls * stride] = 0;
     }
     if (c_end < W + kRows) {
       const int x_hi = min(W + kRows - 1, max(c_end - 1, 2 * kRows - 1));
@@ -330,16 +321,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
         int ls = base + x;
         ls = ls >= buf ? ls - buf : ls;
         ls = ls >= buf ? ls - buf : ls;
-        ring[ls * stride] = kNeg2;
+        ring[ls * stride] = 0;
       }
     }
     // this lane's column Wl + 15 is the next strip's column Wl - 1: outside
-    // the band on the right, its E/H must read as -inf.
+    // the band on the right.
     {
       int ls = base + Wl + kRows - 1;
       ls = ls >= buf ? ls - buf : ls;
       ls = ls >= buf ? ls - buf : ls;
-      ring[ls * stride] = kNeg2;
+      ring[ls * stride] = 0;
     }
     base += kRows;
     if (base >= buf) base -= buf;
@@ -396,6 +387,5 @@ void launch_sw_class(const SwScoreArgs& a, int cls, cudaStream_t st) {
     default: launch_class<1>(a, kSwClassMax[3], st); break;
   }
 }
-
 
 }  // namespace drg
