@@ -268,10 +268,11 @@ struct BandArgs {
 void launch_build_bands(const BandArgs& a, cudaStream_t st);
 
 // ---- banded Smith-Waterman, score only (sw_score.cu) -----------------------
-struct SwTask {        // one warp: up to 32 bands sharing a query window
+constexpr int kSwPart = 16;  // bands of a task at most: the lanes of a half warp
+struct SwTask {        // part of a warp: up to kSwPart bands sharing a query window
   uint32_t first;      // index of the first band in the sorted band order
-  uint32_t count;      // 1..32
-  uint32_t row_first;  // first DP row of the warp (1-based)
+  uint32_t count;      // 1..kSwPart
+  uint32_t row_first;  // first DP row of the task (1-based)
   uint32_t n_strips;   // 16-row strips to run
   uint32_t width;      // widest band of the task, W_max = d1 - d0 + 1
   uint32_t w_min;      // narrowest band of the task

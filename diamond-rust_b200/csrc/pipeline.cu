@@ -6,7 +6,7 @@
 //   hits    radix sort by (target, subject, diagonal, spos), de-duplicate
 //   xdrop   one thread per (target, subject, diagonal) run, cutoff 19
 //   bands   one thread per pair: merge, order, window (search.rs:206-230, 303-312)
-//   sw      packed 16-bit banded SW scores (warp = 32 bands of one query)
+//   sw      packed 16-bit banded SW scores (half warp = 16 bands of one query)
 //   gate    ALP E-value and the max_hsps band walk per pair
 // Host: exact E-values of the kept bands, per-target culling (search.rs:256-270),
 // then the exact traceback kernel for the surviving HSPs only.
@@ -141,6 +141,7 @@ struct SwKeyBits {
 // Task and band-job sort keys: class or route (< 8) above a cost field whose
 // inverse orders longest first; the order only schedules, so costs saturate.
 constexpr int kCostBits = 21;  // 2M column steps: above any warp but the rarest, so the keys sort in 3 passes
+constexpr int kCornerBits = 8;
 constexpr uint64_t kCostMax = (1ull << kCostBits) - 1;
 // Transposed warps (full, their rows a short subject) stay up to this chain.
 constexpr uint64_t kTransposedChain = 4096;
@@ -235,22 +236,22 @@ __device__ __forceinline__ SwRoute sw_route(const Band& b, const uint64_t* s_off
          (r.te - r.ts + 16) / 16 < (r.re - r.rs + 16) / 16;
   return r;
 }
-// Which warps of the packed kernel are given up.  A warp of k_sw runs 32
-// bands, one per lane, strip after strip: steps = strips x (W + 16), over the
-// union of its bands' rows and its widest band, at the same cost for 1 band as
-// for 32.  The lane kernel (k_sys_pair) takes two bands per warp, a step per
-// row and a quarter.  A warp's bands go there
+// Which tasks of the packed kernel are given up.  A task of k_sw runs up to 16
+// bands, one per lane of half a warp, strip after strip: steps = strips x
+// (W + 16), over the union of its bands' rows and its widest band, at the same
+// cost for 1 band as for 16.  The lane kernel (k_sys_pair) takes two bands per
+// warp, a step per row and a quarter.  A task's bands go there
 //  - when its steps alone outlast the pass: the pass takes about sum(chain) /
 //    32 steps over 148 x 12 warps, a step 530 cycles with twelve warps on an
 //    SM and 200 to 350 with few, so steps > sum(chain) / 35,000.  (61 queries,
-//    sensitive, whole search: 3.65 / 3.58 / 3.7 / 4.1 ms at 22,000 / 30,000 /
-//    40,000 / 55,000, and 5.5 ms with every warp kept.)
-//  - when the lane kernel runs its bands in less than half its steps, as it
-//    does for a warp of fewer than some 10 bands (pair_cost, in k_sw steps,
-//    from 1.36M bands in full warps, where that kernel takes 1.53 times as
-//    long).  20,000 queries default: 34.1 ms without this rule, 32.3, 31.9,
-//    33.1 and 35.2 ms at 0.3, 0.5, 0.8 and 0.95 of the steps: beside full
-//    warps the lane kernel is slower than alone.
+//    sensitive, whole search: 3.27, 3.29 and 3.64 ms at 25,000, 35,000 and
+//    50,000.)
+//  - when the lane kernel runs its bands in less than half its half warp's
+//    steps, as it does for a task of fewer than some 5 bands (pair_cost, in
+//    k_sw steps, from 1.36M bands in full warps, where that kernel takes 1.53
+//    times as long).  20,000 queries default: 27.4, 27.4, 27.6 and 28.4 ms at
+//    0.35, 0.5, 0.7 and 0.85 of the steps: beside full warps the lane kernel
+//    is slower than alone.
 constexpr uint64_t kChainShare = 35000;
 constexpr float kPairShare = 0.5f;
 __device__ __forceinline__ float pair_cost(int rows, int W) {
@@ -300,9 +301,9 @@ __global__ void k_sw_keys(const Band* bands, uint64_t n, const uint64_t* s_offse
   const Band b = bands[i];
   const uint64_t W = (uint64_t)(b.d1 - b.d0 + 1);
   const SwRoute r = sw_route(b, s_offsets, max_score, tn);
-  // A subject's transposed bands form warps of their own: only whole warps
+  // A subject's transposed bands form tasks of their own: only whole tasks
   // of them are transposed, the rest stay with their query windows.
-  const bool tr = r.tr && rows[i] < (tr_count[b.subject] & ~31u);
+  const bool tr = r.tr && rows[i] < (tr_count[b.subject] & ~(uint32_t)(kSwPart - 1));
   const int64_t rs = tr ? r.ts : r.rs, re = tr ? r.te : r.re;
   const uint64_t group = tr ? (kb.transposed | ((uint64_t)b.subject << kGroupShift))
                             : ((((uint64_t)b.target << 16) | b.q0) << kGroupShift);
@@ -342,8 +343,8 @@ __device__ __forceinline__ int band_job(uint32_t i, uint64_t at, const Band* ban
   return route;
 }
 
-// Task heads: first band of each (target, window) group and every 32nd after
-// (a group's bands are in width order, so a warp's widths are close).
+// Task heads: first band of each (target, window) group and every 16th after
+// (a group's bands are in width order, so a task's widths are close).
 // (d_n: the count is *d_n, n bounds it)
 __global__ void k_sw_group_start(const uint64_t* keys, uint64_t n, uint32_t* gstart, const int64_t* d_n) {
   uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -352,7 +353,7 @@ __global__ void k_sw_group_start(const uint64_t* keys, uint64_t n, uint32_t* gst
 }
 __global__ void k_sw_task_flags(const uint32_t* gstart, uint64_t n, uint8_t* f, const int64_t* d_n) {
   uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (s < n) f[s] = (!d_n || s < (uint64_t)*d_n) && ((s - gstart[s]) % 32) == 0;
+  if (s < n) f[s] = (!d_n || s < (uint64_t)*d_n) && ((s - gstart[s]) % kSwPart) == 0;
 }
 __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const uint64_t* keys, uint64_t n_fast,
                                 uint64_t transposed_key, const uint32_t* order, const Band* bands,
@@ -371,8 +372,9 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
   int64_t row_first = INT64_MAX, row_last = 0;
   uint32_t wmin = 0xFFFFFFFFu, wmax = 0;
   uint64_t lane_cells = 0;
+  int64_t first_end = INT64_MAX, last_end = INT64_MIN;  // of the bands: d1, m + d1
   float cost = 0.0f;  // the lane kernel's, in steps of this warp
-  while (cnt < 32 && s + cnt < n_fast && (keys[s + cnt] >> kGroupShift) == grp) {
+  while (cnt < kSwPart && s + cnt < n_fast && (keys[s + cnt] >> kGroupShift) == grp) {
     const uint64_t key = keys[s + cnt];
     const Band b = bands[order[s + cnt]];
     int64_t m = (int64_t)(s_offsets[b.subject + 1] - s_offsets[b.subject]);
@@ -383,6 +385,9 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
     if (rs < row_first) row_first = rs;
     if (w < wmin) wmin = w;
     if (w > wmax) wmax = w;
+    const int64_t d1 = transposed ? -(int64_t)b.d0 : (int64_t)b.d1;
+    first_end = min(first_end, d1);
+    last_end = max(last_end, (transposed ? (int64_t)b.n : m) + d1);
     lane_cells += (uint64_t)((re - rs + 16) / 16) * 16ull * (w + 16ull);
     cost += pair_cost((int)(re - rs + 1), (int)w);
     ++cnt;
@@ -404,7 +409,7 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
   // bands would have more rows there.
   const uint64_t limit = *chain_sum / kChainShare;
   if (transposed ? steps > (limit > kTransposedChain ? limit : kTransposedChain)
-                 : (steps > limit || cost < kPairShare * (float)steps)) {
+                 : (steps > limit || cost < kPairShare * (kSwPart / 32.0f) * (float)steps)) {
     const uint64_t at = atomicAdd(n_jobs, (unsigned long long)cnt);
     uint32_t n_route[4] = {0, 0, 0, 0};
     for (uint32_t x = 0; x < cnt; ++x) {
@@ -417,12 +422,21 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
     for (int y = 0; y < 4; ++y)
       if (n_route[y]) atomicAdd(route + 1 + y, (unsigned long long)n_route[y]);
     tasks[t].width = kSwNoClass;
-    sort_key[t] = (uint64_t)kSwClasses << kCostBits;  // after every class
+    sort_key[t] = (uint64_t)kSwClasses << (kCostBits + kCornerBits);  // after every class
     return;
   }
   const int cls = sw_class_of(wmax);
-  // class, then longest first (a scheduling order: 21 bits of steps, saturated, suffice)
-  sort_key[t] = ((uint64_t)cls << kCostBits) | (kCostMax - (steps < kCostMax ? steps : kCostMax));
+  // class, then most strips first (scheduling), then widest, then by the
+  // columns that every band of the task leaves out at its first and past its
+  // last strip, in sixteenths of a strip: k_sw pairs neighbours, which run
+  // the strips and columns that either needs
+  auto sixteenth = [&](int64_t x) {
+    return (uint64_t)(min(max(x, (int64_t)0), (int64_t)wmax + 15) * 16 / (int64_t)(wmax + 16));
+  };
+  const uint64_t corner = (sixteenth(first_end - row_first) << 4) |
+                          sixteenth(last_end - row_first - 16 * ((int64_t)k.n_strips - 1));
+  sort_key[t] = ((uint64_t)cls << (kCostBits + kCornerBits)) |
+                ((kCostMax - ((uint64_t)min(k.n_strips, 1023u) << 11 | wmax)) << kCornerBits) | corner;
   if (cells_gpu) {
     atomicAdd(cells_gpu + 1, (unsigned long long)lane_cells);  // evaluated cells: counted by k_sw
     if (transposed) atomicAdd(cells_gpu + 3, (unsigned long long)cnt);
@@ -725,7 +739,7 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   count_launch();
   k_band_jobs_dev<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(
       swos, cnt, n_bands, bc, s.offsets, jobs_u, jkey, jval, reinterpret_cast<unsigned long long*>(cnt + 6));
-  // ---- narrow bands: warps of up to 32 bands of one group
+  // ---- narrow bands: tasks of up to 16 bands of one group
   uint32_t* gstart = c->idx.as<uint32_t>(n_bands + 1);
   count_launch();
   k_sw_group_start<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(swks, n_bands, gstart, cnt + 1);
@@ -755,7 +769,7 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
                                                                       cnt + 15);
   // by width class, longest warps first within a class
   const uint32_t* task_order =
-      dsort(c, tkey, tkey_s, tval, tval_s, n_bands, 0, kCostBits + 3, reinterpret_cast<const uint64_t*>(cnt + 2))
+      dsort(c, tkey, tkey_s, tval, tval_s, n_bands, 0, kCostBits + kCornerBits + 3, reinterpret_cast<const uint64_t*>(cnt + 2))
           .vals;
   count_launch();
   k_gather_tasks<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(tasks_u, task_order, n_bands, tasks, cnt + 2);
@@ -859,7 +873,7 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
     cudaEvent_t joined = log->event();
     DRG_CUDA(cudaEventRecord(joined, c->stream));
     for (int k = 0; k < kSwClasses; ++k) {
-      st.sw_class_tasks[k] += hi[k] - lo[k];
+      st.sw_class_tasks[k] += (hi[k] - lo[k] + 32 / kSwPart - 1) / (32 / kSwPart);  // warps
       if (hmax[k] > st.sw_class_max_steps[k]) st.sw_class_max_steps[k] = hmax[k];
     }
     st.sw_wide_bands += wide.n;

@@ -13,8 +13,6 @@ namespace sw {
 
 constexpr int kRows = 16;          // rows per strip
 constexpr int kPairs = kRows / 2;  // s16x2 pairs
-constexpr int kProfStride = 24;    // bytes per residue row of the strip profile
-constexpr int kProfBytes = 26 * kProfStride;
 constexpr uint32_t kNeg2 = 0xC000C000u;  // (-16384, -16384)
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {

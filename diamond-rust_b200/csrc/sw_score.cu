@@ -1,8 +1,17 @@
 // Banded affine Smith-Waterman (gapped.rs:67-203) for many bands that share a
 // query window (or a subject, transposed): the score pass of the E-value gate.
 //
-// Mapping (inter-task): one thread = one band; one warp = up to 32 bands of
-// the same query window and width W, so the query profile is shared per warp.
+// Mapping (inter-task): one thread = one band; one half warp = up to 16 bands
+// of the same query window, which share its profile in shared memory; a warp
+// runs two such tasks of nearly equal strips, widths and corners (they are
+// sorted so), of any two queries.  A warp runs the union of its bands' rows
+// and columns: with 32 bands of one window per warp, 64 bands of a query (the
+// 20,000-query search) are two warps whose lanes each need half of it, 1.91
+// computed cells per cell of a band; 16 make it 1.65 (15.9 -> 13.1 ms), and
+// the 1,000-query sensitive search, 40 warps a query, 1.39 -> 1.33 (12.9 ->
+// 12.3 ms).  8 make the former 1.44, but at 12.3 ms, and the latter slower
+// (12.4 ms): the profiles cost twice as much, and class 0 has to end at 134
+// columns for three blocks to fit an SM.
 // The band is swept in strips of 16 DP rows.  Inside a strip, relative column
 // c covers absolute subject column j = i0 - d1 + c, and row r of the strip is
 // in the band for r <= c <= r + W - 1.  The 16 rows are held as 8 pairs of
@@ -58,6 +67,10 @@ namespace {
 
 using namespace sw;
 
+constexpr int kParts = 32 / kSwPart;  // tasks per warp
+constexpr int kProfHigh = 26 * 8;     // profile bytes of rows 8 to 15, after those of rows 0 to 7
+constexpr int kProfBytes = 2 * kProfHigh;
+
 // Registers of one lane's 16-row strip in the score pass.
 struct SRegs {
   uint32_t H[kPairs], F[kPairs];
@@ -78,9 +91,9 @@ __device__ __forceinline__ void sw_step(SRegs& R, Lane& L, int c, const uint8_t*
                                         const uint32_t* __restrict__ rp, uint32_t* __restrict__ wp, uint32_t noc2,
                                         uint32_t nge2, int cw = 0) {
   const uint32_t res = next_residue(L, c);  // subject residue of this column
-  const uint8_t* prow = prof + res * kProfStride;
+  const uint8_t* prow = prof + res * 8;
   const uint2 lo8 = *reinterpret_cast<const uint2*>(prow);
-  const uint2 hi8 = *reinterpret_cast<const uint2*>(R.prow_prev + 8);
+  const uint2 hi8 = *reinterpret_cast<const uint2*>(R.prow_prev + kProfHigh);
   R.prow_prev = prow;
   const uint32_t rw = *rp;  // (H, E') of the row above row 0, column c
   const uint32_t h_top = prmt(rw, R.H[kPairs - 1], 0x5410);
@@ -184,20 +197,24 @@ template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t task_id = a.task_lo + (uint64_t)blockIdx.x * WARPS + warp;
+  const int part = lane / kSwPart, at = lane % kSwPart;
+  const uint64_t task_id = a.task_lo + ((uint64_t)blockIdx.x * WARPS + warp) * kParts;
   const int stride = WARPS * 32;
   int8_t* mat = reinterpret_cast<int8_t*>(smem);  // 25 x 25 scores
-  uint8_t* prof = smem + 640 + warp * kProfBytes;  // strip profile
-  uint32_t* ring = reinterpret_cast<uint32_t*>(smem + 640 + WARPS * kProfBytes) + threadIdx.x;
+  uint8_t* prof = smem + 640 + (warp * kParts + part) * kProfBytes;  // strip profile
+  uint32_t* ring = reinterpret_cast<uint32_t*>(smem + 640 + WARPS * kParts * kProfBytes) + threadIdx.x;
   for (int i = threadIdx.x; i < 625; i += blockDim.x) mat[i] = a.scores625[i];
   __syncthreads();
   if (task_id >= a.task_hi) return;
-  const SwTask task = a.tasks[task_id];
-  const int W = (int)task.width;   // widest band of the warp
-  const int Wmin = (int)task.w_min;
+  // a part past the launch's last task repeats the warp's first, to no effect
+  const bool idle = task_id + part >= a.task_hi;
+  const SwTask task = a.tasks[task_id + (idle ? 0 : part)];
+  const int W = (int)__reduce_max_sync(0xFFFFFFFFu, task.width);     // widest band of the warp
+  const int Wmin = (int)__reduce_min_sync(0xFFFFFFFFu, task.w_min);  // narrowest
+  const uint32_t n_strips = __reduce_max_sync(0xFFFFFFFFu, task.n_strips);
   const int buf = W + 1;
-  const bool active = lane < (int)task.count;
-  const uint32_t bidx = a.order[task.first + (active ? lane : 0)];
+  const bool active = !idle && at < (int)task.count;
+  const uint32_t bidx = a.order[task.first + (at < (int)task.count ? at : 0)];
   const Band band = a.bands[bidx];
   const int Wl = band.d1 - band.d0 + 1;  // this lane's width
   // Rows are the query window and columns the subject, or (a transposed
@@ -226,21 +243,22 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
   SRegs R;
   int best = 0, best_i = 0;
   uint64_t steps_done = 0;  // column steps run (all strips)
-  for (uint32_t k = 0; k < task.n_strips; ++k) {
+  for (uint32_t k = 0; k < n_strips; ++k) {
     const int i0 = (int)task.row_first + (int)(k * kRows);
-    // strip profile: prof[res * stride + r] = S(query letter, subject letter)
-    // of row i0 + r against column residue res
+    // strip profile of each part: the score of row i0 + r against column
+    // residue res at prof[8 res + r] (r < 8), prof[kProfHigh + 8 res + r - 8];
+    // a lane writes one row (rows at..at + kSwPart step)
     __syncwarp();
-    for (int e = lane; e < 26 * kRows; e += 32) {
-      int res = e >> 4, r = e & 15;
-      int i = i0 + r;
-      int v;
-      if (res == 25 || i > n) v = kSentinelScore;
-      else {
-        const int row = (int)min((uint32_t)q[i - 1], 24u);
-        v = tr ? mat[res * 25 + row] : mat[row * 25 + res];
-      }
-      prof[res * kProfStride + r] = (uint8_t)(int8_t)v;
+    for (int r = at; r < kRows; r += kSwPart) {
+      const int i = i0 + r;
+      const bool in = i <= n;
+      const int row = in ? (int)min((uint32_t)q[i - 1], 24u) : 0;
+      const int8_t* sc = mat + (tr ? row : row * 25);
+      const int step = tr ? 25 : 1;
+      uint8_t* out = prof + (r < 8 ? r : kProfHigh + r - 8);
+#pragma unroll 5
+      for (int res = 0; res < 25; ++res) out[res * 8] = (uint8_t)(in ? sc[res * step] : (int8_t)kSentinelScore);
+      out[25 * 8] = (uint8_t)(int8_t)kSentinelScore;
     }
     __syncwarp();
     L.jbase = i0 - d1;
@@ -270,7 +288,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
     R.htop_old = *rg.wp & 0xFFFFu;
     {
       const int jm1 = L.jbase + c_begin - 2;  // column c_begin - 1
-      R.prow_prev = prof + subject_residue(L, jm1) * kProfStride;
+      R.prow_prev = prof + subject_residue(L, jm1) * 8;
 #pragma unroll
       for (int i = 0; i < kQueue; ++i) L.queue[i] = subject_residue(L, jm1 + 1 + i);
     }
@@ -342,9 +360,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
       best_i = i0 + kRows - 1;
     }
   }
-  if (lane == 0 && a.cells_eval) {
-    atomicAdd(a.cells_eval, (unsigned long long)(steps_done * kRows * task.count));
-    atomicAdd(a.cells_eval + 2, (unsigned long long)(steps_done * kRows * 32));  // idle lanes included
+  if (a.cells_eval) {
+    const int lanes = __popc(__ballot_sync(0xFFFFFFFFu, active));
+    if (lane == 0) {
+      atomicAdd(a.cells_eval, (unsigned long long)(steps_done * kRows * lanes));
+      atomicAdd(a.cells_eval + 2, (unsigned long long)(steps_done * kRows * 32));  // idle lanes included
+    }
   }
   if (!active) return;
   a.score[bidx] = best;
@@ -358,13 +379,13 @@ template <int WARPS>
 void launch_class(const SwScoreArgs& a, int max_width, cudaStream_t st) {
   if (a.task_hi <= a.task_lo) return;
   const int threads = WARPS * 32;
-  const size_t smem = 640 + WARPS * kProfBytes + (size_t)threads * (max_width + 1) * 4;
+  const size_t smem = 640 + WARPS * kParts * kProfBytes + (size_t)threads * (max_width + 1) * 4;
   static int configured = 0;  // per template instance
   if ((int)smem > configured) {
     DRG_CUDA(cudaFuncSetAttribute(k_sw<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = (int)smem;
   }
-  const int blocks = ceil_div((long long)(a.task_hi - a.task_lo), WARPS);
+  const int blocks = ceil_div((long long)(a.task_hi - a.task_lo), WARPS * kParts);
   count_launch();
   k_sw<WARPS><<<blocks, threads, smem, st>>>(a);
   DRG_CUDA(cudaGetLastError());
