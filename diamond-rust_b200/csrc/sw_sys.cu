@@ -497,27 +497,36 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
 // depend on its number only, so two bands run in step, each with its own
 // letters, profile and right edge.  Jobs are sorted by route and length, so
 // that a pair's bands end together.  For bands whose best stays below 2^15
-// (the packed kernels' bound); H counts only inside the band and the matrix,
-// and is below 0x7C00 there, so its maximum folds as half-precision bit
-// patterns (max2_pos_f16).
-// A step of 4 rows is about 75 warp instructions for the two bands (8 rows
-// 118, 16 rows 206), ALU-bound like the forms above; 22 bands of a 497-aa
-// query take 142 us (one band per lane: 758 us).  16 rows per lane replace
-// the 16-row groups of lanes on one band each (2,000 bands of 272-559 columns:
-// 708 -> 676 us) up to 511 columns.
+// (the packed kernels' bound).
+// E and F are kept with the open cost added back (E' = max(E' - ge, H) above,
+// F' = max(F' - ge, H) to the left, H = max(0, D, E' - oc, F' - oc): all at
+// least 0).  Outside the band no cell is masked after it is computed: an
+// addend of -16384 on D and on the open cost makes its H 0, and its E' comes
+// only from such cells above it.  Row r is outside in the column that row 0
+// was r columns earlier, so a lane computes one addend per column and keeps
+// the last R + 1; a strip starts with all of them dead, which is its left
+// edge; and what a strip hands down is dead with its last row.  A cell is five
+// ALU operations, half a three-input maximum and three adds on the FMA pipe,
+// which runs beside (ten ALU operations with masks on E and H and selects for
+// the left edge: 22 bands of a 497-aa query 141 -> 129 us, the widest route of
+// 1,000 queries very sensitive 4,620 -> 3,100 us, of 13 queries
+// ultra-sensitive 2,160 -> 1,600 us).
+// 16 rows per lane replace the 16-row groups of lanes on one band each (2,000
+// bands of 272-559 columns: 708 -> 676 us) up to 511 columns.
 using sw::add2;
-using sw::max2_pos_f16;
 using sw::pick_sel;
 using sw::prmt;
 
+constexpr uint32_t kDead2 = 0xC000C000u;  // (-16384, -16384)
+
 template <int R>
 constexpr size_t pair_smem() {
-  return (size_t)kRotWarpsPerBlock * 2 * (R / 4) * kResidues * 32 * sizeof(uint32_t);
+  return (size_t)kRotWarpsPerBlock * 2 * ((R + 3) / 4) * kResidues * 32 * sizeof(uint32_t);
 }
 
 template <int R>
 __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs a) {
-  constexpr int kLag = R + 1, kWords = R / 4;
+  constexpr int kLag = R + 1, kWords = (R + 3) / 4;
   extern __shared__ __align__(16) uint32_t pair_prof[];
   __shared__ int8_t mat[kResidues * 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -546,18 +555,23 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs 
   }
   const uint32_t noc2 = (uint32_t)(uint16_t)(-(a.gap_open + a.gap_extend)) * 0x10001u;
   const uint32_t nge2 = (uint32_t)(uint16_t)(-a.gap_extend) * 0x10001u;
-  uint32_t hl[R], f[R];
+  uint32_t hl[R], f[R];  // H of the last column, F' of this one
+  uint32_t out[kLag];    // per column of the last R + 1: kDead2 where a strip's first row is outside its band
   uint32_t top = 0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     hl[r] = 0;
     f[r] = 0;
   }
+#pragma unroll
+  for (int u = 0; u < kLag; ++u) out[u] = kDead2;
   int best[2] = {0, 0}, bi[2] = {0x7FFFFFFF, 0x7FFFFFFF};
-  int s = lane, c = -kLag * lane;
-  constexpr int kPast = 0x3FFF;  // c - (W - 1) of a lane without a strip: right of the band
-  auto cw_of = [&](int x) { return (uint32_t)(uint16_t)(s < S[x] ? c - (W[x] - 1) : kPast); };
-  uint32_t cw2 = cw_of(0) | cw_of(1) << 16;
+  int s = lane;
+  // per half: column past the right end of the first row's band, c - (W - 1);
+  // kPast (dead throughout) of a lane without a strip, or before its strip
+  // starts: what it passes on then reaches the strip of 32 before
+  constexpr uint32_t kPast = 0x3FFF;
+  uint32_t cw2 = kPast | kPast << 16;
   int p[2] = {g[0].rs - g[0].d1 - 1 - lane, g[1].rs - g[1].d1 - 1 - lane};
   auto letter = [&](int x, int at) -> uint32_t {
     return (unsigned)at < (unsigned)m[x] ? (uint32_t)__ldg(sl[x] + at) : (uint32_t)kSentinel;
@@ -630,28 +644,29 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs 
     if (k >= 31 && lane == ((k + 1) & 31)) {
       fold();
       s += 32;
-      c -= 32 * kLag;
       p[0] -= 32;
       p[1] -= 32;
-      cw2 = cw_of(0) | cw_of(1) << 16;
+      cw2 = kPast | kPast << 16;
     }
     const bool starts = lane == (k & 31);
     if (starts) {
       top = 0;
+      cw2 = (s < S[0] ? (uint32_t)(uint16_t)(1 - W[0]) : kPast) | (s < S[1] ? (uint32_t)(uint16_t)(1 - W[1]) : kPast) << 16;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         hl[r] = 0;
         f[r] = 0;
       }
+#pragma unroll
+      for (int u = 0; u < kLag; ++u) out[u] = kDead2;
     }
     __syncwarp();
 #pragma unroll
     for (int u = 0; u < kLag; ++u) {
+      // cw > 0: right of the first row's band
+      out[u] = ~prmt(add2(cw2, 0xFFFFFFFFu), 0u, 0xBB99u) & kDead2;
+      // (strip 0 has lane 31 above it, which is dead until its first strip)
       uint32_t hu = __shfl_sync(kAll, h_out, src), eu = __shfl_sync(kAll, e_out, src);
-      if (s == 0) {
-        hu = 0;
-        eu = 0;
-      }
       uint32_t w[2][kWords];
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
@@ -664,36 +679,25 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs 
       }
       uint32_t hd = hup;
       hup = hu;
-      uint32_t t = 0;
+      uint32_t h_even = 0;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const uint32_t sc = prmt(w[0][r >> 2], w[1][r >> 2], pick_sel(r & 3));
-        const uint32_t in = prmt(add2(cw2, (uint32_t)(uint16_t)(-(r + 1)) * 0x10001u), 0u, 0xBB99u);
-        // e, fn: E and F with the open cost added back, so that E' = max(E' -
-        // ge, H) above, F' = max(F' - ge, H) to the left and H = max(0, D,
-        // max(E', F') - oc): all at least 0, a dead cell plain 0, and two adds
-        // per pair less than with H - oc (22 bands of a 497-aa query: 156 ->
-        // 142 us)
-        uint32_t e = __viaddmax_s16x2(eu, nge2, hu);
-        uint32_t fn = __viaddmax_s16x2(f[r], nge2, hl[r]);
-        uint32_t h = __viaddmax_s16x2_relu(max2_pos_f16(e, fn), noc2, add2(hd, sc)) & in;
-        e &= in;
-        if (u < R - 1 && r > u && starts) {  // left of the band
-          h = 0;
-          fn = 0;
-        }
-        t = max2_pos_f16(t, h);
+        const uint32_t dead = out[(u - r + kLag) % kLag];
+        const uint32_t no = add2(noc2, dead);
+        const uint32_t e = __viaddmax_s16x2(eu, nge2, hu);
+        const uint32_t h = __viaddmax_s16x2(e, no, __viaddmax_s16x2_relu(f[r], no, add2(hd, add2(sc, dead))));
         hd = hl[r];
         hl[r] = h;
-        f[r] = fn;
+        f[r] = __viaddmax_s16x2(f[r], nge2, h);
         hu = h;
         eu = e;
+        if (r & 1) top = __vimax3_s16x2(top, h_even, h);
+        h_even = h;
       }
-      top = max2_pos_f16(top, t);
       h_out = hu;
-      e_out = eu;
+      e_out = add2(eu, out[(u + 2) % kLag]);  // of row R - 1
       cw2 = add2(cw2, 0x00010001u);
-      ++c;
       ++p[0];
       ++p[1];
     }
