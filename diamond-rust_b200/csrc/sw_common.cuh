@@ -39,9 +39,6 @@ __device__ __forceinline__ uint32_t max2_pos_f16(uint32_t a, uint32_t b) {
   asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
-// keep halves selected by k (0xFFFF per kept half), replace the others with v
-__device__ __forceinline__ uint32_t sel2(uint32_t x, uint32_t k, uint32_t v) { return (x & k) | (v & ~k); }
-
 // Sign-extending byte pick: low half = byte b of lo, high half = byte b of hi.
 __device__ __forceinline__ constexpr uint32_t pick_sel(int b) {
   return (uint32_t)(b) | ((uint32_t)(8 | b) << 4) | ((uint32_t)(4 + b) << 8) | ((uint32_t)(8 | (4 + b)) << 12);
@@ -73,14 +70,6 @@ __device__ __forceinline__ uint32_t next_residue(Lane& L, int c) {
   L.queue[kQueue - 1] = ahead;
   return res;
 }
-
-struct Regs {
-  uint32_t H[kPairs], Hm[kPairs], F[kPairs];
-  uint32_t E7;        // E of pair 7 at the previous step
-  uint32_t htop_old;  // top H of the previous step (D operand of pair 0)
-  uint32_t res_prev;  // subject residue of the previous column
-  uint32_t rowmax[kPairs];            // per row of the strip: max H so far
-};
 
 __device__ __forceinline__ int lo16(uint32_t x) { return (int)(int16_t)(x & 0xFFFFu); }
 __device__ __forceinline__ int hi16(uint32_t x) { return (int)(int16_t)(x >> 16); }
