@@ -22,7 +22,7 @@ struct drg_ctx {
   cudaStream_t side = nullptr;  // concurrent launches (wide-band classes)
   // more of them: each route of the score and traceback passes has its own, so
   // that the launches' longest bands run beside one another
-  cudaStream_t lanes[5] = {};
+  cudaStream_t lanes[7] = {};
   cudaMemPool_t pool = nullptr;  // resident databases and batches (kept across calls)
   std::string err;
   // seed stage

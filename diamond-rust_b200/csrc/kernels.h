@@ -317,13 +317,19 @@ struct SwBandArgs {
 };
 size_t sw_band_smem(int max_width);
 void launch_sw_band(SwBandArgs a, int max_width, cudaStream_t st);
-// Bands of the score pass that do not share a warp 32 at a time, by width:
-// routes 0, 1, 2 run two per warp with rotating strips of 4, 8, 16 rows per
-// lane (k_sys_pair, W <= 151, 271, 511); route 3 (wider) in the block kernel.
-// max_width matters for route 3 only.
+// Bands of the score pass that do not share a half warp of k_sw, by width:
+// routes 0 to 4 run two per warp with rotating strips of pair_rows(route) rows
+// per lane (k_sys_pair, W <= 151, 211, 271, 391, 511), the last route (wider)
+// a warp each (k_sw_band), for which alone max_width matters.
 __host__ __device__ constexpr int sys_rot_max(int R);
+constexpr int kBandRoutes = 6;
+__host__ __device__ constexpr int pair_rows(int route) {
+  return route == 0 ? 4 : route == 1 ? 6 : route == 2 ? 8 : route == 3 ? 12 : 16;
+}
 __host__ __device__ inline int sw_band_route(int width) {
-  return width <= sys_rot_max(4) ? 0 : (width <= sys_rot_max(8) ? 1 : (width <= sys_rot_max(16) ? 2 : 3));
+  int r = 0;
+  while (r < kBandRoutes - 1 && width > sys_rot_max(pair_rows(r))) ++r;
+  return r;
 }
 void launch_sw_band_route(const SwBandArgs& a, int route, int max_width, cudaStream_t st);
 

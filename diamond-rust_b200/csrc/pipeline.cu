@@ -411,15 +411,15 @@ __global__ void k_sw_fill_tasks(const uint32_t* starts, uint64_t n_tasks, const 
   if (transposed ? steps > (limit > kTransposedChain ? limit : kTransposedChain)
                  : (steps > limit || cost < kPairShare * (kSwPart / 32.0f) * (float)steps)) {
     const uint64_t at = atomicAdd(n_jobs, (unsigned long long)cnt);
-    uint32_t n_route[4] = {0, 0, 0, 0};
+    uint32_t n_route[kBandRoutes] = {};
     for (uint32_t x = 0; x < cnt; ++x) {
       const int r = band_job(order[s + x], at + x, bands, s_offsets, jobs, job_key, job_val);
 #pragma unroll
-      for (int y = 0; y < 4; ++y) n_route[y] += r == y;
+      for (int y = 0; y < kBandRoutes; ++y) n_route[y] += r == y;
     }
     atomicMax(route, (unsigned long long)wmax);
 #pragma unroll
-    for (int y = 0; y < 4; ++y)
+    for (int y = 0; y < kBandRoutes; ++y)
       if (n_route[y]) atomicAdd(route + 1 + y, (unsigned long long)n_route[y]);
     tasks[t].width = kSwNoClass;
     sort_key[t] = (uint64_t)kSwClasses << (kCostBits + kCornerBits);  // after every class
@@ -507,7 +507,7 @@ __global__ void k_band_jobs_dev(const uint32_t* order, int64_t* cnt, uint64_t n,
   const bool head = (threadIdx.x & 31) == 0;
   if (head) atomicMax(route, (unsigned long long)W);
 #pragma unroll
-  for (int x = 0; x < 4; ++x) {
+  for (int x = 0; x < kBandRoutes; ++x) {
     const uint32_t in = __ballot_sync(0xFFFFFFFFu, r == x);
     if (head && in) atomicAdd(route + 1 + x, (unsigned long long)__popc(in));
   }
@@ -605,7 +605,7 @@ struct BandJobs {
   SwBandJob* jobs = nullptr;
   uint64_t n = 0;
   int max_width = 0;
-  uint64_t route_lo[5] = {0, 0, 0, 0, 0};  // jobs [route_lo[r], route_lo[r + 1]) take route r
+  uint64_t route_lo[kBandRoutes + 1] = {};  // jobs [route_lo[r], route_lo[r + 1]) take route r
 };
 
 SwBandArgs band_args(const Band* bc, const BandJobs& bj, const DevSeqs& qs, const DevSeqs& s, const Scoring& scr) {
@@ -694,12 +694,12 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   DRG_CUDA(cudaMemsetAsync(tr_count, 0, n_subjects * sizeof(uint32_t), c->stream));
   count_launch();
   // score pass counts, on the device until the one wait before the launches:
-  //   [0] fast bands  [1] narrow bands  [2] tasks  [6] widest job  [7..10]
+  //   [0] fast bands  [1] narrow bands  [2] tasks  [25] widest job  [26..31]
   //   jobs per route  [11..14] longest warp per class  [15] jobs  [16..19]
   //   bands listed for the 32-bit kernel  [20] sum of the packed kernel's
   //   chains  [21..24] tasks up to each class's end
-  int64_t* cnt = c->sw_counts.as<int64_t>(25);
-  DRG_CUDA(cudaMemsetAsync(cnt, 0, 25 * sizeof(int64_t), c->stream));
+  int64_t* cnt = c->sw_counts.as<int64_t>(32);
+  DRG_CUDA(cudaMemsetAsync(cnt, 0, 32 * sizeof(int64_t), c->stream));
   unsigned long long* chain_sum = reinterpret_cast<unsigned long long*>(cnt + 20);
   k_sw_tr_count<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(bc, n_bands, s.offsets, scr.max_score,
                                                                 sw_tune(c), tr_count, rows,
@@ -738,7 +738,7 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   uint32_t* jval_s = c->bj_val_s.as<uint32_t>(n_bands);
   count_launch();
   k_band_jobs_dev<<<ceil_div(n_bands, 256), 256, 0, c->stream>>>(
-      swos, cnt, n_bands, bc, s.offsets, jobs_u, jkey, jval, reinterpret_cast<unsigned long long*>(cnt + 6));
+      swos, cnt, n_bands, bc, s.offsets, jobs_u, jkey, jval, reinterpret_cast<unsigned long long*>(cnt + 25));
   // ---- narrow bands: tasks of up to 16 bands of one group
   uint32_t* gstart = c->idx.as<uint32_t>(n_bands + 1);
   count_launch();
@@ -760,7 +760,7 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   k_sw_fill_tasks<<<ceil_div(n_bands, 128), 128, 0, c->stream>>>(
       tstart, n_bands, swks, n_bands, kb.transposed, swos, bc, s.offsets, tasks_u, tkey, tval, cells_gpu, cnt + 2,
       cnt + 1, chain_sum, jobs_u, jkey, jval,
-      reinterpret_cast<unsigned long long*>(cnt + 15), reinterpret_cast<unsigned long long*>(cnt + 6));
+      reinterpret_cast<unsigned long long*>(cnt + 15), reinterpret_cast<unsigned long long*>(cnt + 25));
   const uint32_t* jorder =
       dsort(c, jkey, jkey_s, jval, jval_s, n_bands, 0, kCostBits + 3, reinterpret_cast<const uint64_t*>(cnt + 15))
           .vals;
@@ -780,8 +780,8 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
                                                                reinterpret_cast<unsigned long long*>(cnt + 11),
                                                                cnt + 2);
   // ---- the one wait: every count the launches need
-  int64_t* h = c->h_stage.as<int64_t>(25);
-  DRG_CUDA(cudaMemcpyAsync(h, cnt, 25 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+  int64_t* h = c->h_stage.as<int64_t>(32);
+  DRG_CUDA(cudaMemcpyAsync(h, cnt, 32 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
   DRG_CUDA(cudaStreamSynchronize(c->stream));
   const uint64_t n_fast = (uint64_t)h[0];
   const int64_t* bounds = h + 21;  // ends of the classes
@@ -790,8 +790,8 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   BandJobs wide;
   wide.jobs = wjobs;
   wide.n = (uint64_t)h[15];
-  wide.max_width = (int)h[6];
-  for (int k = 0; k < 4; ++k) wide.route_lo[k + 1] = wide.route_lo[k] + (uint64_t)h[7 + k];
+  wide.max_width = (int)h[25];
+  for (int k = 0; k < kBandRoutes; ++k) wide.route_lo[k + 1] = wide.route_lo[k] + (uint64_t)h[26 + k];
   // bands the packed kernels do not take, in the 32-bit kernel: the longest
   // chains of the pass, so first, beside the packed classes
   SysArgs xa = sys_args(bc, qs, s, scr);
@@ -838,14 +838,14 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
       return e;
     };
     if (n_bands > n_fast)
-      on(c->lanes[4], [&](cudaStream_t s2) {
+      on(c->lanes[kBandRoutes], [&](cudaStream_t s2) {
         sys_scores(c, xa, c->sys_list, swos, n_fast, n_bands, nullptr, cnt + 16, n_sys, s.max_len, s2);
       });
     std::vector<cudaEvent_t> wide_ends;
     SwBandArgs ba = band_args(bc, wide, qs, s, scr);
     ba.score = scores;
     ba.best_row = best_row;
-    for (int k = 3; k >= 0; --k) {
+    for (int k = kBandRoutes - 1; k >= 0; --k) {
       ba.lo = wide.route_lo[k];
       ba.hi = wide.route_lo[k + 1];
       if (ba.hi == ba.lo) continue;

@@ -511,8 +511,13 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
 // the left edge: 22 bands of a 497-aa query 141 -> 129 us, the widest route of
 // 1,000 queries very sensitive 4,620 -> 3,100 us, of 13 queries
 // ultra-sensitive 2,160 -> 1,600 us).
-// 16 rows per lane replace the 16-row groups of lanes on one band each (2,000
-// bands of 272-559 columns: 708 -> 676 us) up to 511 columns.
+// All 32 lanes run whatever the width, so a band takes the fewest rows per lane
+// that hold it: 4, 6, 8, 12 or 16, the widths up to 151, 211, 271, 391 and 511
+// (with 4, 8 and 16 alone: 26.3 ms for 1,000 queries very sensitive, whose
+// wide bands are mostly 250 to 350 columns; 25.7 with all five).  24 and 32
+// rows, up to 991 columns, were slower than a warp per band (sw_band.cu): a
+// step is then too long a chain (13 queries, ultra-sensitive: 6.9 against 6.6
+// ms).
 using sw::add2;
 using sw::pick_sel;
 using sw::prmt;
@@ -903,9 +908,11 @@ static void launch_pair(const SwBandArgs& a, cudaStream_t st) {
 void launch_sw_band_route(const SwBandArgs& a, int route, int max_width, cudaStream_t st) {
   if (a.hi <= a.lo) return;
   switch (route) {
-    case 0: launch_pair<4>(a, st); break;
-    case 1: launch_pair<8>(a, st); break;
-    case 2: launch_pair<16>(a, st); break;
+    case 0: launch_pair<pair_rows(0)>(a, st); break;
+    case 1: launch_pair<pair_rows(1)>(a, st); break;
+    case 2: launch_pair<pair_rows(2)>(a, st); break;
+    case 3: launch_pair<pair_rows(3)>(a, st); break;
+    case 4: launch_pair<pair_rows(4)>(a, st); break;
     default: launch_sw_band(a, max_width, st); break;
   }
 }

@@ -9,7 +9,7 @@ from drgpu import synth
 
 pytestmark = pytest.mark.gpu
 
-ROWS = [4, 8, 16]
+ROWS = [4, 6, 8, 12, 16]
 WIDEST = [31 * (r + 1) - r for r in ROWS]
 
 
