@@ -474,11 +474,15 @@ __host__ __device__ inline SysBlockPlan sys_block_plan(const SysGeom& g, int m) 
   if (p.stride < 16) p.stride = 16;
   return p;
 }
+// Rows at most of a traced band of the rotating kernel: its maxima carry their
+// place in the low 9 + log2(R) of 32 bits, scores are at most 127 a row.
+__host__ __device__ constexpr int sys_rot_rows(int R) { return (int)((1ll << 32) / (512 * R) / 128); }
 // 0, 1: rotating kernel with 4, 8 rows per lane; 2: block kernel.
 __host__ __device__ inline int sys_route(const SysGeom& g, bool trace) {
   const int W = g.d1 - g.d0 + 1;
-  if (W <= sys_rot_max(4)) return 0;
-  return trace && W <= sys_rot_max(8) ? 1 : 2;
+  if (!trace) return W <= sys_rot_max(4) ? 0 : 2;
+  if (W <= sys_rot_max(4) && g.rows <= sys_rot_rows(4)) return 0;
+  return W <= sys_rot_max(8) && g.rows <= sys_rot_rows(8) ? 1 : 2;
 }
 // Trace bytes of a band and the steps its kernel takes (a scheduling cost).
 __host__ __device__ inline uint64_t sys_trace_bytes(const SysGeom& g, int m, int route, uint64_t* steps) {

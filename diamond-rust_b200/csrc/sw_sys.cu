@@ -17,12 +17,12 @@
 // (R + 1) s, one step behind the strip above it, whose last row's (H, E) it
 // takes by a shuffle.  Relative column c = T - (R + 1) s of a strip covers
 // subject column j = i0 - d1 + c, and row r is in the band for
-// r <= c <= r + W - 1, so that
-//   - exactly one lane is in its first R columns at any step, the one that
-//     started at this turn of the (R + 1)-step loop: the left edge is masked
-//     at compile time for that lane alone;
-//   - the right edge is masked off the chain: a cell past it gets -inf added
-//     to both sources of E and 0 for its diagonal/F part, so H = 0, E = -inf.
+// r <= c <= r + W - 1.  A cell outside is dead by an addend (kNegI) on all that
+// flows into it, so its H is 0 and its E and F are near -inf.  Row r is
+// outside in the column that row 0 was r columns earlier, so a lane computes
+// one addend per column and keeps the last R + 1; its columns before the first
+// are dead as well, which is the left edge of its rows and leaves the state
+// that a strip starts from.
 // Cells off the matrix need no mask: residues and rows there score -64, their
 // H stays below the H it came from, and nothing flows from them to a matrix
 // cell.  A strip's profile (R scores per residue, one word per lane and
@@ -42,22 +42,25 @@
 // looked at only when the best of the others is at most the matrix's largest
 // score, and their alignment is that one pair.
 //
-// In trace mode each step stores one word per lane (a nibble per row: choice
-// | e_ext << 2 | f_ext << 3, gapped.rs:120-200), 32 consecutive words per
-// step.  The walk (gapped.rs:205-279) then takes up to 32 cells at a time:
-// lane k reads the cell k steps back along the diagonal (or the gap), and a
-// ballot finds where the run ends.
+// In trace mode each step stores one word per lane, 32 consecutive words per
+// step, with a nibble per row: whether a gap beat the diagonal, whether F beat
+// E, and whether E and F extend a gap (gapped.rs:120-200).  Each is the sign
+// of a difference, pushed into the word by one funnel shift.  Whether H is 0
+// is not stored: the walk (gapped.rs:205-279) knows H along its way.  It takes
+// up to 32 cells at a time: lane k reads the cell k steps back along the
+// diagonal (or the gap), a scan of the pairs' scores gives H there, and a
+// ballot finds where the run ends.  A band's best cell is the largest of one
+// integer per column made of H, row and column.  A cell costs some nine ALU
+// operations (27 with compares and selects for the masks, a stored choice of
+// four and a maximum and column per row).
 //
 // Measured on one B200 (first figure: the form this replaces, 16 rows per
 // lane in 16-bit pairs with a lane walking alone, and one thread per band
-// where that form did not apply):
-//   traceback of 4 bands of a 497-aa query        415 -> 133 us
-//   of 26,597 bands (20,000 queries)             7394 -> 2250 us
-//   of 4,182 bands (1,000 queries, sensitive)    1283 -> 530 us, routes side by side
-//   13 bands up to 2,000 x 4,000, scores    1,206,000 -> 1,140 us
-// A step of 4 rows in trace mode is about 140 warp instructions, most of them
-// on the ALU pipe at two cycles each (ncu: 0.39 instructions per cycle for a
-// lone warp, stalled on fixed latencies); its chain is shorter than that.
+// where that form did not apply; second: with masks and choices):
+//   traceback of 4 bands of a 497-aa query        415 -> 133 -> 106 us
+//   of 26,597 bands (20,000 queries)             7394 -> 2250 -> 1440 us
+//   of 4,182 bands (1,000 queries, sensitive)    1283 -> 530 -> 385 us, routes side by side
+//   13 bands up to 2,000 x 4,000, scores    1,206,000 -> 1,140 -> 950 us
 #include "kernels.h"
 #include "sw_common.cuh"
 
@@ -93,37 +96,31 @@ __device__ __forceinline__ void stage_scores(int8_t* mat, const int8_t* scores62
   __syncthreads();
 }
 
+// Adds the sign bit of x below the bits of v: one funnel shift.
+__device__ __forceinline__ uint32_t push_sign(uint32_t v, int x) { return __funnelshift_l((uint32_t)x, v, 1); }
+
 // R rows of one column.  up = (hu, eu): the row above row 0 at this column;
-// hd: that row's H one column before.  cw = c - (W - 1): row r is right of the
-// band when cw > r.  left(r): row r is left of the band in this lane.
-template <int R, bool TR, typename Left>
+// hd: that row's H one column before.  dead(r): 0, or kNegI where row r is
+// outside the band: its H is then 0, its E and F near -inf.  In trace mode
+// returns a nibble per row, row 0's highest: f_ext << 3 | e_ext << 2 | (F > E)
+// << 1 | (max(E, F) > D).
+template <int R, bool TR, typename Dead>
 __device__ __forceinline__ uint32_t column(int (&hl)[R], int (&f)[R], int hd, int& hu, int& eu, const uint32_t* w,
-                                           int cw, int oc, int ge, Left left) {
+                                           int oc, int ge, Dead dead) {
   uint32_t nib = 0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const bool in = cw <= r;
-    const int pe = in ? -ge : kNegI, po = in ? -oc : kNegI;
-    const int te = eu + pe, to = hu + po;
-    const int e = max(te, to);
-    const int tf = f[r] - ge, tfo = hl[r] - oc;
-    int fn = max(tf, tfo);
-    const int d = hd + score_byte(w[r >> 2], r & 3);
-    int x = max(max(d, fn), 0);
-    x = in ? x : 0;
-    int h = max(x, e);
+    const int z = dead(r);
+    const int te = eu + z - ge, to = hu + z - oc;
+    const int tf = f[r] + z - ge, tfo = hl[r] + z - oc;
+    const int e = max(te, to), fn = max(tf, tfo), g = max(e, fn);
+    const int d = hd + score_byte(w[r >> 2], r & 3) + z;
+    const int h = __vimax_s32_relu(d, g);
     if (TR) {
-      const int m1 = max(d, 0);
-      uint32_t b = d > 0 ? 1u : 0u;
-      b = e > m1 ? 2u : b;
-      b = fn > max(m1, e) ? 3u : b;
-      b |= te > to ? 4u : 0u;
-      b |= tf > tfo ? 8u : 0u;
-      nib |= b << (4 * r);
-    }
-    if (left(r)) {
-      h = 0;
-      fn = kNegI;
+      nib = push_sign(nib, tfo - tf);
+      nib = push_sign(nib, to - te);
+      nib = push_sign(nib, e - fn);
+      nib = push_sign(nib, d - g);
     }
     hd = hl[r];
     hl[r] = h;
@@ -170,7 +167,8 @@ __device__ __forceinline__ CellOut clamped_rows(CellOut b, const uint8_t* q, con
 }
 
 // The walk of one band by a whole warp.  cell(i, j) is the nibble of a cell of
-// the band with i >= 1 and j >= 1.
+// the band with i >= 1 and j >= 1.  It ends where H is 0, and H is known along
+// it: a pair's score less after a diagonal step, a gap's cost more after a gap.
 template <typename Cell>
 __device__ __forceinline__ void walk_warp(const SysArgs& a, uint32_t band, const Band& b, int m, const CellOut& best,
                                           const int8_t* mat, bool single, Cell cell) {
@@ -185,6 +183,7 @@ __device__ __forceinline__ void walk_warp(const SysArgs& a, uint32_t band, const
   uint32_t ident = 0, pos = 0;  // per lane, summed at the end
   uint32_t cur_op = 3, cur_cnt = 0;
   bool in_gap = false;
+  int h = best.best;  // H of (i, j) in state 0
   // runs are found last to first: they fill the band's slots from the end
   auto emit = [&](uint32_t op, uint32_t cnt) {
     if (op == cur_op) {
@@ -204,26 +203,34 @@ __device__ __forceinline__ void walk_warp(const SysArgs& a, uint32_t band, const
     const int ci = i - di, cj = j - dj;
     const int64_t d = (int64_t)ci - cj;
     const bool ok = single ? lane == 0 : ci > 0 && cj > 0 && d >= b.d0 && d <= b.d1;
-    const uint32_t nb = !ok ? 0u : single ? 1u : cell(ci, cj);
+    const uint32_t nb = !ok || single ? 0u : cell(ci, cj);
     if (__shfl_sync(kAll, (int)ok, 0) == 0) break;  // outside the row's range (gapped.rs:216)
     if (state == 0) {
-      const uint32_t stop = __ballot_sync(kAll, (nb & 3u) != 1u);
+      const uint32_t x = ok ? q[ci - 1] : 0u, y = ok ? s[cj - 1] : 0u;
+      const int sc = mat[min(x, 24u) * 32 + min(y, 24u)];
+      int sum = ok ? sc : 0;  // of this cell's pair and those before it
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kAll, sum, o);
+        if (lane >= o) sum += v;
+      }
+      // a run ends before a cell whose H is 0 or came from a gap
+      const uint32_t stop = __ballot_sync(kAll, !ok || (nb & 1u) != 0 || h - (sum - sc) <= 0);
       const uint32_t run = stop ? (uint32_t)__ffs(stop) - 1u : 32u;
       if (run == 0) {
-        const uint32_t ch = __shfl_sync(kAll, nb, 0) & 3u;
-        if (ch == 0) break;
-        state = ch == 2 ? 1 : 2;
+        if (h <= 0) break;
+        state = (__shfl_sync(kAll, nb, 0) & 2u) ? 2 : 1;
         continue;
       }
       if ((uint32_t)lane < run) {
-        const uint32_t x = q[ci - 1], y = s[cj - 1];
         ident += x == y;
-        pos += mat[min(x, 24u) * 32 + min(y, 24u)] > 0;
+        pos += sc > 0;
       }
       emit(0, run);
       matches += run;
       length += run;
       in_gap = false;
+      h -= __shfl_sync(kAll, sum, (int)run - 1);
       i -= (int)run;
       j -= (int)run;
       if (single) break;  // a row past m + d1 holds one cell
@@ -239,6 +246,7 @@ __device__ __forceinline__ void walk_warp(const SysArgs& a, uint32_t band, const
       gaps += run;
       if (!in_gap) ++openings;
       in_gap = true;
+      h += (int)run * a.ge + (open ? a.oc - a.ge : 0);
       if (state == 1) i -= (int)run;
       else j -= (int)run;
       if (open) state = 0;
@@ -325,19 +333,21 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
     const int turns = sys_rot_turns(S, W, R);
     Word* tr = TR ? reinterpret_cast<Word*>(sys_trace(a, t)) + lane : nullptr;
     int hl[R], f[R];
-    int rowmax[TR ? R : 1], rowcol[TR ? R : 1];
-    int top = 0;  // score mode: the strip's maximum
+    int out[kLag];  // per column of the last R + 1: kNegI where the strip's first row is outside its band
+    // the strip's maximum; in trace mode with its place, the first row-major
+    // one the largest: (H * R + R - 1 - row) * 512 + 511 - column
+    uint32_t top = 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       hl[r] = 0;
       f[r] = kNegI;
     }
 #pragma unroll
-    for (int r = 0; r < (TR ? R : 1); ++r) rowmax[r] = rowcol[r] = 0;
+    for (int u = 0; u < kLag; ++u) out[u] = kNegI;
     CellOut best{0, 0x7FFFFFFF, 0};
     int s = lane;                    // this lane's strip
     int c = -kLag * lane;            // its column at the coming step
-    int cw_off = s < S ? W - 1 : -(1 << 28);  // c - cw_off <= r: inside the right edge
+    unsigned width = s < S ? W : 0;  // columns [0, width) are in its first row's band
     int p = g.rs - g.d1 - 1 - lane;  // subject index of that column
     auto letter = [&](int x) -> uint32_t {
       return (unsigned)x < (unsigned)m ? min((uint32_t)__ldg(sl + x), 24u) : (uint32_t)kSentinel;
@@ -371,25 +381,14 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
     };
     // fold the finished strip's maximum into the lane's best
     auto fold = [&]() {
-      const int i0 = g.rs + R * s;
-      if (TR) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (rowmax[r] > best.best) {
-            best.best = rowmax[r];
-            best.bi = i0 + r;
-            best.bj = i0 - g.d1 + rowcol[r];
-          }
-        }
-      } else if (top > best.best) {
-        best.best = top;
-        best.bi = i0 + R - 1;  // a bound of the best's row
+      const int h = (int)(TR ? top / (512 * R) : top);
+      if (h > best.best) {
+        const int row = TR ? R - 1 - (int)(top / 512 % R) : R - 1;  // score mode: a bound of the best's row
+        best.best = h;
+        best.bi = g.rs + R * s + row;
+        best.bj = g.rs + R * s - g.d1 + 511 - (int)(top % 512);
       }
-    };
-    auto clear_max = [&]() {
       top = 0;
-#pragma unroll
-      for (int r = 0; r < (TR ? R : 1); ++r) rowmax[r] = 0;
     };
     __syncwarp();
     if (S > 0) build(0);
@@ -410,29 +409,19 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
       if (k + 1 < S) build(k + 1);
       if (k >= 31 && lane == ((k + 1) & 31)) {
         fold();
-        clear_max();
         s += 32;
         c -= 32 * kLag;
         p -= 32;
-        if (s >= S) cw_off = -(1 << 28);
+        if (s >= S) width = 0;
       }
-      const bool starts = lane == (k & 31);
-      if (starts) {
-        clear_max();
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          hl[r] = 0;
-          f[r] = kNegI;
-        }
-      }
+      // (the R + 1 dead columns before a strip leave H = 0 and F near -inf)
+      if (lane == (k & 31)) top = 0;
       __syncwarp();
 #pragma unroll
       for (int u = 0; u < kLag; ++u) {
+        // (strip 0 has lane 31 above it, which is dead until its first strip)
         int hu = __shfl_sync(kAll, h_out, src), eu = __shfl_sync(kAll, e_out, src);
-        if (s == 0) {  // above the band's first row
-          hu = 0;
-          eu = kNegI;
-        }
+        out[u] = (unsigned)c < width ? 0 : kNegI;
         uint32_t w[kWords];
 #pragma unroll
         for (int x = 0; x < kWords; ++x) {
@@ -442,23 +431,21 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
         l1 = letter(p + 2);
         const int hd = hup;
         hup = hu;
-        const uint32_t nib = column<R, TR>(hl, f, hd, hu, eu, w, c - cw_off, a.oc, a.ge,
-                                           [&](int r) { return u < R - 1 && r > u && starts; });
+        const uint32_t nib = column<R, TR>(hl, f, hd, hu, eu, w, a.oc, a.ge,
+                                           [&](int r) { return out[(u - r + kLag) % kLag]; });
         h_out = hu;
         e_out = eu;
         if (TR) {
           *tr = (Word)nib;
           tr += 32;
+          uint32_t t = 0;
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            if (hl[r] > rowmax[r]) {
-              rowmax[r] = hl[r];
-              rowcol[r] = c;
-            }
-          }
+          for (int r = 0; r < R; r += 2)
+            t = __vimax3_u32(t, (uint32_t)hl[r] * R + (R - 1 - r), (uint32_t)hl[r + 1] * R + (R - 2 - r));
+          top = max(top, t * 512u + (uint32_t)(511 - c));
         } else {
 #pragma unroll
-          for (int r = 0; r < R; ++r) top = max(top, hl[r]);
+          for (int r = 0; r < R; r += 2) top = __vimax3_u32(top, (uint32_t)hl[r], (uint32_t)hl[r + 1]);
         }
         ++c;
         ++p;
@@ -485,7 +472,7 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
       walk_warp(a, band, b, m, best, mat, single, [&](int i, int j) -> uint32_t {
         const int ii = i - g.rs, sk = ii / R, r = ii % R;
         const int cc = j - (g.rs + R * sk - g.d1);
-        return ((uint32_t)base[(int64_t)(cc + kLag * sk) * 32 + (sk & 31)] >> (4 * r)) & 15u;
+        return ((uint32_t)base[(int64_t)(cc + kLag * sk) * 32 + (sk & 31)] >> (4 * (R - 1 - r))) & 15u;
       });
     }
     __syncwarp();
@@ -662,8 +649,6 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_pair(SwBandArgs 
         hl[r] = 0;
         f[r] = 0;
       }
-#pragma unroll
-      for (int u = 0; u < kLag; ++u) out[u] = kDead2;
     }
     __syncwarp();
 #pragma unroll
@@ -745,6 +730,7 @@ __global__ void __launch_bounds__(kBlkWarps * 32) k_sys_block(SysArgs a) {
     const SysBlockPlan plan = sys_block_plan(g, m);
     uint16_t* tr = TR ? reinterpret_cast<uint16_t*>(sys_trace(a, t)) : nullptr;
     int hl[R], f[R], rowmax[R], rowcol[R];
+    int out[R] = {};  // of the last R columns: kNegI where the lane's first row is outside its band
     CellOut best{0, 0x7FFFFFFF, 0};
     int hup = 0, h_out = 0, e_out = kNegI;
     int s = warp, turn = 0;  // this warp's strip
@@ -781,6 +767,7 @@ __global__ void __launch_bounds__(kBlkWarps * 32) k_sys_block(SysArgs a) {
             hl[r] = 0;
             f[r] = kNegI;
             rowmax[r] = rowcol[r] = 0;
+            out[r] = (unsigned)(32 * B - lane - (il - g.d1) - (R - r)) < (unsigned)W ? 0 : kNegI;
           }
           hup = 0;
           h_out = 0;
@@ -811,8 +798,9 @@ __global__ void __launch_bounds__(kBlkWarps * 32) k_sys_block(SysArgs a) {
             l0 = (unsigned)j < (unsigned)m ? min((uint32_t)__ldg(sl + j), 24u) : (uint32_t)kSentinel;
             const int hd = hup;
             hup = hu;
-            const uint32_t nib = column<R, TR>(hl, f, hd, hu, eu, &w, c - (W - 1), a.oc, a.ge,
-                                               [&](int r) { return c < r; });
+            out[x % R] = (unsigned)c < (unsigned)W ? 0 : kNegI;
+            const uint32_t nib = column<R, TR>(hl, f, hd, hu, eu, &w, a.oc, a.ge,
+                                               [&](int r) { return out[(x - r + R) % R]; });
             h_out = hu;
             e_out = eu;
 #pragma unroll
@@ -866,7 +854,7 @@ __global__ void __launch_bounds__(kBlkWarps * 32) k_sys_block(SysArgs a) {
           const int ii = i - g.rs, sk = ii / kBlkRows, ln = (ii / R) & 31, r = ii % R;
           const int j0 = j + ln;  // lane 0's column when lane ln was at j
           const int64_t at = (int64_t)sk * plan.nb + ((j0 >> 5) - plan.b0(g, sk));
-          return ((uint32_t)tr[(at * 32 + (j0 & 31)) * 32 + ln] >> (4 * r)) & 15u;
+          return ((uint32_t)tr[(at * 32 + (j0 & 31)) * 32 + ln] >> (4 * (R - 1 - r))) & 15u;
         });
       }
     }

@@ -35,3 +35,15 @@ def test_widest_bands(ctx, orc, width):
     for k, (a, b, d0, d1) in enumerate(jobs):
         e, _ = orc.extend_span(qs[a], ss[b], d0, d1, "BLOSUM62")
         assert int(got[k]) == (e[0] if e else 0), jobs[k]
+
+
+@pytest.mark.parametrize("rows,width", [(8191, 151), (8192, 200), (8193, 200), (16384, 100), (16385, 100)])
+def test_longest_traced_bands(ctx, orc, rows, width):
+    # at the row limit of the rotating traceback kernel the block kernel takes over
+    r = np.random.Generator(np.random.PCG64(rows))
+    q = synth.random_protein(r, rows)
+    s = synth.mutate(r, q, 0.8)
+    jobs = [(0, 0, -width // 2, -width // 2 + width - 1)]
+    got = ctx.extend_span([q], [s], jobs)
+    exp, _ = orc.extend_span(q, s, jobs[0][2], jobs[0][3], "BLOSUM62")
+    assert got[0] == exp
