@@ -59,18 +59,49 @@ void upload_seed_params(const ShapeTable& shapes, const SeedParams& params, int 
                                    cudaMemcpyHostToDevice, st));  // pageable source: staged before return
 }
 
-__global__ void k_letter_owner(const uint64_t* __restrict__ offsets, uint64_t n_seqs, uint64_t lo, uint64_t hi,
-                               uint32_t* __restrict__ out) {
-  uint64_t g = lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (g >= hi) return;
-  // largest i with offsets[i] <= g (sequences may be empty)
-  uint64_t a = 0, b = n_seqs;  // answer in [a, b)
-  while (b - a > 1) {
-    uint64_t m = (a + b) >> 1;
-    if (offsets[m] <= g) a = m;
-    else b = m;
+// The sequence of every letter in [lo, hi): out[g - lo] is the largest i with
+// offsets[i] <= g (sequences may be empty).  Four letters per thread, written
+// as one vector.  A block first brackets its 1,024 letters, so that a thread
+// searches the few sequences among them instead of all.  (One search over all
+// per letter: 330 us for the 24M letters of 80,000 sequences, now 93.)  VEC:
+// out is 16-byte aligned.
+constexpr int kOwnerBlock = 256;
+template <bool VEC>
+__global__ void __launch_bounds__(kOwnerBlock) k_letter_owner(const uint64_t* __restrict__ offsets, uint64_t n_seqs,
+                                                              uint64_t lo, uint64_t hi, uint32_t* __restrict__ out) {
+  __shared__ uint64_t bracket[2];
+  const auto find = [&](uint64_t g, uint64_t a, uint64_t b) {  // answer in [a, b)
+    while (b - a > 1) {
+      const uint64_t m = (a + b) >> 1;
+      if (offsets[m] <= g) a = m;
+      else b = m;
+    }
+    return a;
+  };
+  const uint64_t first = lo + blockIdx.x * (uint64_t)(4 * kOwnerBlock);
+  const uint64_t last = min(hi, first + 4 * kOwnerBlock) - 1;
+  if (threadIdx.x % 32 == 0 && threadIdx.x < 64) {
+    const int w = threadIdx.x / 32;
+    bracket[w] = find(w ? last : first, 0, n_seqs) + w;
   }
-  out[g - lo] = (uint32_t)a;
+  __syncthreads();
+  const uint64_t g = first + 4 * threadIdx.x;
+  if (g > last) return;
+  uint64_t i = find(g, bracket[0], bracket[1]);
+  uint32_t v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k > 0 && g + k <= last && i + 1 < bracket[1] && offsets[i + 1] <= g + k) i = find(g + k, i + 1, bracket[1]);
+    v[k] = (uint32_t)i;
+  }
+  uint32_t* o = out + (g - lo);
+  if (VEC && g + 3 <= last) {
+    *reinterpret_cast<uint4*>(o) = make_uint4(v[0], v[1], v[2], v[3]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (g + k <= last) o[k] = v[k];
+  }
 }
 
 // Letter codes above 24 score as 24 (matrix.rs:164-168 clamps both indices)
@@ -114,7 +145,11 @@ void launch_letter_owner(const uint64_t* offsets, uint64_t n_seqs, uint64_t lo, 
                          cudaStream_t st) {
   if (hi <= lo || n_seqs == 0) return;
   count_launch();
-  k_letter_owner<<<ceil_div(hi - lo, 256), 256, 0, st>>>(offsets, n_seqs, lo, hi, out);
+  const unsigned blocks = ceil_div(hi - lo, 4 * kOwnerBlock);
+  if (reinterpret_cast<uintptr_t>(out) % 16 == 0)
+    k_letter_owner<true><<<blocks, kOwnerBlock, 0, st>>>(offsets, n_seqs, lo, hi, out);
+  else
+    k_letter_owner<false><<<blocks, kOwnerBlock, 0, st>>>(offsets, n_seqs, lo, hi, out);
   DRG_CUDA(cudaGetLastError());
 }
 
@@ -363,14 +398,15 @@ void launch_seed_entries(const uint32_t* keys, const uint32_t* vals, uint64_t n,
 // of the query keys.  The bitmap is hashed: a false positive only keeps a
 // seed that then matches no query run, and no key of the query is missed.
 
-
+// (A look at the word before the atomic waits for a random read per key and
+// saves few atomics: run keys are distinct.)
 __global__ void k_key_filter(const uint64_t* __restrict__ run_keys, uint64_t n, uint64_t key_mask,
                              uint32_t* __restrict__ filter, int log2_bits) {
   const uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (u >= n) return;
   const uint32_t h = seed_key_hash(run_keys[u] & key_mask, log2_bits);
   const uint32_t bit = 1u << (h & 31);
-  if (!(filter[h >> 5] & bit)) atomicOr(filter + (h >> 5), bit);
+  atomicOr(filter + (h >> 5), bit);
 }
 
 void launch_key_filter(const uint64_t* run_keys, uint64_t n, uint64_t key_mask, uint32_t* filter, int log2_bits,
