@@ -340,8 +340,7 @@ constexpr int kSwC0 = 136, kSwC1 = 272, kSwC2 = 544, kSwC3 = 1700;
 constexpr int kSwClassMax[4] = {kSwC0, kSwC1, kSwC2, kSwC3};  // 4, 2, 1, 1 warps per block
 constexpr int kSwMaxWidth = 1700;                       // wider bands use the exact kernel
 // Bands whose best can reach this bound are not packed: every H of the packed
-// kernel stays below 0x7C00 (its strip maximum folds H on the FMA pipe as
-// half-precision bit patterns) and far from the 16-bit limit.
+// kernels stays far from the 16-bit limit.
 constexpr int kSwPackedMaxBest = 31743;
 constexpr int kSwClasses = 4;
 int sw_width_class(int width);  // 0..3, or -1 for the exact kernel

@@ -30,13 +30,10 @@ __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
   asm("max.s16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
-// Maximum of two pairs of non-negative 16-bit integers below 0x7C00 on the
-// FMA pipe: such bit patterns are zero, subnormal or finite positive halves,
-// ordered like the integers, and max.f16x2 (no flush to zero) returns one of
-// its inputs.
-__device__ __forceinline__ uint32_t max2_pos_f16(uint32_t a, uint32_t b) {
+// x << n, 0 from n = 32 on.
+__device__ __forceinline__ uint32_t shl_clamp(uint32_t x, int n) {
   uint32_t r;
-  asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(n));
   return r;
 }
 // Sign-extending byte pick: low half = byte b of lo, high half = byte b of hi.

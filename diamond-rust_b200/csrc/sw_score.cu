@@ -30,24 +30,31 @@
 //
 // In this form all of H, E' and F' are at least 0, no H - oc is kept, and a
 // cell outside the band or the matrix is plain 0 (E' = 0 is E = -oc, which
-// raises nothing).  A pair update is six half-rate ALU operations, of which
-// only the last two wait for the pair above:
+// raises nothing).  A pair update is four operations of the ALU pipe, at two
+// cycles a warp each, and three adds of the FMA pipe, which runs beside:
 //   sc = the pair's two scores (one byte permute)
-//   X  = max(F' - oc, Hdiag + sc, 0)   (add, viaddmax.relu)
-//   E' = max(E' - ge, H of the pair above)   (viaddmax)
-//   H  = max(E' - oc, X)               (viaddmax)
-//   F' = max(F' - ge, H)               (viaddmax, for the next column)
-// ALU bound, then by the chain of E' and H down the pairs.  The residues are
-// loaded four columns ahead of their use.  Against the same cell with H - oc
-// kept beside H and residues two columns ahead: 18.05 -> 17.75 ms for the
-// 1,000-query sensitive search, 15.60 -> 15.27 for 250 very-sensitive queries.
-// One operation less on the ALU pipe, G = max(E', F') as a half-precision
-// maximum and H = max(G - oc, D, 0), is slower (17.98 ms): the maximum
-// lengthens the chain.
+//   E' = max(E' - ge, H of the pair above)            (viaddmax)
+//   H  = max(Hdiag + sc, E' - oc, F' - oc, 0)         (three adds, vimax3.relu)
+//   F' = max(F' - ge, H)                              (viaddmax, for the next column)
+// Near a strip's ends a cell outside the band is dead by an addend of -16384 on
+// its diagonal and open cost, as in the lane kernel (sw_sys.cu).
+//
+// ALU bound (that pipe is busy 86 % of the time).  What held it at 76 % before
+// was not the arithmetic: with the first and last 16 steps of a strip
+// unrolled, each with its masks, the twelve warps of an SM were spread over
+// 40 KB of code, and instruction fetch past the SM's own cache ran at 91 % of
+// its peak; neither more warps nor fewer operations changed anything.
+// Now two loops of four steps make up a strip, edges and middle.  A loop holds
+// whole groups of four columns because a load in flight that is moved from
+// register to register waits, so letters come four at a time as words, a group
+// ahead (loaded singly into a rotating queue, with loops of 1, 2, 3 and 4
+// steps: 23.0, 18.4, 17.6 and 17.0 ms for the 1,000-query sensitive search;
+// unrolled edges 16.8; now 15.25, and 13.8 -> 12.6 ms for 250 very-sensitive
+// queries).
 //
 // Exactness: values equal the reference's int32 DP while the band's best is
 // below 31744 = 0x7C00 (bands that could reach it are not given to this
-// kernel); the strip maximum relies on that bound (max2_pos_f16).
+// kernel).
 // Cells with j < 0, j > m or rows past the query read a sentinel residue
 // scoring -64; they can neither raise the maximum above the true band maximum
 // nor feed an in-band cell.  Rows past m + d1 are not computed: the reference
@@ -55,7 +62,7 @@
 // max(largest matrix score, band best - open), so a packed best above the
 // matrix's largest score is the reference's; smaller results are recomputed
 // exactly.  Cells left or right of the band in the first/last 16 steps of
-// a strip are masked to 0: their H does not count and they pass no gap.
+// a strip are dead: their H is 0 and they pass no gap.
 //
 // The traceback of the HSPs that pass the gate runs in sw_sys.cu.
 #include "kernels.h"
@@ -71,6 +78,41 @@ constexpr int kParts = 32 / kSwPart;  // tasks per warp
 constexpr int kProfHigh = 26 * 8;     // profile bytes of rows 8 to 15, after those of rows 0 to 7
 constexpr int kProfBytes = 2 * kProfHigh;
 
+// The column letters of one lane, a group of four columns at a time: taken
+// from the two aligned words that hold them (the second is the next group's
+// first), fetched a group ahead.  Every letter buffer starts on a word
+// boundary and has slack behind its end.
+struct Letters : Lane {
+  uint32_t w0, w1;  // aligned words: of the next group's first letter, and the one after
+  uint32_t shift;   // bits of w0 before the group's first letter
+  int j;            // subject index of the next group's first column
+};
+
+// The aligned word of letters [t, t + 4), s + t on a word boundary; not read
+// where no letter of it is the sequence's.
+__device__ __forceinline__ uint32_t letter_word(const Letters& L, int t) {
+  return (unsigned)t + 3u < (unsigned)L.m + 3u ? __ldg(reinterpret_cast<const uint32_t*>(L.s + t)) : 0u;
+}
+// Before column c (a multiple of 4) of a strip.
+__device__ __forceinline__ void letters_at(Letters& L, int c) {
+  L.j = L.jbase + c - 1;
+  const int off = (int)((reinterpret_cast<uintptr_t>(L.s) + (intptr_t)L.j) & 3);
+  L.shift = 8 * off;
+  L.w0 = letter_word(L, L.j - off);
+  L.w1 = letter_word(L, L.j - off + 4);
+}
+// The next four columns' residues, the sentinel off the sequence.
+__device__ __forceinline__ uint32_t next_letters(Letters& L) {
+  const uint32_t w = __funnelshift_r(L.w0, L.w1, L.shift);
+  L.w0 = L.w1;
+  L.w1 = letter_word(L, L.j + 8 - (int)(L.shift >> 3));
+  const uint32_t below = shl_clamp(0xFFFFFFFFu, 8 * __vimin_s32_relu(-L.j, 4));      // letters from index 0 on
+  const uint32_t past = shl_clamp(0xFFFFFFFFu, 8 * __vimin_s32_relu(L.m - L.j, 4));  // letters from index m on
+  const uint32_t in = below & ~past;
+  L.j += 4;
+  return (w & in) | (0x01010101u * kSentinel & ~in);
+}
+
 // Registers of one lane's 16-row strip in the score pass.
 struct SRegs {
   uint32_t H[kPairs], F[kPairs];
@@ -80,126 +122,71 @@ struct SRegs {
   uint32_t mx0, mx1;  // maximum H of the strip so far, folded over rows
 };
 
-// One column step.  MODE 0: middle (all rows in band), 1: prologue step
-// C (= c), 2: epilogue step C (= c - W) of a warp whose bands share one
-// width, 3: step past the narrowest band of a warp with mixed widths
-// (cw = c - this lane's W, masks computed at run time).  rp holds the
-// (H, E') word of the row above row 0 at column c; wp receives row 15's word of
-// column c - 1.
-template <int MODE, int C>
-__device__ __forceinline__ void sw_step(SRegs& R, Lane& L, int c, const uint8_t* __restrict__ prof,
-                                        const uint32_t* __restrict__ rp, uint32_t* __restrict__ wp, uint32_t noc2,
-                                        uint32_t nge2, int cw = 0) {
-  const uint32_t res = next_residue(L, c);  // subject residue of this column
+// The residue of a group's column k.
+__device__ __forceinline__ uint32_t residue(uint32_t r4, int k) { return prmt(r4, 0u, 0x4440u + k); }
+
+// One column step.  res is the column's residue, rw the (H, E') word of the row above row 0 at column c;
+// wp receives row 15's word of column c - 1.  EDGE: near a strip's first and
+// last columns, where M[p] holds what pair p's cells outside the band add.
+template <bool EDGE>
+__device__ __forceinline__ void sw_step(SRegs& R, uint32_t res, const uint8_t* __restrict__ prof, uint32_t rw,
+                                        uint32_t* __restrict__ wp, uint32_t noc2, uint32_t nge2,
+                                        const uint32_t (&M)[kPairs]) {
   const uint8_t* prow = prof + res * 8;
   const uint2 lo8 = *reinterpret_cast<const uint2*>(prow);
   const uint2 hi8 = *reinterpret_cast<const uint2*>(R.prow_prev + kProfHigh);
   R.prow_prev = prow;
-  const uint32_t rw = *rp;  // (H, E') of the row above row 0, column c
   const uint32_t h_top = prmt(rw, R.H[kPairs - 1], 0x5410);
   uint32_t h_up = h_top;
   uint32_t e_up = prmt(rw, R.E7, 0x5432);
   uint32_t hd = R.htop_old;
 #pragma unroll
   for (int p = 0; p < kPairs; ++p) {
-    // Pairs whose two halves are both outside the band at this compile-time
-    // step are not computed: left of it in the prologue (C < p), right of it
-    // in a one-width epilogue (C >= p + 9).  They take the values the masks
-    // below would give (0) and hand the next pair the same E/H the masked
-    // computation would; in the prologue every pair below is skipped too, and
-    // the E' of pair 7 is first read by row 8 at step 9, when pair 7 is
-    // computed again.
-    if ((MODE == 1 && C < p) || (MODE == 2 && C >= p + 9)) {
-      hd = R.H[p];
-      R.H[p] = 0;
-      R.F[p] = 0;
-      h_up = 0;
-      e_up = 0;
-      continue;
+    uint32_t sc = prmt(p < 4 ? lo8.x : lo8.y, p < 4 ? hi8.x : hi8.y, pick_sel(p & 3));
+    uint32_t no = noc2;
+    if (EDGE) {
+      sc = add2(sc, M[p]);
+      no = add2(no, M[p]);
     }
-    const uint32_t sc = prmt(p < 4 ? lo8.x : lo8.y, p < 4 ? hi8.x : hi8.y, pick_sel(p & 3));
-    uint32_t f = R.F[p];
-    uint32_t e = __viaddmax_s16x2(e_up, nge2, h_up);
-    uint32_t h = __viaddmax_s16x2(e, noc2, __viaddmax_s16x2_relu(f, noc2, add2(hd, sc)));
-    if (MODE == 1) {
-      // left of the band: row p at column C (low), row p+8 at column C-1 (high)
-      const bool lo_left = C < p;
-      const bool hi_left = C <= p + 8;
-      const uint32_t k = (lo_left ? 0u : 0x0000FFFFu) | (hi_left ? 0u : 0xFFFF0000u);
-      if (k != 0xFFFFFFFFu) {
-        h = h & k;  // no score toward the entry cell (F' is 0 there already)
-      }
-    } else if (MODE == 2) {
-      const bool lo_right = C >= p;
-      const bool hi_right = C >= p + 9;
-      const uint32_t k = (lo_right ? 0u : 0x0000FFFFu) | (hi_right ? 0u : 0xFFFF0000u);
-      if (k != 0xFFFFFFFFu) {
-        h = h & k;
-        e = e & k;
-      }
-    } else if (MODE == 3) {
-      // right of this lane's band: row p at column c (low), row p+8 at column c-1 (high)
-      const uint32_t k = (cw >= p ? 0u : 0x0000FFFFu) | (cw >= p + 9 ? 0u : 0xFFFF0000u);
-      h = h & k;
-      e = e & k;
-    }
+    const uint32_t f = R.F[p];
+    const uint32_t e = __viaddmax_s16x2(e_up, nge2, h_up);
+    // (at the edges the FMA pipe has two adds more: one of these goes back)
+    const uint32_t h = EDGE ? __viaddmax_s16x2(e, no, __viaddmax_s16x2_relu(f, no, add2(hd, sc)))
+                            : __vimax3_s16x2_relu(add2(hd, sc), add2(f, no), add2(e, no));
     hd = R.H[p];
     R.H[p] = h;
     R.F[p] = __viaddmax_s16x2(f, nge2, h);
     h_up = h;
     e_up = e;
   }
-  // the strip's maximum, two accumulators of four pairs each, on the FMA
-  // pipe (H is in [0, 0x7C00): see max2_pos_f16), beside the ALU's DP work
-  R.mx0 = max2_pos_f16(R.mx0, max2_pos_f16(R.H[0], R.H[1]));
-  R.mx1 = max2_pos_f16(R.mx1, max2_pos_f16(R.H[4], R.H[5]));
-  R.mx0 = max2_pos_f16(R.mx0, max2_pos_f16(R.H[2], R.H[3]));
-  R.mx1 = max2_pos_f16(R.mx1, max2_pos_f16(R.H[6], R.H[7]));
+  // the strip's maximum, two accumulators of four pairs each
+  R.mx0 = __vimax3_s16x2(R.mx0, R.H[0], R.H[1]);
+  R.mx1 = __vimax3_s16x2(R.mx1, R.H[4], R.H[5]);
+  R.mx0 = __vimax3_s16x2(R.mx0, R.H[2], R.H[3]);
+  R.mx1 = __vimax3_s16x2(R.mx1, R.H[6], R.H[7]);
   R.E7 = e_up;
-  *wp = prmt(R.H[kPairs - 1], R.E7, 0x7632);  // (H, E') of row 15 at column c - 1
+  // (H, E') of row 15 at column c - 1; E' dead with its row
+  *wp = prmt(R.H[kPairs - 1], EDGE ? add2(R.E7, M[kPairs - 1]) : R.E7, 0x7632);
   R.htop_old = h_top;
 }
 
-// The ring of one lane: W + 1 words at stride `stride`; rp reads column c,
-// wp (the slot read one step earlier) takes column c - 1.
-struct RingPtr {
-  uint32_t *rp, *wp;
-  uint32_t* begin;
-  uint32_t* end;
-  int stride;
-  __device__ __forceinline__ void advance() {
-    wp = rp;
-    rp += stride;
-    if (rp == end) rp = begin;
-  }
-};
-
-template <int MODE, int C>
-struct Unroll {
-  static __device__ __forceinline__ void run(SRegs& R, Lane& L, int c0, const uint8_t* prof, RingPtr& rg,
-                                             uint32_t noc2, uint32_t nge2) {
-    sw_step<MODE, C>(R, L, c0 + C, prof, rg.rp, rg.wp, noc2, nge2);
-    rg.advance();
-    Unroll<MODE, C + 1>::run(R, L, c0, prof, rg, noc2, nge2);
-  }
-};
-template <int MODE>
-struct Unroll<MODE, kRows> {
-  static __device__ __forceinline__ void run(SRegs&, Lane&, int, const uint8_t*, RingPtr&, uint32_t, uint32_t) {}
-};
+// Words of a lane's ring: at least W + 1, a whole number of groups.  (A strip
+// may run up to three columns past W + 16, to the end of a group; then the
+// ring has a word more for each but two, which keeps the words that it writes
+// there off those that the next strip reads.)
+__host__ __device__ constexpr int ring_words(int W) { return (W + 4) & ~3; }
 
 // Score pass: scores[band] = the band's best H, best_row[band] = the last row
 // of the first strip that holds it (an upper bound of the reference's best_i,
 // which is all the traceback pass needs).
-// Shared memory holds three blocks per SM in the 4- and 2-warp classes, so
-// registers are budgeted for three (without the hint the compiler spills).
+// Shared memory holds three blocks per SM in the 4- and 2-warp classes.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int part = lane / kSwPart, at = lane % kSwPart;
   const uint64_t task_id = a.task_lo + ((uint64_t)blockIdx.x * WARPS + warp) * kParts;
-  const int stride = WARPS * 32;
+  constexpr int stride = WARPS * 32;
   int8_t* mat = reinterpret_cast<int8_t*>(smem);  // 25 x 25 scores
   uint8_t* prof = smem + 640 + (warp * kParts + part) * kProfBytes;  // strip profile
   uint32_t* ring = reinterpret_cast<uint32_t*>(smem + 640 + WARPS * kParts * kProfBytes) + threadIdx.x;
@@ -212,7 +199,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
   const int W = (int)__reduce_max_sync(0xFFFFFFFFu, task.width);     // widest band of the warp
   const int Wmin = (int)__reduce_min_sync(0xFFFFFFFFu, task.w_min);  // narrowest
   const uint32_t n_strips = __reduce_max_sync(0xFFFFFFFFu, task.n_strips);
-  const int buf = W + 1;
+  const int buf = ring_words(W);
   const bool active = !idle && at < (int)task.count;
   const uint32_t bidx = a.order[task.first + (at < (int)task.count ? at : 0)];
   const Band band = a.bands[bidx];
@@ -227,7 +214,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
   const uint8_t* q = tr ? sj : qw;  // row letters
   const int n = tr ? m_s : (int)band.n;
   const int d1 = tr ? -band.d0 : band.d1;
-  Lane L;
+  Letters L;
   L.s = tr ? qw : sj;  // column letters
   L.m = tr ? (int)band.n : m_s;
   const uint32_t noc2 = (uint32_t)(uint16_t)(-(a.gap_open + a.gap_extend)) * 0x10001u;
@@ -235,10 +222,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
   // a dead cell's word is 0 (H = 0, E' = 0); the row above the first strip, row
   // 0 of the reference, is dead
   for (int g = 0; g < buf; ++g) ring[g * stride] = 0;
-  RingPtr rg;
-  rg.begin = ring;
-  rg.end = ring + buf * stride;
-  rg.stride = stride;
+  uint32_t* const ring_end = ring + buf * stride;
   int base = 0;  // ring slot of relative column 0 of the current strip
   SRegs R;
   int best = 0, best_i = 0;
@@ -275,54 +259,59 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
     // later strip reads need care (below).
     const int lead = __reduce_min_sync(0xFFFFFFFFu, max(0, 1 - L.jbase));
     const int trail = __reduce_max_sync(0xFFFFFFFFu, L.m + 2 - L.jbase);
-    const int c_begin = lead >= kRows ? min(lead, Wmin) : 0;  // whole prologue or none of it
-    const int c_end = max(c_begin, min(W + kRows, max(trail, kRows)));
+    // (whole groups of columns, and the whole prologue or none of it)
+    const int c_begin = lead >= kRows ? min(lead, Wmin) & ~3 : 0;
+    const int c_end = (max(c_begin, min(W + kRows, max(trail, kRows))) + 3) & ~3;
     steps_done += (uint64_t)(c_end - c_begin);
-    {
-      int slot = base + c_begin;
-      slot = slot >= buf ? slot - buf : slot;
-      rg.rp = ring + slot * stride;
-      rg.wp = ring + (slot == 0 ? buf - 1 : slot - 1) * stride;
-    }
+    // rp: the ring word of column c; wp: the slot before, which takes the word
+    // of column c - 1 once that is read.  base, the ring and c are multiples of
+    // 4 here, so only the end of a group meets the wrap of the ring.
+    int slot = base + c_begin;
+    slot = slot >= buf ? slot - buf : slot;
+    uint32_t* rp = ring + slot * stride;
+    uint32_t* wp = slot == 0 ? ring_end - stride : rp - stride;
     // H of column c_begin - 1 of the row above; row 7 not yet computed: 0
-    R.htop_old = *rg.wp & 0xFFFFu;
-    {
-      const int jm1 = L.jbase + c_begin - 2;  // column c_begin - 1
-      R.prow_prev = prof + subject_residue(L, jm1) * 8;
+    R.htop_old = *wp & 0xFFFFu;
+    R.prow_prev = prof + subject_residue(L, L.jbase + c_begin - 2) * 8;  // column c_begin - 1
+    letters_at(L, c_begin);
+    // The steps with an edge of the band among a strip's rows, the first 16 and
+    // those from the narrowest band's width on, are one loop, entered before and
+    // after the steps between.  Pair p is at the edge p columns after pair 0, so
+    // a step computes one new addend and moves the others on.
+    uint32_t M[kPairs];
 #pragma unroll
-      for (int i = 0; i < kQueue; ++i) L.queue[i] = subject_residue(L, jm1 + 1 + i);
-    }
+    for (int p = 0; p < kPairs; ++p) M[p] = kNeg2;
+    const int mid_end = min(Wmin & ~3, c_end);
     int c = c_begin;
-    if (c_begin == 0) {
-      Unroll<1, 0>::run(R, L, 0, prof, rg, noc2, nge2);
-      c = kRows;
-    }
-    const int mid_end = min(Wmin, c_end);
-    {
-      // in runs that end where the read pointer wraps, so that the steps
-      // themselves carry no wrap test
-      uint32_t* rp = rg.rp;
-      uint32_t* wp = rg.wp;
-      while (c < mid_end) {
-        const int stop = min(mid_end, c + (int)((rg.end - rp) / stride));
-#pragma unroll 2
-        for (; c < stop; ++c) {
-          sw_step<0, 0>(R, L, c, prof, rp, wp, noc2, nge2);
-          wp = rp;
-          rp += stride;
+#pragma unroll 1
+    for (int stop = c_begin == 0 ? kRows : c_begin;; stop = c_end) {
+#pragma unroll 1
+      for (; c < stop; c += 4) {
+        const uint32_t res = next_letters(L);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+#pragma unroll
+          for (int p = kPairs - 1; p > 0; --p) M[p] = M[p - 1];
+          const bool in = c + k < Wl;
+          M[0] = (in ? 0u : kNeg2 & 0xFFFFu) | ((unsigned)(c + k - 9) < (unsigned)Wl ? 0u : kNeg2 & 0xFFFF0000u);
+          sw_step<true>(R, residue(res, k), prof, in ? rp[k * stride] : 0u, k == 0 ? wp : rp + (k - 1) * stride, noc2,
+                        nge2, M);
         }
-        if (rp == rg.end) rp = rg.begin;
+        wp = rp + 3 * stride;
+        rp = rp + 4 * stride == ring_end ? ring : rp + 4 * stride;
       }
-      rg.rp = rp;
-      rg.wp = wp;
-    }
-    if (Wmin == W && c == W && c_end == W + kRows) {  // one width in the warp: compile-time masks
-      Unroll<2, 0>::run(R, L, W, prof, rg, noc2, nge2);
-    } else {  // mixed widths or an early stop: each lane masks past its own right edge
-      for (; c < c_end; ++c) {
-        sw_step<3, 0>(R, L, c, prof, rg.rp, rg.wp, noc2, nge2, c - Wl);
-        rg.advance();
+      if (c == c_end) break;
+#pragma unroll 1
+      for (; c < mid_end; c += 4) {
+        const uint32_t res = next_letters(L);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          sw_step<false>(R, residue(res, k), prof, rp[k * stride], k == 0 ? wp : rp + (k - 1) * stride, noc2, nge2, M);
+        wp = rp + 3 * stride;
+        rp = rp + 4 * stride == ring_end ? ring : rp + 4 * stride;
       }
+#pragma unroll
+      for (int p = 0; p < kPairs; ++p) M[p] = 0;
     }
     // Ring words the next strip may read that this strip did not write: the
     // next strip's column x reads this strip's column x + 16.  Skipped columns
@@ -379,7 +368,7 @@ template <int WARPS>
 void launch_class(const SwScoreArgs& a, int max_width, cudaStream_t st) {
   if (a.task_hi <= a.task_lo) return;
   const int threads = WARPS * 32;
-  const size_t smem = 640 + WARPS * kParts * kProfBytes + (size_t)threads * (max_width + 1) * 4;
+  const size_t smem = 640 + WARPS * kParts * kProfBytes + (size_t)threads * ring_words(max_width) * 4;
   static int configured = 0;  // per template instance
   if ((int)smem > configured) {
     DRG_CUDA(cudaFuncSetAttribute(k_sw<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
