@@ -15,7 +15,7 @@ index-chunks 1.
              (upload, search, download of the HSPs inside the timed step)
   roofline   the banded Smith-Waterman score kernel (the dominant kernel):
              reference DP cells per second against the integer-pipe peak
-             measured live (s16x2 DPX issue rate x 2 cells / 4 ops per cell)
+             measured live (s16x2 DPX lane-ops per second / 2.25 per cell)
   cpu_baseline  the C++ restatement of the reference path (oracle) on the
              host cores, on a bounded sample of the workload
 
@@ -506,9 +506,10 @@ def main():
     w = workload(args.queries)
     ctx = drgpu.Context(local)
     peak_ops, probe_mhz = ctx.probe_int_peak()
-    # the recurrence as implemented: 7 s16x2 ALU ops per 2 cells (score pick,
-    # D add, E and F add-max, H max3 with 0, H - open, strip maximum)
-    ops_per_cell = 3.5
+    # the recurrence as implemented: 4.5 ALU-pipe ops per pair of cells (score
+    # pick, E and F add-max, H max3 with 0, half a max3 for the strip maximum);
+    # its three adds run on the FMA pipe beside
+    ops_per_cell = 2.25
     peak_gcups = peak_ops / ops_per_cell / 1e9
     dl, do = drgpu.concat(w.db)
     tl, to = drgpu.concat(w.queries)
