@@ -469,7 +469,12 @@ __global__ void k_task_steps(const SwTask* tasks, uint64_t n, unsigned long long
   if (t >= n || (d_n && t >= (uint64_t)*d_n)) return;
   const SwTask k = tasks[t];
   if (k.width == kSwNoClass) return;
-  atomicMax(mx + sw_class_of(k.width), (unsigned long long)k.n_strips * (k.width + 16ull));
+  // (tasks come longest first in each class, so most read a maximum already
+  // reached: atomics of every task on one word took 86 us of a 501-query
+  // very-sensitive search)
+  unsigned long long* const at = mx + sw_class_of(k.width);
+  const unsigned long long steps = (unsigned long long)k.n_strips * (k.width + 16ull);
+  if (steps > *(volatile unsigned long long*)at) atomicMax(at, steps);
 }
 
 // Ops of the traced bands, compacted in band order (each band owns n + m slots).
