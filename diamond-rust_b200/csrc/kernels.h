@@ -506,7 +506,14 @@ struct SysJob {
   uint32_t pad;
   uint64_t trace_off;  // first trace byte
 };
-constexpr unsigned kSysBlocks = 148 * 4;  // blocks of the block kernel at once
+// Blocks of the block kernel at once: each has a row of `words` words, one per
+// subject column and one more, and all rows together take 256 MB (one row at
+// least).
+constexpr unsigned kSysBlocks = 148 * 4;
+inline unsigned sys_wrap_blocks(uint64_t words) {
+  const uint64_t fit = (256ull << 20) / (words * sizeof(int2));
+  return fit < 1 ? 1u : fit < kSysBlocks ? (unsigned)fit : kSysBlocks;
+}
 struct SysArgs {
   const Band* bands;
   const SysJob* jobs;      // trace mode: jobs [lo, hi)
@@ -526,8 +533,9 @@ struct SysArgs {
   const uint64_t* ops_off; // trace mode, per band: its first op slot (n + m slots)
   uint32_t* ops;
   ExactOut* out;
-  int2* wrap;              // block kernel: wrap_words words per block, one per subject column
-  uint64_t wrap_words;
+  int2* wrap;              // block kernel: wrap_blocks rows of wrap_words words, a row per block,
+  uint64_t wrap_words;     // a word per column of the longest subject that a band has
+  unsigned wrap_blocks;    // (no launch has more blocks)
   int8_t scores625[628];
 };
 void launch_sys_score(SysArgs a, int route, uint64_t n_max, cudaStream_t st);

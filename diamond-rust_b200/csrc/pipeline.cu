@@ -546,7 +546,8 @@ __global__ void k_sys_lists(const uint32_t* order, uint64_t lo, uint64_t hi, con
 }
 
 // Traceback jobs: by kernel route, then longest first; count[r] = jobs of
-// route r.
+// route r, count[3] = columns of the block route's longest subject (one long
+// sequence of a set, which no such band has, leaves the others their blocks).
 __global__ void k_sys_jobs(const Band* bands, uint64_t n, const uint64_t* s_offsets, uint64_t* sort_key,
                            uint32_t* sort_val, unsigned long long* count) {
   const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -560,6 +561,7 @@ __global__ void k_sys_jobs(const Band* bands, uint64_t n, const uint64_t* s_offs
   sort_key[k] = ((uint64_t)route << kCostBits) | (kCostMax - (steps < kCostMax ? steps : kCostMax));
   sort_val[k] = (uint32_t)k;
   atomicAdd(count + route, 1ull);
+  if (route == 2) atomicMax(count + 3, (unsigned long long)m);
 }
 __global__ void k_sys_sizes(const uint32_t* idx, uint64_t n, const Band* bands, const uint64_t* s_offsets,
                             SysJob* jobs, uint64_t* size) {
@@ -642,14 +644,11 @@ SysArgs sys_args(const Band* bc, const DevSeqs& qs, const DevSeqs& s, const Scor
   std::memcpy(a.scores625, scr.scores, 625);
   return a;
 }
-// The block kernel's rows of the subject columns, for as many blocks as
-// 256 MB hold (one at least).
-unsigned sys_wrap(drg_ctx* c, SysArgs& a, uint64_t max_m) {
+// The block kernel's rows, for bands on subjects of up to max_m columns.
+void sys_wrap(drg_ctx* c, SysArgs& a, uint64_t max_m) {
   a.wrap_words = max_m + 1;
-  const uint64_t fit = (256ull << 20) / (a.wrap_words * sizeof(int2));
-  const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(fit, kSysBlocks));
-  a.wrap = c->sys_wrap.as<int2>(a.wrap_words * blocks);
-  return blocks;
+  a.wrap_blocks = sys_wrap_blocks(a.wrap_words);
+  a.wrap = c->sys_wrap.as<int2>(a.wrap_words * a.wrap_blocks);
 }
 
 // Scores of the bands at positions [lo, hi) of the sorted order through the
@@ -663,10 +662,10 @@ void sys_scores(drg_ctx* c, SysArgs a, DevBuf& lists, const uint32_t* order, uin
   k_sys_lists<<<ceil_div(hi - lo, 256), 256, 0, st>>>(order, lo, hi, below, a.exact_below, a.bands, a.s_offsets, l0,
                                                        l1, counts, total);
   DRG_CUDA(cudaGetLastError());
-  const unsigned blocks = sys_wrap(c, a, max_m);
+  sys_wrap(c, a, max_m);
   a.list = l1;
   a.d_count = counts + 1;
-  launch_sys_score(a, 2, std::min<uint64_t>(hi - lo, blocks), st);
+  launch_sys_score(a, 2, hi - lo, st);
   a.list = l0;
   a.d_count = counts;
   launch_sys_score(a, 0, hi - lo, st);
@@ -944,8 +943,8 @@ void trace_bands(drg_ctx* c, const Band* bc, uint64_t n, const DevSeqs& qs, cons
   SysJob* jobs = c->sys_jobs.as<SysJob>(n);
   uint64_t* size = c->bj_size.as<uint64_t>(n + 1);
   uint64_t* off = c->bj_off.as<uint64_t>(n + 1);
-  unsigned long long* count = c->bj_max.as<unsigned long long>(3);
-  DRG_CUDA(cudaMemsetAsync(count, 0, 3 * sizeof(unsigned long long), c->stream));
+  unsigned long long* count = c->bj_max.as<unsigned long long>(4);
+  DRG_CUDA(cudaMemsetAsync(count, 0, 4 * sizeof(unsigned long long), c->stream));
   count_launch();
   k_sys_jobs<<<ceil_div(n, 256), 256, 0, c->stream>>>(bc, n, s.offsets, key, val, count);
   const uint32_t* idx = dsort(c, key, key_s, val, val_s, n, 0, kCostBits + 2).vals;
@@ -956,18 +955,18 @@ void trace_bands(drg_ctx* c, const Band* bc, uint64_t n, const DevSeqs& qs, cons
   });
   count_launch();
   k_sys_offsets<<<ceil_div(n, 256), 256, 0, c->stream>>>(jobs, off, n);
-  // jobs per route and the trace bytes, in one wait
-  unsigned long long* h = c->h_stage.as<unsigned long long>(4);
-  DRG_CUDA(cudaMemcpyAsync(h, count, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-  DRG_CUDA(cudaMemcpyAsync(h + 3, off + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
+  // jobs per route, the longest subject and the trace bytes, in one wait
+  unsigned long long* h = c->h_stage.as<unsigned long long>(5);
+  DRG_CUDA(cudaMemcpyAsync(h, count, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
+  DRG_CUDA(cudaMemcpyAsync(h + 4, off + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
   DRG_CUDA(cudaStreamSynchronize(c->stream));
-  const uint64_t lo[4] = {0, h[0], h[0] + h[1], h[0] + h[1] + h[2]}, total = h[3];
+  const uint64_t lo[4] = {0, h[0], h[0] + h[1], h[0] + h[1] + h[2]}, longest = h[3], total = h[4];
   SysArgs a = sys_args(bc, qs, s, scr);
   a.jobs = jobs;
   a.ops_off = d_ops_off;
   a.ops = ops;
   a.out = out;
-  if (h[2] > 0) sys_wrap(c, a, s.max_len);
+  if (lo[3] > lo[2]) sys_wrap(c, a, longest);
   constexpr uint64_t kBudget = 24ull << 30;
   std::vector<uint64_t> hoff;
   if (total > kBudget) fetch_n(c, hoff, off, n + 1);

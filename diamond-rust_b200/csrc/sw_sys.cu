@@ -862,6 +862,9 @@ __global__ void __launch_bounds__(kBlkWarps * 32) k_sys_block(SysArgs a) {
   }
 }
 
+// Blocks for n bands of the block kernel: each has a wrap row.
+unsigned block_grid(const SysArgs& a, uint64_t n) { return (unsigned)(n < a.wrap_blocks ? n : a.wrap_blocks); }
+
 }  // namespace
 
 // Bands that the packed score kernels did not settle (k_sys_lists): one warp
@@ -874,7 +877,7 @@ void launch_sys_score(SysArgs a, int route, uint64_t n_max, cudaStream_t st) {
     const uint64_t blocks = (n_max + kRotWarpsPerBlock - 1) / kRotWarpsPerBlock;
     k_sys_rot<4, false><<<(unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), kRotWarpsPerBlock * 32, 0, st>>>(a);
   } else {
-    k_sys_block<false><<<(unsigned)(n_max < kSysBlocks ? n_max : kSysBlocks), kBlkWarps * 32, 0, st>>>(a);
+    k_sys_block<false><<<block_grid(a, n_max), kBlkWarps * 32, 0, st>>>(a);
   }
   DRG_CUDA(cudaGetLastError());
 }
@@ -913,7 +916,7 @@ void launch_sys_trace(SysArgs a, int route, cudaStream_t st) {
   switch (route) {
     case 0: k_sys_rot<4, true><<<(unsigned)blocks, kRotWarpsPerBlock * 32, 0, st>>>(a); break;
     case 1: k_sys_rot<8, true><<<(unsigned)blocks, kRotWarpsPerBlock * 32, 0, st>>>(a); break;
-    default: k_sys_block<true><<<(unsigned)(n < kSysBlocks ? n : kSysBlocks), kBlkWarps * 32, 0, st>>>(a); break;
+    default: k_sys_block<true><<<block_grid(a, n), kBlkWarps * 32, 0, st>>>(a); break;
   }
   DRG_CUDA(cudaGetLastError());
 }
