@@ -25,6 +25,7 @@
 //
 // Scores equal the packed inter-band kernel's and hence the reference's.
 #include "kernels.h"
+#include "smem_limit.h"
 #include "sw_common.cuh"
 
 namespace drg {
@@ -200,11 +201,7 @@ void launch_sw_band(SwBandArgs a, int max_width, cudaStream_t st) {
   if (a.hi <= a.lo) return;
   a.xbuf_words = (uint32_t)(((size_t)(max_width + kRows + 2)) & ~(size_t)1);
   const size_t smem = sw_band_smem(max_width);
-  static int configured = 0;
-  if ((int)smem > configured) {
-    DRG_CUDA(cudaFuncSetAttribute(k_sw_band, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = (int)smem;
-  }
+  allow_smem((const void*)k_sw_band, sw_band_smem(kSwMaxWidth));
   const int blocks = ceil_div((long long)(a.hi - a.lo), kBandWarps);
   count_launch();
   k_sw_band<<<blocks, kBandWarps * 32, smem, st>>>(a);

@@ -66,6 +66,7 @@
 //
 // The traceback of the HSPs that pass the gate runs in sw_sys.cu.
 #include "kernels.h"
+#include "smem_limit.h"
 #include "sw_common.cuh"
 
 namespace drg {
@@ -365,15 +366,17 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS >= 2 ? 3 : 1) k_sw(SwScoreAr
 }
 
 template <int WARPS>
+constexpr size_t class_smem(int max_width) {
+  return 640 + WARPS * kParts * kProfBytes + (size_t)WARPS * 32 * ring_words(max_width) * 4;
+}
+
+template <int WARPS>
 void launch_class(const SwScoreArgs& a, int max_width, cudaStream_t st) {
   if (a.task_hi <= a.task_lo) return;
   const int threads = WARPS * 32;
-  const size_t smem = 640 + WARPS * kParts * kProfBytes + (size_t)threads * ring_words(max_width) * 4;
-  static int configured = 0;  // per template instance
-  if ((int)smem > configured) {
-    DRG_CUDA(cudaFuncSetAttribute(k_sw<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = (int)smem;
-  }
+  const size_t smem = class_smem<WARPS>(max_width);
+  // (classes 2 and 3 are the same kernel)
+  allow_smem((const void*)k_sw<WARPS>, WARPS == 1 ? class_smem<1>(kSwC3) : smem);
   const int blocks = ceil_div((long long)(a.task_hi - a.task_lo), WARPS * kParts);
   count_launch();
   k_sw<WARPS><<<blocks, threads, smem, st>>>(a);

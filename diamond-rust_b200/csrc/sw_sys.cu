@@ -62,6 +62,7 @@
 //   of 4,182 bands (1,000 queries, sensitive)    1283 -> 530 -> 385 us, routes side by side
 //   13 bands up to 2,000 x 4,000, scores    1,206,000 -> 1,140 -> 950 us
 #include "kernels.h"
+#include "smem_limit.h"
 #include "sw_common.cuh"
 
 namespace drg {
@@ -884,11 +885,7 @@ void launch_sys_score(SysArgs a, int route, uint64_t n_max, cudaStream_t st) {
 
 template <int R>
 static void launch_pair(const SwBandArgs& a, cudaStream_t st) {
-  static bool configured = false;
-  if (!configured) {
-    DRG_CUDA(cudaFuncSetAttribute(k_sys_pair<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem<R>()));
-    configured = true;
-  }
+  allow_smem((const void*)k_sys_pair<R>, pair_smem<R>());
   const uint64_t warps = (a.hi - a.lo + 1) / 2;
   count_launch();
   k_sys_pair<R><<<(unsigned)((warps + kRotWarpsPerBlock - 1) / kRotWarpsPerBlock), kRotWarpsPerBlock * 32,
