@@ -23,6 +23,7 @@
 
 #include "context.h"
 #include "kernels.h"
+#include "stream_fork.h"
 
 namespace drg {
 
@@ -833,7 +834,9 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
     cudaEvent_t fork = log->event();
     DRG_CUDA(cudaEventRecord(fork, c->stream));
     std::vector<cudaEvent_t> ends;  // of the other streams
+    ForkGuard forked;
     auto on = [&](cudaStream_t s2, auto&& launch) {
+      forked.add(s2);
       DRG_CUDA(cudaStreamWaitEvent(s2, fork, 0));
       launch(s2);
       cudaEvent_t e = log->event();
@@ -874,6 +877,7 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
       });
     launch_cls(0, c->stream);
     for (cudaEvent_t e : ends) DRG_CUDA(cudaStreamWaitEvent(c->stream, e, 0));
+    forked.joined();
     cudaEvent_t joined = log->event();
     DRG_CUDA(cudaEventRecord(joined, c->stream));
     for (int k = 0; k < kSwClasses; ++k) {
@@ -983,9 +987,13 @@ void trace_bands(drg_ctx* c, const Band* bc, uint64_t n, const DevSeqs& qs, cons
     streams[1] = c->lanes[1];
     streams[2] = c->lanes[2];
   }
+  ForkGuard forked;
   for (int r = 2; r >= 0; --r) {
     if (lo[r + 1] == lo[r]) continue;
-    if (streams[r] != c->stream) DRG_CUDA(cudaStreamWaitEvent(streams[r], e0, 0));
+    if (streams[r] != c->stream) {
+      forked.add(streams[r]);
+      DRG_CUDA(cudaStreamWaitEvent(streams[r], e0, 0));
+    }
     for (uint64_t k = lo[r]; k < lo[r + 1];) {
       uint64_t e = lo[r + 1];
       uint64_t from = 0;
@@ -1009,6 +1017,7 @@ void trace_bands(drg_ctx* c, const Band* bc, uint64_t n, const DevSeqs& qs, cons
     DRG_CUDA(cudaEventRecord(done, streams[r]));
     DRG_CUDA(cudaStreamWaitEvent(c->stream, done, 0));
   }
+  forked.joined();
   DRG_CUDA(cudaEventRecord(e1, c->stream));
   log->span(e0, e1, &st.ms_trace_kernel);
   if (!times) {  // a call of its own: its kernel times are read now
@@ -1369,9 +1378,9 @@ void Search::start_early_ref() {
     DRG_CUDA(cudaEventCreateWithFlags(&ev_ref, cudaEventDisableTiming));
   }
   early_chunks = merge ? chunks.size() : 1;
+  early_ref = true;  // before its first launch: a failure waits for the side stream
   early = filtered_seeds(0, early_chunks, c->side, c->sort_tmp_side);
   DRG_CUDA(cudaEventRecord(ev_ref, c->side));
-  early_ref = true;
 }
 
 void Search::build_key_filter(uint64_t n_runs) {
