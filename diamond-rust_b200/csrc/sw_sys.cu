@@ -167,9 +167,23 @@ __device__ __forceinline__ CellOut clamped_rows(CellOut b, const uint8_t* q, con
   return v.best > b.best ? v : b;
 }
 
+// A record without an alignment: score 0, or -1, which the host reports as an
+// internal error.
+__device__ __forceinline__ void write_none(const SysArgs& a, uint32_t band, int score = 0) {
+  ExactOut R;
+  R.score = score;
+  R.q_begin = R.q_end = R.s_begin = R.s_end = 0;
+  R.identities = R.positives = R.mismatches = R.gap_openings = R.gaps = R.length = 0;
+  R.n_ops = 0;
+  R.cells = 0;
+  a.out[band] = R;
+}
+
 // The walk of one band by a whole warp.  cell(i, j) is the nibble of a cell of
 // the band with i >= 1 and j >= 1.  It ends where H is 0, and H is known along
 // it: a pair's score less after a diagonal step, a gap's cost more after a gap.
+// A best cell outside the matrix or the band (single: of a row past m + d1,
+// which has one cell) cannot be, and is reported.
 template <typename Cell>
 __device__ __forceinline__ void walk_warp(const SysArgs& a, uint32_t band, const Band& b, int m, const CellOut& best,
                                           const int8_t* mat, bool single, Cell cell) {
@@ -177,6 +191,11 @@ __device__ __forceinline__ void walk_warp(const SysArgs& a, uint32_t band, const
   const uint8_t* q = a.q_letters + a.q_offsets[b.target] + b.q0;
   const uint8_t* s = a.s_letters + a.s_offsets[b.subject];
   const int n = (int)b.n;
+  const int64_t d_best = (int64_t)best.bi - best.bj;
+  if (best.bi < 1 || best.bi > n || best.bj < 1 || best.bj > m || (!single && (d_best < b.d0 || d_best > b.d1))) {
+    if (lane == 0) write_none(a, band, -1);
+    return;
+  }
   uint32_t* ops = a.ops + a.ops_off[band];
   const uint32_t cap = (uint32_t)n + (uint32_t)m;  // op slots of the band
   int i = best.bi, j = best.bj;
@@ -283,16 +302,6 @@ __device__ __forceinline__ void walk_warp(const SysArgs& a, uint32_t band, const
     R.cells = 0;
     a.out[band] = R;
   }
-}
-
-__device__ __forceinline__ void write_none(const SysArgs& a, uint32_t band) {
-  ExactOut R;
-  R.score = 0;
-  R.q_begin = R.q_end = R.s_begin = R.s_end = 0;
-  R.identities = R.positives = R.mismatches = R.gap_openings = R.gaps = R.length = 0;
-  R.n_ops = 0;
-  R.cells = 0;
-  a.out[band] = R;
 }
 
 // Job t's trace.
