@@ -15,7 +15,7 @@
 // highest sensitivity), so the chain of a step bounds them: eight pairs of two
 // DPX operations.  Everything else is kept off it.  Cells outside the band are
 // dead through an addend on their diagonal and open cost instead of masks on
-// what they give (as in the lane kernel): -16384 for pair p in the columns
+// what they give (as in the lane kernel, sw_sys.cu): -16384 for pair p in the columns
 // where it was for pair 0 p columns earlier, one new value per column.  A lane
 // runs dead columns before its strip starts and after it ends, without a
 // branch.  Letters are loaded four columns ahead, profile words lie one lane

@@ -37,7 +37,8 @@
 //   H  = max(Hdiag + sc, E' - oc, F' - oc, 0)         (three adds, vimax3.relu)
 //   F' = max(F' - ge, H)                              (viaddmax, for the next column)
 // Near a strip's ends a cell outside the band is dead by an addend of -16384 on
-// its diagonal and open cost, as in the lane kernel (sw_sys.cu).
+// its diagonal and open cost, as in the lane kernel (sw_sys.cu, which says why
+// the H that it may keep beside scores above 16384 changes none).
 //
 // ALU bound (that pipe is busy 86 % of the time).  What held it at 76 % before
 // was not the arithmetic: with the first and last 16 steps of a strip
@@ -61,8 +62,7 @@
 // keeps one cell per such row, clamped to column m, whose H is at most
 // max(largest matrix score, band best - open), so a packed best above the
 // matrix's largest score is the reference's; smaller results are recomputed
-// exactly.  Cells left or right of the band in the first/last 16 steps of
-// a strip are dead: their H is 0 and they pass no gap.
+// exactly.
 //
 // The traceback of the HSPs that pass the gate runs in sw_sys.cu.
 #include "kernels.h"

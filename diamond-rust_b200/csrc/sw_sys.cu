@@ -498,16 +498,21 @@ __global__ void __launch_bounds__(kRotWarpsPerBlock * 32) k_sys_rot(SysArgs a) {
 // E and F are kept with the open cost added back (E' = max(E' - ge, H) above,
 // F' = max(F' - ge, H) to the left, H = max(0, D, E' - oc, F' - oc): all at
 // least 0).  Outside the band no cell is masked after it is computed: an
-// addend of -16384 on D and on the open cost makes its H 0, and its E' comes
-// only from such cells above it.  Row r is outside in the column that row 0
-// was r columns earlier, so a lane computes one addend per column and keeps
-// the last R + 1; a strip starts with all of them dead, which is its left
-// edge; and what a strip hands down is dead with its last row.  A cell is five
-// ALU operations, half a three-input maximum and three adds on the FMA pipe,
-// which runs beside (ten ALU operations with masks on E and H and selects for
-// the left edge: 22 bands of a 497-aa query 141 -> 129 us, the widest route of
-// 1,000 queries very sensitive 4,620 -> 3,100 us, of 13 queries
-// ultra-sensitive 2,160 -> 1,600 us).
+// addend of -16384 on D and on the open cost makes its H 0 below 16384 + oc.
+// Scores go up to 31743, so a cell beside the band may keep an H of up to some
+// 15300.  That changes no score: a path that turns outside the band pays 16384
+// for it, again for each further cell there that it aligns or turns at and for
+// each strip that its E' leaves (e_out), and comes back at most R rows below
+// where it left, which a path inside reaches for some R mismatches.  Row r is
+// outside in the column that row 0 was r columns earlier, so a lane computes
+// one addend per column and keeps the last R + 1; a strip starts with all of
+// them dead, which is its left edge; and the E' that a strip hands down is dead
+// with its last row.  A cell is five ALU operations, half a three-input
+// maximum and three adds on the FMA pipe, which runs beside (ten ALU
+// operations with masks on E and H and selects for the left edge: 22 bands of
+// a 497-aa query 141 -> 129 us, the widest route of 1,000 queries very
+// sensitive 4,620 -> 3,100 us, of 13 queries ultra-sensitive 2,160 -> 1,600
+// us).
 // All 32 lanes run whatever the width, so a band takes the fewest rows per lane
 // that hold it: 4, 6, 8, 12 or 16, the widths up to 151, 211, 271, 391 and 511
 // (with 4, 8 and 16 alone: 26.3 ms for 1,000 queries very sensitive, whose
