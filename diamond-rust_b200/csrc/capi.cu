@@ -391,7 +391,7 @@ int drg_seed_build(drg_ctx* c, const uint8_t* letters, const uint64_t* offsets, 
   const uint64_t N = s.total;
   // The sort covers the bits of the shape's largest key and one more, so that
   // "no seed" (all ones) sorts last; keys that then fit 32 bits are sorted as
-  // 32-bit words (2.26M letters, weight 8: 255 -> 110 us).
+  // 32-bit words (2.26M letters, weight 8: 255 -> 121 us).
   double mx = 1.0;
   for (int k = 0; k < sh.weight; ++k) mx *= (double)red.size;
   int bits = 64;

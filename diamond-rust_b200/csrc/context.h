@@ -19,7 +19,7 @@ struct drg_ctx {
   int device = 0;
   int slot = -1;                // constant-memory bank of this context (kConstSlots of them)
   cudaStream_t stream = nullptr;
-  cudaStream_t side = nullptr;  // concurrent launches (wide-band classes)
+  cudaStream_t side = nullptr;  // concurrent launches (the score kernel's wider classes, early reference seeds)
   // more of them: each route of the score and traceback passes has its own, so
   // that the launches' longest bands run beside one another
   cudaStream_t lanes[7] = {};
@@ -55,7 +55,7 @@ struct drg_ctx {
 
 struct drg_db {
   drg_ctx* ctx = nullptr;
-  uint8_t* letters = nullptr;   // device, 16 bytes of slack after the end
+  uint8_t* letters = nullptr;   // device, 64 sentinel letters after the end
   uint8_t* score_letters = nullptr;  // device: letters clamped to 24, only when some code is above 24
   uint64_t* offsets = nullptr;  // device, n + 1
   uint32_t* owner = nullptr;    // device: letter -> sequence

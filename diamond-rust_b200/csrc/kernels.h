@@ -289,12 +289,12 @@ struct SwScoreArgs {
   const uint8_t* s_letters;
   const uint64_t* s_offsets;
   int gap_open, gap_extend;
-  int32_t* score;     // score mode: per band (indexed like bands)
-  int32_t* best_row;  // score mode: first DP row holding the best (0 if none)
+  int32_t* score;     // per band (indexed like bands)
+  int32_t* best_row;  // a bound of the first DP row holding the best (0 if none)
   unsigned long long* cells_eval;  // optional: [0] DP cells the lanes evaluated (after skipping), [2] the warps' (idle lanes too)
   int8_t scores625[628];  // substitution scores, row-major
 };
-// One band of the intra-band (one warp per band) kernel.
+// One band of the kernels that spread a band over lanes (k_sys_pair, k_sw_band).
 struct SwBandJob {
   uint32_t band;       // index into bands
   uint32_t row_first;  // first DP row (1-based)
@@ -335,16 +335,14 @@ void launch_sw_band_route(const SwBandArgs& a, int route, int max_width, cudaStr
 
 // Width classes of the packed kernel by the widest band of a warp (the shared
 // ring holds W + 1 words per thread); each fits 3 blocks per SM but the last.
-constexpr int kSwMinWidth = 17;   // narrower bands use the exact kernel
 constexpr int kSwC0 = 136, kSwC1 = 272, kSwC2 = 544, kSwC3 = 1700;
 constexpr int kSwClassMax[4] = {kSwC0, kSwC1, kSwC2, kSwC3};  // 4, 2, 1, 1 warps per block
-constexpr int kSwMaxWidth = 1700;                       // wider bands use the exact kernel
+constexpr int kSwMaxWidth = 1700;  // wider bands run in 32-bit lanes (sw_sys.cu)
 // Bands whose best can reach this bound are not packed: every H of the packed
 // kernels stays far from the 16-bit limit.
 constexpr int kSwPackedMaxBest = 31743;
 constexpr int kSwClasses = 4;
-int sw_width_class(int width);  // 0..3, or -1 for the exact kernel
-void launch_sw_class(const SwScoreArgs& a, int cls, cudaStream_t st);  // score mode
+void launch_sw_class(const SwScoreArgs& a, int cls, cudaStream_t st);
 
 // ---- device radix sort (radix_sort.cu) --------------------------------------
 // The sort's scratch and the epoch of its last pass (look-back words carry

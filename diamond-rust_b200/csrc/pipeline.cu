@@ -9,7 +9,7 @@
 //   sw      packed 16-bit banded SW scores (half warp = 16 bands of one query)
 //   gate    ALP E-value and the max_hsps band walk per pair
 // Host: exact E-values of the kept bands, per-target culling (search.rs:256-270),
-// then the exact traceback kernel for the surviving HSPs only.
+// then the traceback of the surviving HSPs only, in 32-bit lanes.
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 
@@ -128,7 +128,7 @@ __host__ __device__ __forceinline__ int sw_class_of(uint32_t w) {
 }
 
 // Score-pass sort key, radix-sorted over bits kKeyLo..end:
-//   end - 1 wide band (one warp per band, after every packed-kernel band),
+//   end - 1 wide band (spread over lanes, after every band of k_sw),
 //   end - 2 transposed band, 24..end - 3 group (target << 16 | window start,
 //   or the subject of a transposed band), 13..23 width.  Not computed: ~0.
 // (Medium bands share warps with the narrow bands of their group: giving
@@ -206,7 +206,7 @@ __global__ void k_count_fast_narrow(const uint64_t* keys, uint64_t n, uint64_t w
 }
 
 // The tuned routing (drg_tuning): where the packed 16-bit kernel starts, where
-// the score pass hands bands to the band kernel, and whether it transposes.
+// the score pass hands bands to the lane kernels, and whether it transposes.
 struct SwTune {
   int wide_min, min_packed, transpose;
 };
@@ -214,8 +214,8 @@ SwTune sw_tune(const drg_ctx* c) {
   return {c->tuning.sw_wide_min_width, c->tuning.sw_min_packed_width, c->tuning.sw_transpose};
 }
 
-// Which kernel a band goes to: the packed kernel (fast), its wide-band
-// variant (wide), and whether the band has fewer strips transposed.
+// Where a band goes: 16-bit lanes (fast), several of them per band (wide); and
+// whether it has fewer strips transposed.
 struct SwRoute {
   bool fast, wide, tr;
   int64_t rs, re, ts, te;
@@ -608,7 +608,7 @@ __global__ void k_gather_bands_dev(const uint32_t* idx, uint64_t n, const int64_
 
 namespace {
 
-// Jobs of the band kernel by route.
+// Jobs of the lane kernels by route.
 struct BandJobs {
   SwBandJob* jobs = nullptr;
   uint64_t n = 0;
@@ -733,8 +733,8 @@ void score_bands(drg_ctx* c, const Band* bc, uint64_t n_bands, const DevSeqs& qs
   }
   count_launch();
   k_count_fast_narrow<<<1, 1, 0, c->stream>>>(swks, n_bands, kb.wide, cnt);
-  // ---- wide bands (positions [narrow, fast) of the sorted order): band-
-  // kernel jobs by route, then longest first
+  // ---- wide bands (positions [narrow, fast) of the sorted order): lane
+  // kernels' jobs by route, then longest first
   SwBandJob* jobs_u = c->band_jobs_u.as<SwBandJob>(n_bands);
   SwBandJob* wjobs = c->band_jobs.as<SwBandJob>(n_bands);
   uint64_t* jkey = c->bj_key.as<uint64_t>(n_bands);

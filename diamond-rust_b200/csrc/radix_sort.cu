@@ -152,12 +152,11 @@ __device__ __forceinline__ void load_tile(const K* __restrict__ src, uint64_t ba
   }
 }
 
-// The lanes whose 8-bit digit equals this lane's: a ballot per bit, four
-// instructions each (the compiler's form of the same loop takes thirteen).
-// match.any runs on the ADU pipe, some 34 cycles an instruction and SM, which
-// bounded a pass (ncu: ADU 48 %, issue 19 %).  Per pass, by match.any / this, with
-// the values loaded ahead of the look-back: 5.75M u32 pairs 78.7 / 51.5 us,
-// 13.4M u64 pairs 192 / 140, 2.8M u64 keys 42.6 / 31.6.
+// The lanes whose 8-bit digit equals this lane's: a ballot per bit, written out
+// as the four instructions it needs.  match.any has a slower pipe of its own,
+// which bounded a pass.  Per pass, by match.any / this, with the values loaded
+// ahead of the look-back: 5.75M u32 pairs 78.7 / 51.5 us, 13.4M u64 pairs 192 /
+// 140, 2.8M u64 keys 42.6 / 31.6.
 __device__ __forceinline__ uint32_t same_digit(uint32_t d) {
   uint32_t peers = 0xFFFFFFFFu;
 #pragma unroll

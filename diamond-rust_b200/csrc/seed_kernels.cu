@@ -348,7 +348,7 @@ void launch_seed_enum(const uint8_t* letters, const uint64_t* offsets, const uin
 // ---- seed::build's entries (seed.rs:76-104) ------------------------------------
 // Sorted keys and letter indices to (key, sequence, position) records, and the
 // number of valid ones ("no seed" keys sort last).  One thread per entry, two
-// gathers (owner, offset) and one 16-byte store: 2.2M entries take 40 us, where
+// gathers (owner, offset) and one 16-byte store: 2.2M entries take 22 us, where
 // a host loop with a binary search per entry took 95 ms.
 template <typename K>
 __global__ void k_seed_entries(const K* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t n,

@@ -38,6 +38,27 @@ constexpr int kLag = kRows + 2;   // steps between consecutive lanes
 constexpr int kProfWords = 26 * 4 * 32;  // profile of a warp's strips: [residue][rows 4w..4w+3][lane]
 constexpr int kBandWarps = 4;
 
+// Columns that a residue is loaded ahead of its use.
+constexpr int kQueue = 4;
+
+struct Lane {
+  const uint8_t* s;  // subject letters
+  int m;             // subject length
+  int jbase;         // absolute column of relative column 0 in this strip
+  uint32_t queue[kQueue];  // prefetched residues of the next columns
+};
+
+// The residue of column c (subject index jbase + c - 1) from the prefetch
+// queue, issuing the load of column c + kQueue.
+__device__ __forceinline__ uint32_t next_residue(Lane& L, int c) {
+  const uint32_t ahead = subject_residue(L, L.jbase + c + kQueue - 1);
+  const uint32_t res = L.queue[0];
+#pragma unroll
+  for (int i = 0; i + 1 < kQueue; ++i) L.queue[i] = L.queue[i + 1];
+  L.queue[kQueue - 1] = ahead;
+  return res;
+}
+
 // State of a lane's strip; M[p]: what the cells of pair p add at this column.
 struct BandRegs {
   uint32_t H[kPairs], F[kPairs], M[kPairs];

@@ -1,8 +1,6 @@
-// Shared pieces of the packed 16-bit banded Smith-Waterman kernels: the
-// s16x2 helpers, the per-thread register state of one 16-row strip and the
-// per-lane subject view.  A strip's 16 rows are 8 pairs of 16-bit lanes: pair
-// p holds row p at column c (low half) and row p + 8 at column c - 1 (high
-// half).
+// Shared pieces of the packed 16-bit banded Smith-Waterman kernels.  A strip's
+// 16 rows are 8 pairs of 16-bit lanes: pair p holds row p at column c (low half)
+// and row p + 8 at column c - 1 (high half).
 #pragma once
 #include <cstdint>
 
@@ -41,31 +39,10 @@ __device__ __forceinline__ constexpr uint32_t pick_sel(int b) {
   return (uint32_t)(b) | ((uint32_t)(8 | b) << 4) | ((uint32_t)(4 + b) << 8) | ((uint32_t)(8 | (4 + b)) << 12);
 }
 
-// Columns that a residue is loaded ahead of its use (2, 3, 6 and 8 measured
-// beside 4: 17.92, 18.10, 17.82 and 17.81 ms against 17.82 for the 1,000-query
-// sensitive search).
-constexpr int kQueue = 4;
-
-struct Lane {
-  const uint8_t* s;  // subject letters
-  int m;             // subject length
-  int jbase;         // absolute column of relative column 0 in this strip
-  uint32_t queue[kQueue];  // prefetched residues of the next columns
-};
-
 // Residue of subject index j, or the sentinel off the sequence.
+template <typename Lane>
 __device__ __forceinline__ uint32_t subject_residue(const Lane& L, int j) {
   return ((unsigned)j < (unsigned)L.m) ? (uint32_t)__ldg(L.s + j) : (uint32_t)kSentinel;
-}
-// The residue of column c (subject index jbase + c - 1) from the prefetch
-// queue, issuing the load of column c + kQueue.
-__device__ __forceinline__ uint32_t next_residue(Lane& L, int c) {
-  const uint32_t ahead = subject_residue(L, L.jbase + c + kQueue - 1);
-  const uint32_t res = L.queue[0];
-#pragma unroll
-  for (int i = 0; i + 1 < kQueue; ++i) L.queue[i] = L.queue[i + 1];
-  L.queue[kQueue - 1] = ahead;
-  return res;
 }
 
 __device__ __forceinline__ int lo16(uint32_t x) { return (int)(int16_t)(x & 0xFFFFu); }

@@ -40,11 +40,12 @@
 // its diagonal and open cost, as in the lane kernel (sw_sys.cu, which says why
 // the H that it may keep beside scores above 16384 changes none).
 //
-// ALU bound (that pipe is busy 86 % of the time).  What held it at 76 % before
-// was not the arithmetic: with the first and last 16 steps of a strip
-// unrolled, each with its masks, the twelve warps of an SM were spread over
-// 40 KB of code, and instruction fetch past the SM's own cache ran at 91 % of
-// its peak; neither more warps nor fewer operations changed anything.
+// ALU bound: that pipe is busy 86.5 % of the time, at 3.35 operations per computed
+// cell (ncu, 200 queries).  The recurrence above is 2.25 of them; the edges'
+// addends, the letters, the byte picks of a column and the ring are the rest.
+// Before, neither more warps nor fewer operations changed anything: with the
+// first and last 16 steps of a strip unrolled, each with its masks, the code
+// of an SM's twelve warps did not stay in its instruction cache.
 // Now two loops of four steps make up a strip, edges and middle.  A loop holds
 // whole groups of four columns because a load in flight that is moved from
 // register to register waits, so letters come four at a time as words, a group
@@ -83,7 +84,10 @@ constexpr int kProfBytes = 2 * kProfHigh;
 // from the two aligned words that hold them (the second is the next group's
 // first), fetched a group ahead.  Every letter buffer starts on a word
 // boundary and has slack behind its end.
-struct Letters : Lane {
+struct Letters {
+  const uint8_t* s;  // column letters
+  int m;             // how many
+  int jbase;         // absolute column of relative column 0 in this strip
   uint32_t w0, w1;  // aligned words: of the next group's first letter, and the one after
   uint32_t shift;   // bits of w0 before the group's first letter
   int j;            // subject index of the next group's first column
@@ -384,13 +388,6 @@ void launch_class(const SwScoreArgs& a, int max_width, cudaStream_t st) {
 }
 
 }  // namespace
-
-int sw_width_class(int width) {
-  if (width < kSwMinWidth) return -1;
-  for (int c = 0; c < kSwClasses; ++c)
-    if (width <= kSwClassMax[c]) return c;
-  return -1;
-}
 
 void launch_sw_class(const SwScoreArgs& a, int cls, cudaStream_t st) {
   switch (cls) {

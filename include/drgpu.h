@@ -102,16 +102,17 @@ typedef struct {
   double ms_h2d, ms_d2h;
   double ms_sw_kernel;      /* device time of the packed score kernel launches alone */
   uint64_t sw_launches, kernel_launches;
-  uint64_t exact_bands;     /* bands the exact kernel handled (not the packed one) */
+  uint64_t exact_bands;     /* bands scored in 32-bit lanes (not, or not only, in the packed kernels) */
   /* packed score kernel per class of the widest band in a warp
    * (W <= 136, <= 272, <= 544, <= 1700) */
-  uint64_t sw_class_tasks[4];      /* warps (32 bands each at most) */
+  uint64_t sw_class_tasks[4];      /* warps (two tasks of up to 16 bands each) */
   uint64_t sw_class_max_steps[4];  /* longest warp: strips x (W + 16) column steps */
   double ms_sw_class[4];           /* device time of each class launch */
   double ms_trace_kernel;          /* device time of the trace-mode kernel launches */
   uint64_t dp_cells_lane;          /* score kernel: each band's own rows x (W + 16), without warp padding */
-  uint64_t sw_wide_bands;          /* score pass: bands wider than 272 columns, one warp per band */
-  double ms_sw_wide;               /* device time of their launch (concurrent with the classes) */
+  uint64_t sw_wide_bands;          /* score pass: bands spread over the lanes of a warp (wider than 272 columns,
+                                    * or in too few or too long warps of the classes) */
+  double ms_sw_wide;               /* device time of their launches (concurrent with the classes) */
   uint64_t dp_cells_issued;        /* score kernel: warps x column steps x 16 x 32, idle lanes included */
   uint64_t index_hits;             /* index chunks whose sorted reference seeds came from the db's cache */
   uint64_t sw_transposed_bands;    /* score kernel: bands run with the subject as rows */
@@ -133,11 +134,11 @@ typedef struct {
 
 /* Tile and routing choices of a context (none changes a result).  The
  * defaults are the first value of each list; drg_autotune picks among them.
- *  sw_wide_min_width   score pass: bands at least this wide run in the lane-
- *                      group band kernel instead of one band per lane
- *                      (273; 137 = two bands per warp from 137, 545, 1701 = never)
- *  sw_min_packed_width bands narrower than this run in int32 lanes (exact
- *                      kernel) instead of 16-bit lanes (17, 33)
+ *  sw_wide_min_width   score pass: bands at least this wide run spread over the
+ *                      lanes of a warp instead of one band per lane
+ *                      (273; 137; 545; 1701 = never)
+ *  sw_min_packed_width bands narrower than this run in 32-bit lanes instead of
+ *                      16-bit ones (17, 33)
  *  sw_transpose        short-subject bands may run with the subject as rows (1, 0)
  *  sort_small_tiles    radix sort tiles of 8 (u32) / 6 (u64) keys per thread
  *                      instead of 16 / 12 (0, 1) */
@@ -204,8 +205,8 @@ int drg_extend_span_batch(drg_ctx* ctx, const uint8_t* q_letters, const uint64_t
                           int32_t gap_extend, drg_aligned* out, uint32_t** ops, uint64_t* n_ops);
 
 /* gapped::extend_span, score only (gapped.rs:67-203): the band score the
- * search's E-value gate uses, computed by the same packed 16-bit kernel
- * (exact kernel where that one does not apply).  scores[i] = 0 is None. */
+ * search's E-value gate uses, computed by the same packed 16-bit kernels
+ * (32-bit lanes where those do not apply).  scores[i] = 0 is None. */
 int drg_extend_span_scores(drg_ctx* ctx, const uint8_t* q_letters, const uint64_t* q_offsets, uint64_t n_q,
                            const uint8_t* s_letters, const uint64_t* s_offsets, uint64_t n_s,
                            const drg_span_job* jobs, uint64_t n_jobs, const char* matrix, int32_t gap_open,
