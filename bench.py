@@ -43,7 +43,7 @@ METRIC = "bit-exact queries/sec + SW GCUPS, batched vs plain on 1 B200; p50/p99 
 # 200-query case over that pass's evaluated cells (profiles/); scaled to a full
 # pass by its evaluated cells (the traffic is the bands, query windows and
 # subjects the warps read, in proportion to the work).
-SW_TRAFFIC_PER_CELL = 19.898624e6 / 13.531323984e9
+SW_TRAFFIC_PER_CELL = 17.855744e6 / 10.108165056e9
 SENS = "sensitive"
 
 
